@@ -40,6 +40,14 @@ struct PixView {
     __device__ __forceinline__ float operator[](int k) const { return p[k * ld].x; }
 };
 
+// The same over the column pairs of PairPixels.
+template <int R>
+struct PairView {
+    const float *p;
+    int slot, ld;
+    __device__ __forceinline__ float operator[](int k) const { return p[PairPixels<R>::value(k, slot, ld)]; }
+};
+
 template <int R, int KIND>
 struct SmemLayout {
     enum {
@@ -85,8 +93,8 @@ __device__ __forceinline__ void zero_row(float *loc, int id) {
     dst[2] = z;
 }
 
-template <int R>
-__device__ __forceinline__ void edge_means(const PixView &img, float &Mean1, float &Mean2, float &Mean3, float &Mean4) {
+template <int R, class View>
+__device__ __forceinline__ void edge_means(const View &img, float &Mean1, float &Mean2, float &Mean3, float &Mean4) {
     Mean1 = 0;
     Mean2 = 0;
     Mean3 = 0;
@@ -159,8 +167,8 @@ struct SinglePrep {
 // point Ininf of the fit from the ROI's edge means and centre pixel.
 // PRE = false: the mask widths and bounds only, Ininf untouched (the
 // learned-start fit takes its start point from elsewhere).
-template <int R, int KIND, bool PRE = true>
-__device__ __forceinline__ SinglePrep single_prefit(const PixView &img, const float *pw, const CorePara &c,
+template <int R, int KIND, bool PRE = true, class View>
+__device__ __forceinline__ SinglePrep single_prefit(const View &img, const float *pw, const CorePara &c,
                                                     float *Ininf) {
     SinglePrep sp;
     sp.Simga_Max_Th = R / 1.5f / 2.35f;
@@ -337,38 +345,56 @@ struct SingleLayout {
     };
 };
 
-// Stage a block's records: pixel k of slot s at s_img[k * S + s] as
-// (max((adu - offset) * gain, 1), its __logf).  WORDS: the records are
-// 4-byte aligned and read two pixels per load; element (word, slot) is taken
-// slot-fastest so a warp's shared-memory stores fall in distinct banks.
-template <int R, bool WORDS, int S = kTPB>
-__device__ __forceinline__ void stage_single(float2 *s_img, const uint16_t *rois, const Queue &q, int base, int cnt,
+// Stage a block's records: pixel k of slot s as (max((adu - offset) * gain,
+// 1), its __logf), at s_img[k * S + s] or (PAIRED) in PairPixels.  WORDS: the
+// records are 4-byte aligned and read two pixels per load; element (word,
+// slot) is taken slot-fastest, so that a warp's shared-memory stores run over
+// consecutive slots.
+template <int R, bool WORDS, bool PAIRED, int S = kTPB>
+__device__ __forceinline__ void stage_single(float *s_img, const uint16_t *rois, const Queue &q, int base, int cnt,
                                              float Offset, float KAdc) {
     enum { PIX = R * R, WHOLE = R * (R + 1), WPR = (PIX + 1) / 2 };
+    auto put = [&](int k, int slot, float v) {
+        if (PAIRED) {
+            float *d = s_img + PairPixels<R>::value(k, slot, S);
+            d[0] = v;
+            d[PairPixels<R>::log_off(k)] = __logf(v);
+        } else {
+            reinterpret_cast<float2 *>(s_img)[k * S + slot] = make_float2(v, __logf(v));
+        }
+    };
     if (WORDS) {
-        for (int idx = threadIdx.x; idx < cnt * WPR; idx += kTPB) {
+        for (int idx = threadIdx.x; idx < cnt * WPR; idx += blockDim.x) {
             const int wd = idx / cnt;
             const int slot = idx - wd * cnt;
             const int id = queue_at(q, base + slot);
             const uint32_t u = __ldg(reinterpret_cast<const uint32_t *>(rois + (size_t)id * WHOLE) + wd);
             const int k = 2 * wd;
-            const float v0 = fmaxf(((float)(u & 0xFFFFu) - Offset) * KAdc, 1.0f);
-            s_img[k * S + slot] = make_float2(v0, __logf(v0));
-            if (k + 1 < PIX) {
-                const float v1 = fmaxf(((float)(u >> 16) - Offset) * KAdc, 1.0f);
-                s_img[(k + 1) * S + slot] = make_float2(v1, __logf(v1));
-            }
+            put(k, slot, fmaxf(((float)(u & 0xFFFFu) - Offset) * KAdc, 1.0f));
+            if (k + 1 < PIX) put(k + 1, slot, fmaxf(((float)(u >> 16) - Offset) * KAdc, 1.0f));
         }
     } else {
-        for (int idx = threadIdx.x; idx < cnt * PIX; idx += kTPB) {
+        for (int idx = threadIdx.x; idx < cnt * PIX; idx += blockDim.x) {
             const int k = idx / cnt;
             const int slot = idx - k * cnt;
             const int id = queue_at(q, base + slot);
             const uint16_t u = __ldg(rois + (size_t)id * WHOLE + k);
-            const float pixval = fmaxf((u - Offset) * KAdc, 1.0f);
-            s_img[k * S + slot] = make_float2(pixval, __logf(pixval));
+            put(k, slot, fmaxf((u - Offset) * KAdc, 1.0f));
         }
     }
+}
+
+// The pixel view and evaluator of a thread's slot: PairEval where the
+// distance's rounding is fixed in the source (kPaired), else StagedEval.
+template <int R, int KIND, int DIST, bool FULL>
+using SingleEval = std::conditional_t<kPaired<R, DIST>, PairEval<R, KIND, DIST, FULL>, StagedEval<R, KIND, DIST, FULL>>;
+
+template <int R, int DIST>
+__device__ __forceinline__ auto single_view(const float *s_img, int slot, int S) {
+    if constexpr (kPaired<R, DIST>)
+        return PairView<R>{s_img, slot, S};
+    else
+        return PixView{reinterpret_cast<const float2 *>(s_img) + slot, S};
 }
 
 // One block's tile of the single-emitter fit: queue entries base .. base+S-1
@@ -383,14 +409,14 @@ __device__ __forceinline__ void single_tile(float *smem, int base, int n, const 
     enum { P = KindTraits<KIND>::P, PIX = R * R, WHOLE = R * (R + 1) };
     if (base >= n) return;
     const int cnt = min(S, n - base);
-    float2 *s_img = reinterpret_cast<float2 *>(smem + L::IMG);
-    stage_single<R, WORDS, S>(s_img, rois, q, base, cnt, c.Offset, c.KAdc);
+    float *s_img = smem + L::IMG;
+    stage_single<R, WORDS, kPaired<R, DIST>, S>(s_img, rois, q, base, cnt, c.Offset, c.KAdc);
     __syncthreads();
     const int tid = threadIdx.x;
     if (tid >= cnt) return;
 
     const int CurFluoID = queue_at(q, base + tid);
-    const PixView img{s_img + tid, S};
+    const auto img = single_view<R, DIST>(s_img, tid, S);
     // the mask: FULL, pixel k at mask[k * S]; else float4 chunk j at ((float4 *)mask)[j * S]
     float *mask = smem + L::WU + (FULL ? tid : 4 * tid);
     const uint16_t *hdr = rois + (size_t)CurFluoID * WHOLE + PIX;
@@ -407,8 +433,8 @@ __device__ __forceinline__ void single_tile(float *smem, int base, int n, const 
         wle_weights_unique<R, MASK>(reinterpret_cast<float4 *>(mask), S, sp.WLE_SigmaX, sp.WLE_SigmaY,
                                     sp.MoleculeType);
     float D[P * P];  // the inverse Hessian, in registers
-    bfgs_fit<P, KindTraits<KIND>::IT>(StagedEval<R, KIND, DIST, FULL>{s_img + tid, mask, S}, Ininf, D, 1);
-    if (ll) ll[CurFluoID] = model_loglik<R, KIND, DIST, kCompiler>(s_img + tid, S, Ininf, 0, 1);
+    bfgs_fit<P, KindTraits<KIND>::IT>(SingleEval<R, KIND, DIST, FULL>(s_img, mask, tid, S), Ininf, D, 1);
+    if (ll) ll[CurFluoID] = model_loglik<R, KIND, DIST, kCompiler>(img, Ininf, 0, 1);
     float row[12];
     bool accepted;
     float CurSNR;
@@ -646,14 +672,17 @@ __global__ void __launch_bounds__(kTPB, (SingleLayout<R, FULL>::BLOCKS))
                        int direct2e) {
     typedef SingleLayout<R, FULL> L;
     enum { P = KindTraits<KIND>::P, PIX = R * R, WHOLE = R * (R + 1) };
-    typedef StagedAnalyticEval<R, KIND, DIST, FULL> Eval;
+    typedef StagedAnalyticEval<R, KIND, SingleEval<R, KIND, DIST, FULL>, FULL> Eval;
     extern __shared__ __align__(16) float smem[];
     const int n = queue_len(q);
     const int base = blockIdx.x * kTPB;
     if (base >= n) return;
     const int cnt = min(kTPB, n - base);
-    float2 *s_img = reinterpret_cast<float2 *>(smem + L::IMG);
-    stage_rois<R>(s_img, rois, q, base, cnt, c.Offset, c.KAdc);
+    float *s_img = smem + L::IMG;
+    if ((reinterpret_cast<uintptr_t>(rois) & 3) == 0)
+        stage_single<R, true, kPaired<R, DIST>>(s_img, rois, q, base, cnt, c.Offset, c.KAdc);
+    else
+        stage_single<R, false, kPaired<R, DIST>>(s_img, rois, q, base, cnt, c.Offset, c.KAdc);
     __syncthreads();
     const int tid = threadIdx.x;
     if (tid >= cnt) return;
@@ -664,7 +693,7 @@ __global__ void __launch_bounds__(kTPB, (SingleLayout<R, FULL>::BLOCKS))
     const int XOffset = hdr[0], YOffset = hdr[1];
     const int CurFrame = hdr[2] + 65536 * hdr[3];
     const float *pw = wle + (size_t)id * QCS_WLE_PARA_NUM;
-    const PixView img{s_img + tid, kTPB};
+    const auto img = single_view<R, DIST>(s_img, tid, kTPB);
 
     float Ininf[P];
     const SinglePrep sp = single_prefit<R, KIND, false>(img, pw, c, Ininf);  // mask widths only
@@ -685,7 +714,8 @@ __global__ void __launch_bounds__(kTPB, (SingleLayout<R, FULL>::BLOCKS))
         Ininf[P - 1] = st[5] * rBScalFactor;
     }
     float D[P * P];  // the inverse Hessian, in registers
-    bfgs_fit<P, ITERS, Eval, NB>(Eval{{s_img + tid, mask, kTPB}}, Ininf, D, 1);
+    const Eval ev(s_img, mask, tid, kTPB);
+    bfgs_fit<P, ITERS, Eval, NB>(ev, Ininf, D, 1);
 
     float row[12];
     bool accepted;
@@ -698,7 +728,7 @@ __global__ void __launch_bounds__(kTPB, (SingleLayout<R, FULL>::BLOCKS))
 #pragma unroll 1
     for (int r = 0; r < R; r++)
         for (int col = 0; col < R; col++) {
-            const float2 pl = s_img[tid + (r * R + col) * kTPB];
+            const float2 pl = ev.pixel(r, col);
             const float e = single_expo<KIND, DIST>(col + 0.5f, r + 0.5f, Ininf);
             dev += single_term<KIND>(e, Ininf, pl.x, pl.y);
         }
@@ -998,7 +1028,7 @@ __global__ void __launch_bounds__(kTPB) fit_multi_kernel(const uint16_t *__restr
     multi_prefit<R, KIND>(img, c, Ininf, WLE_SigmaX);
     if (KIND == k2E) wle_weights<R, MASK>(w, kTPB, WLE_SigmaX, WLE_SigmaX, QCS_MOLECULE_MULTIFIT);
     mle_fit<R, KIND, DIST, SUM2>(roi, Ininf, D, kTPB);
-    if (ll) ll[CurFluoID] = model_loglik<R, KIND, DIST, SUM2>(s_img + tid, kTPB, Ininf, 0, 1);
+    if (ll) ll[CurFluoID] = model_loglik<R, KIND, DIST, SUM2>(PixView{s_img + tid, kTPB}, Ininf, 0, 1);
     if (KIND == k3E && mo.params) {
 #pragma unroll
         for (int k = 0; k < P; k++) mo.params[(size_t)slot * P + k] = Ininf[k];
@@ -1091,7 +1121,7 @@ __global__ void __launch_bounds__(kGroupTPB, 4) fit_multi_group_kernel(const uin
         MultiGroupEval<R, KIND, DIST, SUM2, G>{img2, w, part, lane, mask}, Ininf, hess, hess + P * P,
         hess + 2 * P * P, lane, mask);
     if (ll) {  // the lanes' pixel sums, combined in a fixed order
-        double s = model_loglik<R, KIND, DIST, SUM2>(img2, 1, Ininf, lane, G);
+        double s = model_loglik<R, KIND, DIST, SUM2>(PixView{img2, 1}, Ininf, lane, G);
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(mask, s, o, G);
         if (lane == 0) ll[CurFluoID] = s;

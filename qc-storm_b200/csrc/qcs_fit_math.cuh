@@ -940,12 +940,12 @@ __device__ __forceinline__ float model_value(float colpos, float rowpos, const f
 }
 
 // Unweighted Poisson log-likelihood of the model at the fitted parameters Ininf
-// over pixels k0, k0 + step, ... of the ROI (pixel k's (value, log) pair at
-// img[k * ld]): sum n ln(mu) - mu, accumulated in FP64 (the data's ln n!
-// term is common to every model of the ROI and left out).  The parameters are
-// clamped as the loss clamps them.
-template <int R, int KIND, int DIST, int SUM2>
-__device__ __forceinline__ double model_loglik(const float2 *img, int ld, const float *Ininf, int k0, int step) {
+// over pixels k0, k0 + step, ... of the ROI (pixel k's value at img[k]): sum n
+// ln(mu) - mu, accumulated in FP64 (the data's ln n! term is common to every
+// model of the ROI and left out).  The parameters are clamped as the loss
+// clamps them.
+template <int R, int KIND, int DIST, int SUM2, class View>
+__device__ __forceinline__ double model_loglik(const View &img, const float *Ininf, int k0, int step) {
     typedef KindTraits<KIND> T;
     float v[T::P];
 #pragma unroll
@@ -954,9 +954,88 @@ __device__ __forceinline__ double model_loglik(const float2 *img, int ld, const 
     for (int k = k0; k < R * R; k += step) {
         const int row = k / R, col = k - (k / R) * R;
         const double mu = (double)model_value<KIND, DIST, SUM2>(col + 0.5f, row + 0.5f, v);
-        s += (double)img[k * ld].x * log(mu) - mu;
+        s += (double)img[k] * log(mu) - mu;
     }
     return s;
+}
+
+// ------------------------------------------------------- packed pairs ---
+// Two floats in one 64-bit register pair.  The f32x2 instructions of sm_100
+// round each half as the scalar instruction does, at half the issue slots.
+// (A packed product whose only use is a packed sum is fused into one
+// multiply-add even with .rn on both, so no sum of that shape is written.)
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// e^x = 2^(x log2 e) and ln x = log2(x) ln 2 through the flushing base-2
+// instructions: without the scaling around subnormal results and arguments
+// that __expf and __logf carry (about 6.7 of the 22.8 instructions the loss
+// issued per pixel).  Where the result of exp and the argument of log are
+// normal the values are those of __expf and __logf bit for bit (every float
+// was compared); a subnormal exp is 0 here.  The loss takes this form only
+// where that changes no sum (flush_safe).
+__device__ __forceinline__ float ex2_flush(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float lg2_flush(float x) {
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ f32x2 ex2_flush2(f32x2 x) {
+    float a, b;
+    unpack2(x, a, b);
+    return pack2(ex2_flush(a), ex2_flush(b));
+}
+__device__ __forceinline__ f32x2 lg2_flush2(f32x2 x) {
+    float a, b;
+    unpack2(x, a, b);
+    return pack2(lg2_flush(a), lg2_flush(b));
+}
+constexpr float kLog2E = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
+
+// Whether the single-emitter loss at v (already clamped) is the same with the
+// flushing forms.  Either the background is large enough that a flushed exp
+// (below 2^-126) times the amplitude is under half a unit in the last place
+// of every pixel's model value, which then is the background in both forms
+// (and a normal number); or (GS2D, whose background may be clamped to zero)
+// no pixel's exponent reaches 2^-126 and the amplitude is at least one
+// photoelectron, so nothing is subnormal.  The distance of the farthest
+// corner bounds every pixel's exponent; 86 leaves its rounding below
+// 126 ln 2 = 87.3.  NaN parameters fail both or give NaN in both forms.
+template <int R, int KIND>
+__device__ __forceinline__ bool flush_safe(const float *v) {
+    const float A = v[0] * QCS_ASCALE, B = v[KindTraits<KIND>::P - 1] * QCS_BSCALE;
+    bool ok = B >= fmaxf(1e-30f, A * 0x1p-90f);
+    if (KIND == kGS2D) {
+        const float dx = fmaxf(fabsf(0.5f - v[1]), fabsf((R - 0.5f) - v[1]));
+        const float dy = fmaxf(fabsf(0.5f - v[2]), fabsf((R - 0.5f) - v[2]));
+        ok = ok || (A >= 1.0f && (dx * dx + dy * dy) * v[3] * QCS_SSCALE <= 86.0f);
+    }
+    return ok;
 }
 
 // ------------------------------------------ staged single-emitter eval ---
@@ -1013,24 +1092,16 @@ __device__ __forceinline__ float single_expo_d(float dx, float dy, const float *
     return __expf(-(sum_of_products<DIST>(dx * dx * v[3], QCS_SSCALE, dy * dy * v[4], QCS_SSCALE)));
 }
 
-// Loss and gradient of one single-emitter ROI (GS2D / AS3D) evaluated by its
-// own thread, with the pixels' (value, log) pairs at img[k * ld] and the
-// mask's unique values (MaskShape) at wu[(ur * C4 + c) * ld].  Same terms,
-// same order, same roundings as loss() / numerical_gradient_shared(), with
-// fewer instructions: one 16-byte mask load per row, the column offsets of
-// the position computed once per evaluation, the row centre kept as a float.
-template <int R, int KIND, int DIST, bool FULL = false>
-struct StagedEval {
-    typedef KindTraits<KIND> T;
+// A thread's weighted-MLE mask (MaskShape): unique values as float4 chunks at
+// ((const float4 *)mask)[(ur * C4 + c) * ld] (16-byte aligned), or (FULL) the
+// R x R values, pixel k at mask[k * ld].
+template <int R, bool FULL>
+struct MaskView {
     typedef MaskShape<R> M;
-    enum { P = T::P, UNROLL = R <= kUnrollMaxR };
-    const float2 *img;
-    // the mask: unique values as float4 chunks at ((const float4 *)mask)[(ur * C4 + c) * ld] (16-byte
-    // aligned), or (FULL) the R x R values, pixel k at mask[k * ld]
     const float *mask;
     int ld;
 
-    // the mask values of `row`, indexed by mirror_index(col) (FULL: by col)
+    // the mask values of `row`, indexed by wcol(col)
     __device__ __forceinline__ void mask_row(int row, float (&w)[FULL ? R : M::C4 * 4]) const {
         if constexpr (FULL) {
 #pragma unroll
@@ -1054,6 +1125,67 @@ struct StagedEval {
         const int ur = mirror_index(row, R), uc = mirror_index(col, R);
         return mask[((ur * M::C4 + uc / 4) * ld) * 4 + uc % 4];
     }
+};
+
+// The 2P central-difference points of the gradient at Ininf, as
+// numerical_gradient produces them (each loss call clamps its point in place
+// and the next point starts from the clamped values): v[2k] and v[2k + 1] are
+// parameter k's lower and upper point.  Returns whether the amplitude and
+// background points share the first point's exponent inputs bit for bit.
+template <int KIND>
+__device__ __forceinline__ bool gradient_points(const float *Ininf, float (&v)[2 * KindTraits<KIND>::P][KindTraits<KIND>::P]) {
+    typedef KindTraits<KIND> T;
+    enum { P = T::P, NE = 2 * P };
+    float t[P];
+#pragma unroll
+    for (int k = 0; k < P; k++) t[k] = Ininf[k];
+#pragma unroll
+    for (int k = 0; k < P; k++) {
+        t[k] = t[k] - 0.002f;
+#pragma unroll
+        for (int c = 0; c < P; c++) {
+            if (T::CLAMP001) { if (t[c] < 0.01f) t[c] = 0.01f; } else { if (t[c] < 0.0f) t[c] = 0.0f; }
+            v[2 * k][c] = t[c];
+        }
+        t[k] = t[k] + 0.004f;
+#pragma unroll
+        for (int c = 0; c < P; c++) {
+            if (T::CLAMP001) { if (t[c] < 0.01f) t[c] = 0.01f; } else { if (t[c] < 0.0f) t[c] = 0.0f; }
+            v[2 * k + 1][c] = t[c];
+        }
+        t[k] = t[k] - 0.002f;
+    }
+    bool share = true;
+#pragma unroll
+    for (int c = 1; c < P - 1; c++) {
+        const unsigned b = __float_as_uint(v[0][c]);
+        share = share && (__float_as_uint(v[1][c]) == b) && (__float_as_uint(v[NE - 2][c]) == b) &&
+                (__float_as_uint(v[NE - 1][c]) == b);
+    }
+    return share;
+}
+
+// Loss and gradient of one single-emitter ROI (GS2D / AS3D) evaluated by its
+// own thread, with the pixels' (value, log) pairs at img[k * ld] and the mask
+// of MaskView.  Same terms, same order, same roundings as loss() /
+// numerical_gradient_shared(), with fewer instructions: one 16-byte mask load
+// per row, the column offsets of the position computed once per evaluation,
+// the row centre kept as a float.  For the sizes whose distance rounding is
+// nvcc's (kCompiler); the others take PairEval.
+template <int R, int KIND, int DIST, bool FULL = false>
+struct StagedEval : MaskView<R, FULL> {
+    typedef KindTraits<KIND> T;
+    typedef MaskShape<R> M;
+    typedef MaskView<R, FULL> V;
+    using V::ld;
+    using V::mask_at;
+    using V::mask_row;
+    using V::wcol;
+    enum { P = T::P, UNROLL = R <= kUnrollMaxR };
+    const float2 *img;
+    __device__ __forceinline__ StagedEval(const float *pix, const float *mask_, int slot, int ld_)
+        : V{mask_, ld_}, img(reinterpret_cast<const float2 *>(pix) + slot) {}
+    __device__ __forceinline__ float2 pixel(int row, int col) const { return img[(row * R + col) * ld]; }
 
     __device__ __forceinline__ float loss(float *Ininf) const {
 #pragma unroll
@@ -1106,34 +1238,7 @@ struct StagedEval {
     __device__ __forceinline__ void gradient(const float *Ininf, float *grad) const {
         enum { NE = 2 * P };
         float v[NE][P];
-        {
-            float t[P];
-#pragma unroll
-            for (int k = 0; k < P; k++) t[k] = Ininf[k];
-#pragma unroll
-            for (int k = 0; k < P; k++) {
-                t[k] = t[k] - 0.002f;
-#pragma unroll
-                for (int c = 0; c < P; c++) {
-                    if (T::CLAMP001) { if (t[c] < 0.01f) t[c] = 0.01f; } else { if (t[c] < 0.0f) t[c] = 0.0f; }
-                    v[2 * k][c] = t[c];
-                }
-                t[k] = t[k] + 0.004f;
-#pragma unroll
-                for (int c = 0; c < P; c++) {
-                    if (T::CLAMP001) { if (t[c] < 0.01f) t[c] = 0.01f; } else { if (t[c] < 0.0f) t[c] = 0.0f; }
-                    v[2 * k + 1][c] = t[c];
-                }
-                t[k] = t[k] - 0.002f;
-            }
-        }
-        bool share = true;
-#pragma unroll
-        for (int c = 1; c < P - 1; c++) {
-            const unsigned b = __float_as_uint(v[0][c]);
-            share = share && (__float_as_uint(v[1][c]) == b) && (__float_as_uint(v[NE - 2][c]) == b) &&
-                    (__float_as_uint(v[NE - 1][c]) == b);
-        }
+        const bool share = gradient_points<KIND>(Ininf, v);
         if (!__all_sync(__activemask(), share)) {
             float tI[P];
 #pragma unroll
@@ -1176,14 +1281,260 @@ struct StagedEval {
     }
 };
 
+// Pixels of S slots (threads) for PairEval: per row R / 2 column pairs as
+// float4 (value, value, log, log), [row][pair][slot], then the last column's
+// (value, log) pairs, [row][slot]; 2 R^2 floats per slot in all.
+template <int R>
+struct PairPixels {
+    enum { NP = R / 2, SINGLES = R * NP * 4 };  // SINGLES: floats per slot before the last columns
+    __host__ __device__ static constexpr int value(int k, int slot, int S) {
+        const int row = k / R, col = k - (k / R) * R;
+        return col < 2 * NP ? ((row * NP + col / 2) * S + slot) * 4 + (col & 1) : SINGLES * S + (row * S + slot) * 2;
+    }
+    // offset of a pixel's log from its value
+    __host__ __device__ static constexpr int log_off(int k) { return k - (k / R) * R < 2 * NP ? 2 : 1; }
+};
+
+// StagedEval's loss and gradient with the pixels in column pairs (PairPixels)
+// and the arithmetic of a pair, or of a parameter's two difference points, in
+// packed instructions, exp and log in their flushing forms where flush_safe
+// says that this changes nothing.  Term for term the values of StagedEval.
+// StagedEval's sums are bound by the issue slots (22.8 instructions a pixel,
+// 85% issue, 61% of the special-function pipe); these issue 9.8 and are bound
+// by the special-function pipe (79%, two operations of 8 cycles a pixel and
+// warp).  100,000 fits in one launch: GS2D 7x7 715 -> 508 us, AS3D 9x9 1645 ->
+// 1214 us, GS2D 11x11 1823 -> 1292 us; 600,000 GS2D 7x7 3.72 -> 2.64 ms.  Of
+// the line search's evaluations 1.8% (GS2D) run in warps where some ROI is not
+// flush_safe (background clamped to zero) and take loss_general.
+// pix: this thread's slot of PairPixels, ld the slots.
+template <int R, int KIND, int DIST, bool FULL = false>
+struct PairEval : MaskView<R, FULL> {
+    typedef KindTraits<KIND> T;
+    typedef MaskShape<R> M;
+    typedef MaskView<R, FULL> V;
+    using V::ld;
+    using V::mask_row;
+    using V::wcol;
+    enum { P = T::P, NP = PairPixels<R>::NP, NW = FULL ? R : M::C4 * 4 };
+    static_assert(DIST == kFuseFirst || DIST == kFuseSecond, "a fixed distance rounding");
+    static_assert(KIND == kGS2D || DIST == kFuseFirst, "AS3D: the x term fused");
+    const float4 *pairs;
+    const float2 *last;
+    __device__ __forceinline__ PairEval(const float *pix, const float *mask_, int slot, int ld_)
+        : V{mask_, ld_}, pairs(reinterpret_cast<const float4 *>(pix) + slot),
+          last(reinterpret_cast<const float2 *>(pix + PairPixels<R>::SINGLES * ld_) + slot) {}
+    __device__ __forceinline__ float2 pixel(int row, int col) const {
+        if (col == R - 1) return last[row * ld];
+        const float4 q = pairs[(row * NP + col / 2) * ld];
+        return (col & 1) ? make_float2(q.y, q.w) : make_float2(q.x, q.z);
+    }
+
+    // the packed deviance terms of two pixels or points with models I
+    __device__ __forceinline__ static f32x2 terms(f32x2 I, f32x2 pix, f32x2 logpix, f32x2 nln2) {
+        // single_term's ln I - ln n is one fused multiply-add, lg2 I * ln 2 - ln n; here its negation
+        return fma2(pix, fma2(lg2_flush2(I), nln2, logpix), sub2(I, pix));
+    }
+
+    __device__ __forceinline__ float loss(float *v) const {
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            if (T::CLAMP001) {
+                if (v[k] < 0.01f) v[k] = 0.01f;
+            } else {
+                if (v[k] < 0.0f) v[k] = 0.0f;
+            }
+        }
+        if (!__all_sync(__activemask(), flush_safe<R, KIND>(v))) return loss_general(v);
+        const float A = v[0] * QCS_ASCALE, B = v[P - 1] * QCS_BSCALE;
+        const f32x2 A2 = pack2(A, A), B2 = pack2(B, B), nln2 = pack2(-kLn2, -kLn2);
+        const f32x2 s01 = pack2(QCS_SSCALE, QCS_SSCALE), l2e = pack2(kLog2E, kLog2E), nl2e = pack2(-kLog2E, -kLog2E);
+        const f32x2 nS = pack2(-v[3], -v[3]);
+        // the column's part of the exponent: dx, dx^2 or dx^2 Sx
+        float cx[R];
+#pragma unroll
+        for (int col = 0; col < R; col++) {
+            const float dx = (col + 0.5f) - v[1];
+            cx[col] = KIND == kAS3D ? __fmul_rn(__fmul_rn(dx, dx), v[3]) : (DIST == kFuseFirst ? dx : __fmul_rn(dx, dx));
+        }
+        float total = 0.0f, rowpos = 0.5f;
+        const float4 *pr = pairs;
+        const float2 *lr = last;
+        // rows overlap two at a time (7x7: all): 1-4% over one row at a time
+#pragma unroll(R <= 7 ? R : 2)
+        for (int row = 0; row < R; row++) {
+            float w[NW];
+            mask_row(row, w);
+            const float dy = rowpos - v[2];
+            const float ry = KIND == kAS3D ? __fmul_rn(__fmul_rn(__fmul_rn(dy, dy), v[P - 2]), QCS_SSCALE)
+                                           : (DIST == kFuseFirst ? __fmul_rn(dy, dy) : dy);
+            const f32x2 ry2 = pack2(ry, ry);
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                const float4 q = pr[p * ld];
+                const f32x2 c2 = pack2(cx[2 * p], cx[2 * p + 1]), pix = pack2(q.x, q.y), lp = pack2(q.z, q.w);
+                f32x2 t;
+                if (KIND == kAS3D)
+                    t = mul2(fma2(c2, s01, ry2), nl2e);
+                else
+                    t = mul2(mul2(mul2(DIST == kFuseFirst ? fma2(c2, c2, ry2) : fma2(ry2, ry2, c2), nS), s01), l2e);
+                float a, b;
+                unpack2(terms(fma2(A2, ex2_flush2(t), B2), pix, lp, nln2), a, b);
+                total = __fmaf_rn(w[wcol(2 * p)], a, total);
+                total = __fmaf_rn(w[wcol(2 * p + 1)], b, total);
+            }
+            {
+                const float2 q = lr[0];
+                float t;
+                if (KIND == kAS3D)
+                    t = __fmul_rn(__fmaf_rn(cx[R - 1], QCS_SSCALE, ry), -kLog2E);
+                else
+                    t = __fmul_rn(__fmul_rn(__fmul_rn(DIST == kFuseFirst ? __fmaf_rn(cx[R - 1], cx[R - 1], ry)
+                                                                         : __fmaf_rn(ry, ry, cx[R - 1]), -v[3]),
+                                            QCS_SSCALE), kLog2E);
+                const float I = __fmaf_rn(A, ex2_flush(t), B);
+                const float a = __fmaf_rn(lg2_flush(I), -kLn2, q.y);
+                total = __fmaf_rn(w[wcol(R - 1)], __fmaf_rn(q.x, a, __fsub_rn(I, q.x)), total);
+            }
+            rowpos += 1.0f;
+            pr += NP * ld;
+            lr += ld;
+        }
+        return total;
+    }
+
+    // the same loss with __expf and __logf, at a clamped v
+    __device__ __forceinline__ float loss_general(const float *v) const {
+        float dxs[R];
+#pragma unroll
+        for (int col = 0; col < R; col++) dxs[col] = (col + 0.5f) - v[1];
+        float total = 0.0f, rowpos = 0.5f;
+#pragma unroll 1
+        for (int row = 0; row < R; row++) {
+            float w[NW];
+            mask_row(row, w);
+            const float dy = rowpos - v[2];
+#pragma unroll
+            for (int col = 0; col < R; col++) {
+                const float2 pl = pixel(row, col);
+                total = __fmaf_rn(w[wcol(col)], single_term<KIND>(single_expo_d<KIND, DIST>(dxs[col], dy, v), v, pl.x, pl.y),
+                                  total);
+            }
+            rowpos += 1.0f;
+        }
+        return total;
+    }
+
+    // The central differences in one sweep over the pixels, the two points of a
+    // parameter in one packed value.  The amplitude's points have the same
+    // exponential, and so have the background's (the parameters between them
+    // are not moved back exactly, so the two differ): 2 (P - 1) exponentials a
+    // pixel instead of 2P.
+    __device__ __forceinline__ void gradient(const float *Ininf, float *grad) const {
+        enum { NE = 2 * P };
+        float v[NE][P];
+        gradient_points<KIND>(Ininf, v);
+        bool ok = true;
+#pragma unroll
+        for (int j = 0; j < NE; j++)
+            ok = ok && v[j][P - 1] * QCS_BSCALE >= fmaxf(1e-30f, v[j][0] * QCS_ASCALE * 0x1p-90f);  // flush_safe
+        if (!__all_sync(__activemask(), ok)) {
+            float tot[NE];
+#pragma unroll 1
+            for (int j = 0; j < NE; j++) {
+                float x[P];
+#pragma unroll
+                for (int c = 0; c < P; c++) {
+                    x[c] = v[0][c];
+#pragma unroll
+                    for (int i = 1; i < NE; i++) x[c] = j == i ? v[i][c] : x[c];
+                }
+                const float f = loss_general(x);
+#pragma unroll
+                for (int i = 0; i < NE; i++) tot[i] = j == i ? f : (j == 0 ? 0.0f : tot[i]);
+            }
+#pragma unroll
+            for (int k = 0; k < P; k++) grad[k] = (tot[2 * k + 1] - tot[2 * k]) * 250.0f;
+            return;
+        }
+        const f32x2 nln2 = pack2(-kLn2, -kLn2), s01 = pack2(QCS_SSCALE, QCS_SSCALE);
+        const f32x2 l2e = pack2(kLog2E, kLog2E), nl2e = pack2(-kLog2E, -kLog2E);
+        f32x2 tot[P], A2[P], B2[P];
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            tot[k] = pack2(0.0f, 0.0f);
+            A2[k] = pack2(v[2 * k][0] * QCS_ASCALE, v[2 * k + 1][0] * QCS_ASCALE);
+            B2[k] = pack2(v[2 * k][P - 1] * QCS_BSCALE, v[2 * k + 1][P - 1] * QCS_BSCALE);
+        }
+        // exponential pair q: the amplitude's and the background's (q = 0), else parameter q's two points
+        auto lo = [&](int q, int c) { return v[q == 0 ? 0 : 2 * q][c]; };
+        auto hi = [&](int q, int c) { return v[q == 0 ? NE - 1 : 2 * q + 1][c]; };
+        float rowpos = 0.5f;
+#pragma unroll 1
+        for (int row = 0; row < R; row++) {
+            float w[NW];
+            mask_row(row, w);
+            // the row's part of each exponent
+            auto row_part = [&](float y, float Sy) {
+                const float dy = rowpos - y;
+                return KIND == kAS3D ? __fmul_rn(__fmul_rn(__fmul_rn(dy, dy), Sy), QCS_SSCALE)
+                                     : (DIST == kFuseFirst ? __fmul_rn(dy, dy) : dy);
+            };
+            f32x2 ry[P - 1];
+#pragma unroll
+            for (int q = 0; q < P - 1; q++)
+                ry[q] = pack2(row_part(lo(q, 2), lo(q, P - 2)), row_part(hi(q, 2), hi(q, P - 2)));
+#pragma unroll
+            for (int col = 0; col < R; col++) {
+                const float2 pl = pixel(row, col);
+                const float wk = w[wcol(col)];
+                const f32x2 pix = pack2(pl.x, pl.x), lp = pack2(pl.y, pl.y), w2 = pack2(wk, wk);
+                f32x2 e[P - 1];
+#pragma unroll
+                for (int q = 0; q < P - 1; q++) {
+                    const f32x2 dx = pack2((col + 0.5f) - lo(q, 1), (col + 0.5f) - hi(q, 1));
+                    f32x2 t;
+                    if (KIND == kAS3D) {
+                        const f32x2 Sx = pack2(lo(q, 3), hi(q, 3));
+                        t = mul2(fma2(mul2(mul2(dx, dx), Sx), s01, ry[q]), nl2e);
+                    } else {
+                        const f32x2 nS = pack2(-lo(q, 3), -hi(q, 3));
+                        t = mul2(mul2(mul2(DIST == kFuseFirst ? fma2(dx, dx, ry[q]) : fma2(ry[q], ry[q], mul2(dx, dx)), nS),
+                                      s01), l2e);
+                    }
+                    e[q] = ex2_flush2(t);
+                }
+                float e_first, e_last;
+                unpack2(e[0], e_first, e_last);
+#pragma unroll
+                for (int k = 0; k < P; k++) {
+                    const f32x2 ek = k == 0 ? pack2(e_first, e_first) : (k == P - 1 ? pack2(e_last, e_last) : e[k]);
+                    tot[k] = fma2(w2, terms(fma2(A2[k], ek, B2[k]), pix, lp, nln2), tot[k]);
+                }
+            }
+            rowpos += 1.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            float n, p;
+            unpack2(tot[k], n, p);
+            grad[k] = (p - n) * 250.0f;
+        }
+    }
+};
+
+// The single-emitter evaluator of a thread: packed where the distance's
+// rounding is fixed in the source.
+template <int R, int DIST>
+constexpr bool kPaired = DIST != kCompiler && R <= kUnrollMaxR;
+
 // The learned-start single fit's loss and analytic gradient over the staged
 // layout of fit_single_kernel (pixels as (value, log) pairs, the mask's unique
 // values): StagedEval's loss, the gradient of AnalyticEvalGS2D /
 // AnalyticEvalAS3D term for term (the mask values are the same, so the
 // results are those of the full-mask evaluators).
-template <int R, int KIND, int DIST, bool FULL = false>
-struct StagedAnalyticEval : StagedEval<R, KIND, DIST, FULL> {
-    typedef StagedEval<R, KIND, DIST, FULL> B;
+template <int R, int KIND, class B, bool FULL>
+struct StagedAnalyticEval : B {
+    using B::B;
     __device__ __forceinline__ void gradient(const float *v, float *g) const {
         enum { NW = FULL ? R : B::M::C4 * 4 };
         if constexpr (KIND == kGS2D) {
@@ -1199,7 +1550,7 @@ struct StagedAnalyticEval : StagedEval<R, KIND, DIST, FULL> {
                 const float dy = (row + 0.5f) - c[2];
 #pragma unroll(R <= kUnrollMaxR ? R : 1)
                 for (int col = 0; col < R; col++) {
-                    const float2 pl = this->img[(row * R + col) * this->ld];
+                    const float2 pl = this->pixel(row, col);
                     const float w = wr[B::wcol(col)];
                     const float dx = (col + 0.5f) - c[1];
                     const float r2 = __fmaf_rn(dx, dx, dy * dy);
@@ -1234,7 +1585,7 @@ struct StagedAnalyticEval : StagedEval<R, KIND, DIST, FULL> {
                 const float qy = dy * dy;
 #pragma unroll(R <= kUnrollMaxR ? R : 1)
                 for (int col = 0; col < R; col++) {
-                    const float2 pl = this->img[(row * R + col) * this->ld];
+                    const float2 pl = this->pixel(row, col);
                     const float w = wr[B::wcol(col)];
                     const float dx = (col + 0.5f) - c[1];
                     const float qx = dx * dx;
