@@ -85,7 +85,7 @@ struct qcs_loc_data {
     int capture3 = 0;  // qcs_loc_set_three_emitter_capture
     const qcs::ThreeEmitterStart *three = nullptr;  // set for the duration of a learned call with a 3E net
     // autotuned lanes per ROI of the single-emitter fit by batch size: batches of
-    // at most tune_n[k] records use tune_lanes[k] (first match); none: 1
+    // at most tune_n[k] records use tune_lanes[k] (first match), larger ones 1; an empty table: by queue length
     int tune_count = 0;
     int tune_n[8] = {0};
     int tune_lanes[8] = {0};
@@ -318,7 +318,7 @@ static int ensure_three(qcs_loc_data *c) {
 static int tuned_lanes(const qcs_loc_data *c, int n) {
     for (int k = 0; k < c->tune_count; ++k)
         if (n <= c->tune_n[k]) return c->tune_lanes[k];
-    return 1;
+    return c->tune_count ? 1 : 0;  // longer than tuned: one thread per ROI; not tuned: by the queue's length
 }
 
 int qcs_loc_localize_device(qcs_loc_data *c, const uint16_t *d_rois, const float *d_wle, const qcs_loc_para *p,
@@ -742,7 +742,7 @@ int fit_from_start(qcs_loc_data *c, const uint16_t *d_rois, const float *d_wle, 
     QCS_CUDA(cudaStreamWaitEvent(c->side, c->ev_fork, 0), "fork");
     f.q = qcs::Queue{c->st.q_single, c->st.counters + qcs::kCntSingle, 0};
     f.stream = c->side;
-    QCS_CUDA(qcs::launch_fit_group(kind, p->ROISize, 8, f), "plain refit");
+    QCS_CUDA(qcs::launch_fit_group(kind, p->ROISize, 0, f), "plain refit");
     QCS_CUDA(qcs::launch_crlb(c->d_loc, c->st.counters + qcs::kCntSingle, 0, n, p->LocType, p->ReadNoise_e, p->QE,
                               p->PixelSize, c->side, c->st.q_single, nullptr),
              "refit CRLB");

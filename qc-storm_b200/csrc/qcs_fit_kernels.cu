@@ -48,6 +48,12 @@ struct PairView {
     __device__ __forceinline__ float operator[](int k) const { return p[PairPixels<R>::value(k, slot, ld)]; }
 };
 
+// Pixel values on their own, pixel k at p[k].
+struct ValueView {
+    const float *p;
+    __device__ __forceinline__ float operator[](int k) const { return p[k]; }
+};
+
 template <int R, int KIND>
 struct SmemLayout {
     enum {
@@ -110,8 +116,8 @@ __device__ __forceinline__ void edge_means(const View &img, float &Mean1, float 
 
 // Start positions of the extra emitters: the brightest (and for three
 // emitters also the second brightest) non-central block of a 3 x 3 tiling.
-template <int R>
-__device__ __forceinline__ void block_starts(const PixView &img, int nstart, float *xs, float *ys) {
+template <int R, class View>
+__device__ __forceinline__ void block_starts(const View &img, int nstart, float *xs, float *ys) {
     const int ROISize_Half = R / 2;
     const float ROICenter = R / 2.0f;
     const int SumROILen = R / 3 + 1;
@@ -452,10 +458,11 @@ template <int R, int KIND, bool WORDS, int DIST = ArithSpec<KIND, R>::DIST, int 
           bool FULL = MASK == kCompiler>
 __global__ void __launch_bounds__(kTPB, (SingleLayout<R, FULL>::BLOCKS)) fit_single_kernel(
     const uint16_t *__restrict__ rois, const float *__restrict__ wle, Queue q, float *__restrict__ loc,
-    uint8_t *__restrict__ to2e, CorePara c, double *__restrict__ ll) {
+    uint8_t *__restrict__ to2e, CorePara c, double *__restrict__ ll, int min_n) {
     extern __shared__ __align__(16) float smem[];
-    single_tile<R, KIND, WORDS, DIST, MASK, FULL, kTPB>(smem, blockIdx.x * kTPB, queue_len(q), rois, wle, q, loc,
-                                                         to2e, c, ll);
+    const int n = queue_len(q);
+    if (n <= min_n) return;  // a queue this short is the lane-group kernel's
+    single_tile<R, KIND, WORDS, DIST, MASK, FULL, kTPB>(smem, blockIdx.x * kTPB, n, rois, wle, q, loc, to2e, c, ll);
 }
 
 // ------------------------------------------------ mixed-size single fits ---
@@ -549,102 +556,12 @@ __global__ void __launch_bounds__(kTPB, kMixedBlocks) fit_mixed_kernel(const __g
     }
 }
 
-// The same fit with G lanes per ROI (GroupEval): bit for bit the rows of
-// fit_single_kernel, with about half the latency per ROI and about twice the
-// instructions.  For short queues (refits, small calls), where one thread
-// per ROI leaves the GPU mostly idle and the launch lasts as long as one
-// thread's serial fit.  Each ROI's pixels, weights and loss terms are
-// contiguous in shared memory (rows padded to 4 floats); D per lane.
 constexpr int kGroupTPB = 128;
-// Lanes per ROI of the multi-emitter group kernel: one central-difference
-// point per lane (2E: 16 points; 3E, AS3D-2E: 22 points).
-__host__ __device__ constexpr int multi_lanes(int kind) { return kind == k2E ? 16 : 32; }
-
-// Multi-emitter kinds and sizes whose roundings (pixel distance and the first
-// two emitters' model sum) are fixed in the source: there the group kernel's
-// rows equal the thread kernel's bit for bit.
+// Kinds and sizes whose roundings (pixel distance and the first two emitters'
+// model sum) are fixed in the source: there the lane-group kernel's rows equal
+// the thread kernels' bit for bit.
 __host__ __device__ constexpr bool multi_group_supported(int kind, int R) {
     return ((kind == k2E || kind == k3E) && (R == 7 || R == 11)) || (kind == kAS3D2E && R == 7);
-}
-
-template <int R, int KIND>
-struct GroupLayout {
-    enum {
-        P = KindTraits<KIND>::P,
-        PIX = R * R,
-        PIXP = (PIX + 3) / 4 * 4,
-    };
-    template <int G>
-    struct At {
-        enum {
-            SLOTS = kGroupTPB / G,
-            IMG = 0,                       // float2 per pixel
-            W = IMG + 2 * PIXP * SLOTS,    // floats
-            PART = W + PIXP * SLOTS,
-            D = PART + PIXP * SLOTS,
-            TOTAL = D + P * P * kGroupTPB,
-        };
-    };
-};
-
-template <int R, int KIND, int G, int DIST = ArithSpec<KIND, R>::DIST, int MASK = ArithSpec<KIND, R>::MASK>
-__global__ void __launch_bounds__(kGroupTPB) fit_single_group_kernel(const uint16_t *__restrict__ rois,
-                                                                     const float *__restrict__ wle, Queue q,
-                                                                     float *__restrict__ loc,
-                                                                     uint8_t *__restrict__ to2e, CorePara c) {
-    typedef GroupLayout<R, KIND> GL;
-    typedef typename GL::template At<G> L;
-    enum { P = KindTraits<KIND>::P, PIX = R * R, PIXP = GL::PIXP, WHOLE = R * (R + 1), SLOTS = L::SLOTS };
-    static_assert(G == 4 || G == 8 || G == 16, "lanes per ROI");
-    static_assert(DIST != kCompiler, "the group sums equal the thread kernel's only for a fixed distance rounding");
-    extern __shared__ __align__(16) float smem[];
-    const int n = queue_len(q);
-    const int base = blockIdx.x * SLOTS;
-    if (base >= n) return;
-    const int cnt = min(SLOTS, n - base);
-    float2 *s_img = reinterpret_cast<float2 *>(smem + L::IMG);
-    for (int idx = threadIdx.x; idx < cnt * PIX; idx += kGroupTPB) {
-        const int slot = idx / PIX;
-        const int k = idx - slot * PIX;
-        const int id = queue_at(q, base + slot);
-        const uint16_t u = __ldg(rois + (size_t)id * WHOLE + k);
-        const float pixval = fmaxf((u - c.Offset) * c.KAdc, 1.0f);
-        s_img[slot * PIXP + k] = make_float2(pixval, __logf(pixval));
-    }
-    __syncthreads();
-    const int slot = threadIdx.x / G;
-    const int lane = threadIdx.x % G;
-    if (slot >= cnt) return;
-    const unsigned mask = ((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
-
-    const int CurFluoID = queue_at(q, base + slot);
-    const float2 *img2 = s_img + slot * PIXP;
-    float *w = smem + L::W + slot * PIXP;
-    float *part = smem + L::PART + slot * PIXP;
-    float *D = smem + L::D + threadIdx.x;
-    const uint16_t *hdr = rois + (size_t)CurFluoID * WHOLE + PIX;
-    const int XOffset = hdr[0];
-    const int YOffset = hdr[1];
-    const int CurFrame = hdr[2] + 65536 * hdr[3];
-    const float *pw = wle + (size_t)CurFluoID * QCS_WLE_PARA_NUM;
-
-    float Ininf[P];
-    const SinglePrep sp = single_prefit<R, KIND>(PixView{img2, 1}, pw, c, Ininf);
-    if (lane == 0) wle_weights<R, MASK>(w, 1, sp.WLE_SigmaX, sp.WLE_SigmaY, sp.MoleculeType);
-    __syncwarp(mask);
-    bfgs_fit<P, KindTraits<KIND>::IT>(GroupEval<R, KIND, DIST, G>{img2, w, part, lane, mask}, Ininf, D, kGroupTPB);
-    float row[12];
-    bool accepted;
-    float CurSNR;
-    int IsFittingValid;
-    single_finish<R, KIND>(Ininf, c, sp.Simga_Max_Th, XOffset, YOffset, CurFrame, row, accepted, CurSNR,
-                           IsFittingValid);
-    if (lane != 0) return;
-    if (accepted)
-        store_row(loc, CurFluoID, row);
-    else
-        zero_row(loc, CurFluoID);
-    if (to2e) to2e[CurFluoID] = (!accepted && c.MultiEmitterFitEn && IsFittingValid && (CurSNR > 6.0f)) ? 1 : 0;
 }
 
 // ------------------------------------------- learned-start single fits ---
@@ -914,8 +831,8 @@ __device__ __forceinline__ void multi_finish(float *Ininf, const CorePara &c, in
 // AS3D_2Emitter_core.h:648-750) from the ROI's pixels, and the weighted-MLE
 // mask width of the 2E fit (a fixed R / 1.8 / 2.35, or R without WLE; the
 // other kinds are unweighted).
-template <int R, int KIND>
-__device__ __forceinline__ void multi_prefit(const PixView &img, const CorePara &c, float *Ininf, float &WLE_SigmaX) {
+template <int R, int KIND, class View>
+__device__ __forceinline__ void multi_prefit(const View &img, const CorePara &c, float *Ininf, float &WLE_SigmaX) {
     enum { ROISize_Half = R / 2 };
     const float ROICenter = R / 2.0f;
     WLE_SigmaX = R;
@@ -1037,15 +954,120 @@ __global__ void __launch_bounds__(kTPB) fit_multi_kernel(const uint16_t *__restr
     multi_finish<R, KIND>(Ininf, c, XOffset, YOffset, CurFrame, NearNeighborDistance, loc, CurFluoID, mo, slot);
 }
 
-// The multi-emitter fit of fit_multi_kernel with G lanes per ROI
-// (MultiGroupEval): bit for bit the same rows, stage results and second
-// emitters.  The thread kernel runs a stage's queue with one thread per ROI at
-// ~255 registers (two warps per SM), so a queue shorter than a wave (the
-// usual 2E / 3E queue) takes as long as one thread's whole fit; here a ROI's
-// pixel terms and gradient points are spread over G lanes.  Per slot: the
-// ROI's (value, log) pairs, its mask and loss terms contiguous (rows padded to
-// 4 floats), and one inverse Hessian with its update scratch and the search
-// direction, which the group's first lane alone updates (bfgs_fit_shared).
+// The fits of fit_single_kernel and fit_multi_kernel with G lanes per ROI
+// (LaneFit): bit for bit the same rows, stage results and second emitters.
+// For queues too short to fill the GPU with one thread per ROI, where that
+// launch lasts as long as one thread's whole fit.  Each group takes queue
+// entries g, g + groups, ... on its own (no block barrier after the table of
+// pixel centres); a queue outside min_n < n <= max_n (< 0: no bound) is
+// another launch's.
+template <int R, int KIND, int G>
+struct LaneShape {
+    typedef LaneLayout<R, KIND> L;
+    enum {
+        SLOTS = kGroupTPB / G,
+        // 16 banks apart, so that two groups of a warp read their rows without conflicts
+        STRIDE = (L::TOTAL + 15) / 32 * 32 + 16,
+        FLOATS = 2 * L::PIXP + STRIDE * SLOTS,
+        FIT = (228 * 1024) / (FLOATS * 4 + 1024),
+        BLOCKS = FIT < 4 ? FIT : 4,  // per SM: 128 registers a thread
+    };
+    static_assert((int)STRIDE >= (int)L::TOTAL, "a slot holds its layout");
+};
+
+template <int R, int KIND, int G, int DIST = ArithSpec<KIND, R>::DIST, int MASK = ArithSpec<KIND, R>::MASK,
+          int SUM2 = ArithSpec<KIND, R>::SUM2>
+__global__ void __launch_bounds__(kGroupTPB, (LaneShape<R, KIND, G>::BLOCKS)) fit_lanes_kernel(
+    const uint16_t *__restrict__ rois, const float *__restrict__ wle, Queue q, float *__restrict__ loc,
+    uint8_t *__restrict__ to2e, MultiOut mo, CorePara c, double *__restrict__ ll, int min_n, int max_n) {
+    typedef LaneLayout<R, KIND> L;
+    typedef LaneShape<R, KIND, G> S;
+    constexpr bool MULTI = Emitters<KIND>::M > 1;
+    enum { P = KindTraits<KIND>::P, PIX = R * R, WHOLE = R * (R + 1) };
+    static_assert(DIST != kCompiler && (!MULTI || SUM2 == kFuseFirst), "roundings fixed in the source");
+    extern __shared__ __align__(16) float smem[];
+    const int n = queue_len(q);
+    if (n <= min_n || (max_n >= 0 && n > max_n)) return;
+    float *pos = smem;
+    for (int k = threadIdx.x; k < L::PIXP; k += kGroupTPB) {
+        pos[k] = k % R + 0.5f;
+        pos[L::PIXP + k] = k / R + 0.5f;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x % G;
+    const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G % 32)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
+    float *s = smem + 2 * L::PIXP + threadIdx.x / G * S::STRIDE;
+    for (int slot = blockIdx.x * S::SLOTS + threadIdx.x / G; slot < n; slot += gridDim.x * S::SLOTS) {
+        const int CurFluoID = queue_at(q, slot);
+        const uint16_t *rec = rois + (size_t)CurFluoID * WHOLE;
+        for (int k = lane; k < L::PIXP; k += G) {
+            const float v = k < PIX ? fmaxf((__ldg(rec + k) - c.Offset) * c.KAdc, 1.0f) : 1.0f;
+            s[L::VAL + k] = v;
+            s[L::LOG + k] = __logf(v);
+        }
+        __syncwarp(mask);
+        const int XOffset = rec[PIX], YOffset = rec[PIX + 1];
+        const int CurFrame = rec[PIX + 2] + 65536 * rec[PIX + 3];
+        const float *pw = wle + (size_t)CurFluoID * QCS_WLE_PARA_NUM;
+        const ValueView view{s + L::VAL};
+        float x[P], sx = 0.0f, sy = 0.0f, sigma_th = 0.0f;
+        int type = QCS_MOLECULE_MULTIFIT;
+        if constexpr (MULTI) {
+            multi_prefit<R, KIND>(view, c, x, sx);
+            sy = sx;
+        } else {
+            const SinglePrep sp = single_prefit<R, KIND>(view, pw, c, x);
+            sx = sp.WLE_SigmaX;
+            sy = sp.WLE_SigmaY;
+            type = sp.MoleculeType;
+            sigma_th = sp.Simga_Max_Th;
+        }
+        if constexpr (KindTraits<KIND>::WEIGHTED) {
+            // where nvcc chooses the mask's contraction, its choice holds for this loop as a whole
+            if (MASK == kCompiler) {
+                if (lane == 0) wle_weights<R, MASK>(s + L::W, 1, sx, sy, type);
+            } else {
+                for (int k = lane; k < PIX; k += G) s[L::W + k] = wle_weight<R, MASK>(pos[k], pos[L::PIXP + k], sx, sy, type);
+            }
+            __syncwarp(mask);
+        }
+        LaneFit<R, KIND, DIST, G>{pos, s, lane, mask}.fit(x);
+        if (MULTI && ll) {  // the lanes' pixel sums, combined in a fixed order
+            double sum = model_loglik<R, KIND, DIST, SUM2>(view, x, lane, G);
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(mask, sum, o, G);
+            if (lane == 0) ll[CurFluoID] = sum;
+        }
+        if (lane == 0) {
+            if constexpr (MULTI) {
+                if (KIND == k3E && mo.params) {
+#pragma unroll
+                    for (int k = 0; k < P; k++) mo.params[(size_t)slot * P + k] = x[k];
+                }
+                // the 2E fit's selection reads the nearest-neighbour distance of the WLE pre-pass
+                multi_finish<R, KIND>(x, c, XOffset, YOffset, CurFrame, KIND == k2E ? pw[0] : 1000.0f, loc, CurFluoID,
+                                      mo, slot);
+            } else {
+                float row[12];
+                bool accepted;
+                float CurSNR;
+                int IsFittingValid;
+                single_finish<R, KIND>(x, c, sigma_th, XOffset, YOffset, CurFrame, row, accepted, CurSNR, IsFittingValid);
+                if (accepted)
+                    store_row(loc, CurFluoID, row);
+                else
+                    zero_row(loc, CurFluoID);
+                if (to2e)
+                    to2e[CurFluoID] = (!accepted && c.MultiEmitterFitEn && IsFittingValid && (CurSNR > 6.0f)) ? 1 : 0;
+            }
+        }
+        __syncwarp(mask);  // the slot's shared memory is free again
+    }
+}
+
+// Shared memory per slot of fit_learned_3e_warp_kernel: pixels, and one
+// inverse Hessian with its update scratch and the search direction, which lane
+// 0 alone updates (bfgs_fit_shared).
 template <int R, int KIND>
 struct MultiGroupLayout {
     enum {
@@ -1053,11 +1075,9 @@ struct MultiGroupLayout {
         PIX = R * R,
         PIXP = (PIX + 3) / 4 * 4,
         HP = (2 * P * P + P + 3) / 4 * 4,  // D, T and the direction per slot
-        SLOTS = kGroupTPB / multi_lanes(KIND),
+        SLOTS = kGroupTPB / 32,
         IMG = 0,                       // float2 per pixel
-        W = IMG + 2 * PIXP * SLOTS,    // floats
-        PART = W + PIXP * SLOTS,
-        H = PART + PIXP * SLOTS,
+        H = IMG + 2 * PIXP * SLOTS,
         TOTAL = H + HP * SLOTS,
     };
 };
@@ -1067,72 +1087,6 @@ struct MultiGroupLayout {
 // building both forms against the reference's multi-emitter cascades: only
 // the fused one gives their rows bit for bit).
 constexpr bool kSkskFused = true;
-
-template <int R, int KIND, int DIST = ArithSpec<KIND, R>::DIST, int MASK = ArithSpec<KIND, R>::MASK,
-          int SUM2 = ArithSpec<KIND, R>::SUM2>
-__global__ void __launch_bounds__(kGroupTPB, 4) fit_multi_group_kernel(const uint16_t *__restrict__ rois,
-                                                                    const float *__restrict__ wle, Queue q,
-                                                                    float *__restrict__ loc, MultiOut mo,
-                                                                    CorePara c, double *__restrict__ ll, int max_n) {
-    typedef MultiGroupLayout<R, KIND> L;
-    enum { G = multi_lanes(KIND), P = KindTraits<KIND>::P, PIX = R * R, PIXP = L::PIXP, WHOLE = R * (R + 1),
-           SLOTS = L::SLOTS };
-    static_assert(DIST != kCompiler && SUM2 != kCompiler, "the group sums equal the thread kernel's only for "
-                                                          "roundings fixed in the source");
-    extern __shared__ __align__(16) float smem[];
-    const int n = queue_len(q);
-    if (n > max_n) return;  // a longer queue is the one-thread-per-ROI kernel's
-    const int base = blockIdx.x * SLOTS;
-    if (base >= n) return;
-    const int cnt = min(SLOTS, n - base);
-    float2 *s_img = reinterpret_cast<float2 *>(smem + L::IMG);
-    for (int idx = threadIdx.x; idx < cnt * PIX; idx += kGroupTPB) {
-        const int sl = idx / PIX;
-        const int k = idx - sl * PIX;
-        const int id = queue_at(q, base + sl);
-        const uint16_t u = __ldg(rois + (size_t)id * WHOLE + k);
-        const float pixval = fmaxf((u - c.Offset) * c.KAdc, 1.0f);
-        s_img[sl * PIXP + k] = make_float2(pixval, __logf(pixval));
-    }
-    __syncthreads();
-    const int sl = threadIdx.x / G;
-    const int lane = threadIdx.x % G;
-    if (sl >= cnt) return;
-    const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G % 32)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
-
-    const int slot = base + sl;
-    const int CurFluoID = queue_at(q, slot);
-    const float2 *img2 = s_img + sl * PIXP;
-    float *w = smem + L::W + sl * PIXP;
-    float *part = smem + L::PART + sl * PIXP;
-    float *hess = smem + L::H + sl * L::HP;  // D (P x P), T (P x P), direction (P)
-    const uint16_t *hdr = rois + (size_t)CurFluoID * WHOLE + PIX;
-    const int XOffset = hdr[0];
-    const int YOffset = hdr[1];
-    const int CurFrame = hdr[2] + 65536 * hdr[3];
-    const float NearNeighborDistance = KIND == k2E ? wle[(size_t)CurFluoID * QCS_WLE_PARA_NUM + 0] : 1000.0f;
-
-    float Ininf[P];
-    float WLE_SigmaX;
-    multi_prefit<R, KIND>(PixView{img2, 1}, c, Ininf, WLE_SigmaX);
-    if (KIND == k2E && lane == 0) wle_weights<R, MASK>(w, 1, WLE_SigmaX, WLE_SigmaX, QCS_MOLECULE_MULTIFIT);
-    __syncwarp(mask);
-    bfgs_fit_shared<P, KindTraits<KIND>::IT, MultiGroupEval<R, KIND, DIST, SUM2, G>, kSkskFused>(
-        MultiGroupEval<R, KIND, DIST, SUM2, G>{img2, w, part, lane, mask}, Ininf, hess, hess + P * P,
-        hess + 2 * P * P, lane, mask);
-    if (ll) {  // the lanes' pixel sums, combined in a fixed order
-        double s = model_loglik<R, KIND, DIST, SUM2>(PixView{img2, 1}, Ininf, lane, G);
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(mask, s, o, G);
-        if (lane == 0) ll[CurFluoID] = s;
-    }
-    if (KIND == k3E && mo.params && lane == 0) {
-#pragma unroll
-        for (int k = 0; k < P; k++) mo.params[(size_t)slot * P + k] = Ininf[k];
-    }
-    if (lane == 0)
-        multi_finish<R, KIND>(Ininf, c, XOffset, YOffset, CurFrame, NearNeighborDistance, loc, CurFluoID, mo, slot);
-}
 
 // -------------------------------------- learned-start two-emitter fits ---
 // The GS2D two-emitter fit of fit_multi_kernel<R, k2E> over the records of
@@ -1448,7 +1402,7 @@ cudaError_t launch_learned_3e(const FitLaunch &a, const float *start, float dev_
 }
 
 template <int R, int KIND>
-cudaError_t launch_single(const FitLaunch &a) {
+cudaError_t launch_single(const FitLaunch &a, int min_n = -1) {
     const size_t smem = SingleLayout<R, ArithSpec<KIND, R>::MASK == kCompiler>::BYTES;
     // two pixels per load when every record starts on a 4-byte boundary
     auto k = (reinterpret_cast<uintptr_t>(a.rois) & 3) == 0 ? fit_single_kernel<R, KIND, true>
@@ -1457,53 +1411,70 @@ cudaError_t launch_single(const FitLaunch &a) {
     if (e != cudaSuccess) return e;
     const int grid = (a.max_count + kTPB - 1) / kTPB;
     if (grid == 0) return cudaSuccess;
-    k<<<grid, kTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.to2e, a.para, a.ll);
+    k<<<grid, kTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.to2e, a.para, a.ll, min_n);
     return cudaGetLastError();
 }
 
+// Queues of min_n < n <= max_n (< 0: any length) entries with G lanes per ROI.
 template <int R, int KIND, int G>
-cudaError_t launch_single_group(const FitLaunch &a) {
-    typedef typename GroupLayout<R, KIND>::template At<G> L;
-    const size_t smem = L::TOTAL * sizeof(float);
-    auto k = fit_single_group_kernel<R, KIND, G>;
+cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n) {
+    typedef LaneShape<R, KIND, G> S;
+    const size_t smem = S::FLOATS * sizeof(float);
+    auto k = fit_lanes_kernel<R, KIND, G>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int grid = (a.max_count + L::SLOTS - 1) / L::SLOTS;
-    if (grid == 0) return cudaSuccess;
-    k<<<grid, kGroupTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.to2e, a.para);
+    const long long most = max_n >= 0 && max_n < a.max_count ? max_n : a.max_count;
+    const long long need = (most + S::SLOTS - 1) / S::SLOTS;
+    const int grid = (int)(need < 148 * S::BLOCKS ? need : 148 * S::BLOCKS);
+    if (grid <= 0) return cudaSuccess;
+    k<<<grid, kGroupTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.to2e, a.mo, a.para, a.ll, min_n, max_n);
     return cudaGetLastError();
 }
 
-// Queue lengths up to which the lane-group kernel fits a multi-emitter stage:
-// about three waves of the ROIs it holds at once.  Beyond that the lanes'
-// repeated pixel sums cost more than the latency they save, and the
-// one-thread-per-ROI kernel (whose single wave holds far more ROIs) is faster.
+// The ROIs that G lanes each fit at once on the whole GPU.
+template <int R, int KIND, int G>
+constexpr int kLaneWave = 148 * (int)LaneShape<R, KIND, G>::BLOCKS * (int)LaneShape<R, KIND, G>::SLOTS;
+
+// A single-emitter queue by its length: as many lanes per ROI as fit the
+// whole queue at once (32, 16, at 7x7 also 8), beyond that one thread per ROI.
+// A wave costs one ROI's latency, which more lanes shorten; a second wave
+// costs it again, and past the narrowest wave the one-thread kernel, whose own
+// latency covers 18,944 ROIs, is as fast.  Fits of
+// n ROIs, us (one thread / 8 / 16 / 32 lanes): GS2D 7x7 1,000: 142 / 97 / 58 /
+// 40, 2,500: 142 / 105 / 71 / 79, 7,500: 143 / 132 / 140 / 167, 10,000: 144 /
+// 209 / 195 / 216; AS3D 9x9 1,000: 273 / 175 / 107 / 84, 5,000: 273 / 361 / 247
+// / 261, 7,500: 273 / 377 / 278 / 356.
+// The length is on the device unless a.exact: then every launch whose range
+// the queue can reach is made, and all but one return at once.
 template <int R, int KIND>
-int group_queue_limit() {
-    static int limit = -2;
-    if (limit == -2) {
-        typedef MultiGroupLayout<R, KIND> L;
-        int dev = 0, sms = 0, blocks = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(fit_multi_group_kernel<R, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(L::TOTAL * sizeof(float)));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fit_multi_group_kernel<R, KIND>, kGroupTPB,
-                                                      L::TOTAL * sizeof(float));
-        limit = 3 * sms * (blocks > 0 ? blocks : 1) * L::SLOTS;
-    }
-    return limit;
+cudaError_t launch_by_length(const FitLaunch &a) {
+    int done = 0;
+    cudaError_t e = cudaSuccess;
+    auto step = [&](auto width) {
+        constexpr int G = decltype(width)::value, wave = kLaneWave<R, KIND, G>;
+        if (e != cudaSuccess || a.max_count <= done) return;
+        if (!a.exact || a.max_count <= wave) e = launch_lanes<R, KIND, G>(a, done > 0 ? done : -1, wave);
+        done = wave;
+    };
+    step(std::integral_constant<int, 32>{});
+    step(std::integral_constant<int, 16>{});
+    if (R == 7) step(std::integral_constant<int, 8>{});
+    if (e != cudaSuccess || a.max_count <= done) return e;
+    return launch_single<R, KIND>(a, a.exact ? -1 : done);
 }
+
+// Longest multi-emitter queue that lane groups fit by default: the two- and
+// three-emitter stages of 100,000 1-3 emitter records of 7x7 (27,300 and 6,600
+// ROIs) take as long with lane groups as with one thread per ROI, shorter
+// queues and 11x11 ROIs up to ten times less (1,000 records of 7x7: the whole
+// call 257 us against 1,493 us; 20,000: 611 against 1,649; 11x11: 244 against
+// 1,156 and 808 against 3,396).
+constexpr int kGroupQueueLimit = 30000;
 
 }  // namespace
 
 int multi_group_default_limit(int kind, int R) {
-    if (kind == k2E && R == 7) return group_queue_limit<7, k2E>();
-    if (kind == k2E && R == 11) return group_queue_limit<11, k2E>();
-    if (kind == k3E && R == 7) return group_queue_limit<7, k3E>();
-    if (kind == k3E && R == 11) return group_queue_limit<11, k3E>();
-    if (kind == kAS3D2E && R == 7) return group_queue_limit<7, kAS3D2E>();
-    return 0;
+    return multi_group_supported(kind, R) ? kGroupQueueLimit : 0;
 }
 
 bool multi_group_available(int kind, int R) { return multi_group_supported(kind, R); }
@@ -1515,26 +1486,24 @@ namespace {
 template <int R, int KIND>
 cudaError_t launch_multi(const FitLaunch &a) {
     int min_n = -1;
+    cudaError_t e;
     if constexpr (multi_group_supported(KIND, R)) {
         if (!a.thread_per_roi) {
-            typedef MultiGroupLayout<R, KIND> L;
-            const size_t smem = L::TOTAL * sizeof(float);
-            auto k = fit_multi_group_kernel<R, KIND>;
-            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
             // group_limit > 0: tuned; < 0: one thread per ROI always; 0: the default
-            min_n = a.group_limit > 0 ? a.group_limit : (a.group_limit < 0 ? -1 : group_queue_limit<R, KIND>());
-            const int grid = (min(a.max_count, min_n) + L::SLOTS - 1) / L::SLOTS;
-            if (grid > 0) {
-                k<<<grid, kGroupTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.mo, a.para, a.ll, min_n);
-                if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            }
+            min_n = a.group_limit > 0 ? a.group_limit : (a.group_limit < 0 ? -1 : kGroupQueueLimit);
+            // a warp per ROI; at 7x7 half a warp beyond one wave of those (the sums, which every lane of a
+            // group repeats, are then shared by two ROIs); at 11x11 half the warps' shared memory would not fit
+            const int wave = R == 7 ? min(min_n, kLaneWave<R, KIND, 32>) : min_n;
+            if (min_n > 0 && (e = launch_lanes<R, KIND, 32>(a, -1, wave)) != cudaSuccess) return e;
+            if constexpr (R == 7)
+                if (min_n > wave && a.max_count > wave && (e = launch_lanes<R, KIND, 16>(a, wave, min_n)) != cudaSuccess)
+                    return e;
             if (a.max_count <= min_n) return cudaSuccess;  // the queue cannot outgrow the group kernel
         }
     }
     const size_t smem = SmemLayout<R, KIND>::TOTAL * sizeof(float);
     auto k = fit_multi_kernel<R, KIND>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int grid = (a.max_count + kTPB - 1) / kTPB;
     if (grid == 0) return cudaSuccess;
@@ -1677,19 +1646,22 @@ bool group_fit_supported(int kind, int R) {
 }
 
 cudaError_t launch_fit_group(int kind, int R, int lanes, const FitLaunch &a) {
-    if (!group_fit_supported(kind, R)) return cudaErrorInvalidValue;
+    if (!group_fit_supported(kind, R) || (lanes != 0 && lanes != 4 && lanes != 8 && lanes != 16))
+        return cudaErrorInvalidValue;
     const bool gs = kind == kGS2D;
-    if (lanes == 4 || lanes == 16) {
-        if (!gs || R != 7) return cudaErrorInvalidValue;
-        return lanes == 4 ? launch_single_group<7, kGS2D, 4>(a) : launch_single_group<7, kGS2D, 16>(a);
-    }
-    if (lanes != 8) return cudaErrorInvalidValue;
+    // at 7x7 fewer than 8 lanes are 8; the larger ROIs' terms leave room for 16 lanes a ROI at least
+#define QCS_LANES(RR)                                                                                         \
+    case RR:                                                                                                  \
+        if (lanes == 0) return gs ? launch_by_length<RR, kGS2D>(a) : launch_by_length<RR, kAS3D>(a);          \
+        if (RR == 7 && lanes <= 8) return gs ? launch_lanes<7, kGS2D, 8>(a, -1, -1) : launch_lanes<7, kAS3D, 8>(a, -1, -1); \
+        return gs ? launch_lanes<RR, kGS2D, 16>(a, -1, -1) : launch_lanes<RR, kAS3D, 16>(a, -1, -1);
     switch (R) {
-    case 7: return gs ? launch_single_group<7, kGS2D, 8>(a) : launch_single_group<7, kAS3D, 8>(a);
-    case 9: return gs ? launch_single_group<9, kGS2D, 8>(a) : launch_single_group<9, kAS3D, 8>(a);
-    case 11: return gs ? launch_single_group<11, kGS2D, 8>(a) : launch_single_group<11, kAS3D, 8>(a);
-    case 13: return launch_single_group<13, kGS2D, 8>(a);
+        QCS_LANES(7)
+        QCS_LANES(9)
+        QCS_LANES(11)
+    case 13: return lanes == 0 ? launch_by_length<13, kGS2D>(a) : launch_lanes<13, kGS2D, 16>(a, -1, -1);
     }
+#undef QCS_LANES
     return cudaErrorInvalidValue;
 }
 

@@ -549,128 +549,6 @@ struct AnalyticEval3E {
     }
 };
 
-// Loss and gradient of one single-emitter ROI (GS2D / AS3D) evaluated by a
-// group of G consecutive lanes of a warp, bit for bit equal to ThreadEval:
-//  - loss: the lanes compute the pixel terms k = lane, lane + G, ... (the
-//    same expressions as loss()) into the ROI's scratch row; then every lane
-//    accumulates the row in pixel order with the same fused multiply-adds,
-//    so all lanes hold the serial sum;
-//  - gradient: the 2P central-difference points are replayed as
-//    numerical_gradient does (in-place clamping); lane l accumulates the
-//    sums of points l, l + G, ... over all pixels in pixel order.  Each
-//    point evaluates its own exponential, which equals the shared one of
-//    numerical_gradient_shared whenever that one applies.
-// img / w / part: the ROI's PIX (value, log) pairs, weights and scratch,
-// contiguous and 16-byte aligned; mask: the group's lanes.  The sums equal
-// the serial kernel's only where the pixel distance's contraction is fixed in
-// the source (DIST != kCompiler).
-template <int R, int KIND, int DIST, int G>
-struct GroupEval {
-    const float2 *img;
-    const float *w;
-    float *part;
-    int lane;
-    unsigned mask;
-
-    __device__ __forceinline__ float loss(float *Ininf) const {
-        typedef KindTraits<KIND> T;
-        enum { PIX = R * R };
-#pragma unroll
-        for (int k = 0; k < T::P; k++) {
-            if (T::CLAMP001) {
-                if (Ininf[k] < 0.01f) Ininf[k] = 0.01f;
-            } else {
-                if (Ininf[k] < 0.0f) Ininf[k] = 0.0f;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < (PIX + G - 1) / G; i++) {
-            const int k = lane + i * G;
-            if (k < PIX) {
-                const int row = k / R, col = k - (k / R) * R;
-                const float2 pl = img[k];
-                part[k] = single_term<KIND>(single_expo<KIND, DIST>(col + 0.5f, row + 0.5f, Ininf), Ininf, pl.x,
-                                            pl.y);
-            }
-        }
-        __syncwarp(mask);
-        float TotalLoss = 0;
-        const float4 *w4 = reinterpret_cast<const float4 *>(w);
-        const float4 *p4 = reinterpret_cast<const float4 *>(part);
-#pragma unroll
-        for (int q = 0; q < PIX / 4; q++) {
-            const float4 a = w4[q], t = p4[q];
-            TotalLoss = __fmaf_rn(a.x, t.x, TotalLoss);
-            TotalLoss = __fmaf_rn(a.y, t.y, TotalLoss);
-            TotalLoss = __fmaf_rn(a.z, t.z, TotalLoss);
-            TotalLoss = __fmaf_rn(a.w, t.w, TotalLoss);
-        }
-#pragma unroll
-        for (int k = PIX / 4 * 4; k < PIX; k++) TotalLoss = __fmaf_rn(w[k], part[k], TotalLoss);
-        __syncwarp(mask);
-        return TotalLoss;
-    }
-
-    __device__ __forceinline__ void gradient(const float *Ininf, float *grad) const {
-        typedef KindTraits<KIND> T;
-        enum { P = T::P, NE = 2 * P, NC = (NE + G - 1) / G, PIX = R * R };
-        float v[NC][P] = {};
-        {
-            float t[P];
-#pragma unroll
-            for (int k = 0; k < P; k++) t[k] = Ininf[k];
-#pragma unroll
-            for (int k = 0; k < P; k++) {
-                t[k] = t[k] - 0.002f;
-#pragma unroll
-                for (int c = 0; c < P; c++) {
-                    if (T::CLAMP001) { if (t[c] < 0.01f) t[c] = 0.01f; } else { if (t[c] < 0.0f) t[c] = 0.0f; }
-                }
-#pragma unroll
-                for (int j = 0; j < NC; j++)
-                    if (lane + j * G == 2 * k)
-#pragma unroll
-                        for (int c = 0; c < P; c++) v[j][c] = t[c];
-                t[k] = t[k] + 0.004f;
-#pragma unroll
-                for (int c = 0; c < P; c++) {
-                    if (T::CLAMP001) { if (t[c] < 0.01f) t[c] = 0.01f; } else { if (t[c] < 0.0f) t[c] = 0.0f; }
-                }
-#pragma unroll
-                for (int j = 0; j < NC; j++)
-                    if (lane + j * G == 2 * k + 1)
-#pragma unroll
-                        for (int c = 0; c < P; c++) v[j][c] = t[c];
-                t[k] = t[k] - 0.002f;
-            }
-        }
-        float tot[NC];
-#pragma unroll
-        for (int j = 0; j < NC; j++) tot[j] = 0;
-#pragma unroll 1
-        for (int row = 0; row < R; row++) {
-#pragma unroll(R <= kUnrollMaxR ? R : 1)
-            for (int col = 0; col < R; col++) {
-                const float2 pl = img[row * R + col];
-                const float wk = w[row * R + col];
-#pragma unroll
-                for (int j = 0; j < NC; j++) {
-                    if (lane + j * G < NE) {
-                        const float e = single_expo<KIND, DIST>(col + 0.5f, row + 0.5f, v[j]);
-                        tot[j] = __fmaf_rn(wk, single_term<KIND>(e, v[j], pl.x, pl.y), tot[j]);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < P; k++) {
-            const float tn = __shfl_sync(mask, tot[(2 * k) / G], (2 * k) % G, G);
-            const float tp = __shfl_sync(mask, tot[(2 * k + 1) / G], (2 * k + 1) % G, G);
-            grad[k] = (tp - tn) * 250.0f;
-        }
-    }
-};
-
 // Poisson deviance term of one pixel of the multi-emitter kinds at the
 // parameters v: the expressions of loss(), term for term.
 template <int KIND, int DIST, int SUM2>
@@ -772,139 +650,6 @@ struct AnalyticWarpEval3E {
     }
 };
 
-// Loss and gradient of one multi-emitter ROI (2E, 3E, AS3D-2E) evaluated by
-// a group of G consecutive lanes, bit for bit equal to ThreadEval:
-//  - loss: lane l computes the pixel terms k = l, l + G, ... (multi_term)
-//    into the ROI's scratch row; then every lane sums the row in pixel order
-//    with the thread kernel's operations (the weighted 2E fit: fused
-//    multiply-adds with the mask; 3E and AS3D-2E: plain adds);
-//  - gradient: the 2P central-difference points are replayed as
-//    numerical_gradient produces them (each loss call clamps its point in
-//    place and the next point starts from the clamped values); lane l sums
-//    points l, l + G, ... over all pixels in pixel order, and the lanes
-//    exchange the sums.
-// img / w / part: the ROI's pixels, mask and scratch, contiguous and 16-byte
-// aligned; mask: the group's lanes.  Only for roundings fixed in the source
-// (DIST, SUM2 != kCompiler).
-template <int R, int KIND, int DIST, int SUM2, int G>
-struct MultiGroupEval {
-    const float2 *img;
-    const float *w;
-    float *part;
-    int lane;
-    unsigned mask;
-
-    __device__ __forceinline__ float loss(float *Ininf) const {
-        typedef KindTraits<KIND> T;
-        enum { PIX = R * R };
-#pragma unroll
-        for (int k = 0; k < T::P; k++) {
-            if (T::CLAMP001) {
-                if (Ininf[k] < 0.01f) Ininf[k] = 0.01f;
-            } else {
-                if (Ininf[k] < 0.0f) Ininf[k] = 0.0f;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < (PIX + G - 1) / G; i++) {
-            const int k = lane + i * G;
-            if (k < PIX) {
-                const int row = k / R, col = k - (k / R) * R;
-                const float2 pl = img[k];
-                part[k] = multi_term<KIND, DIST, SUM2>(col + 0.5f, row + 0.5f, Ininf, pl.x, pl.y);
-            }
-        }
-        __syncwarp(mask);
-        float TotalLoss = 0;
-        const float4 *p4 = reinterpret_cast<const float4 *>(part);
-        if (T::WEIGHTED) {
-            const float4 *w4 = reinterpret_cast<const float4 *>(w);
-#pragma unroll 8
-            for (int q = 0; q < PIX / 4; q++) {
-                const float4 a = w4[q], t = p4[q];
-                TotalLoss = __fmaf_rn(a.x, t.x, TotalLoss);
-                TotalLoss = __fmaf_rn(a.y, t.y, TotalLoss);
-                TotalLoss = __fmaf_rn(a.z, t.z, TotalLoss);
-                TotalLoss = __fmaf_rn(a.w, t.w, TotalLoss);
-            }
-#pragma unroll
-            for (int k = PIX / 4 * 4; k < PIX; k++) TotalLoss = __fmaf_rn(w[k], part[k], TotalLoss);
-        } else {
-#pragma unroll 8
-            for (int q = 0; q < PIX / 4; q++) {
-                const float4 t = p4[q];
-                TotalLoss = __fadd_rn(TotalLoss, t.x);
-                TotalLoss = __fadd_rn(TotalLoss, t.y);
-                TotalLoss = __fadd_rn(TotalLoss, t.z);
-                TotalLoss = __fadd_rn(TotalLoss, t.w);
-            }
-#pragma unroll
-            for (int k = PIX / 4 * 4; k < PIX; k++) TotalLoss = __fadd_rn(TotalLoss, part[k]);
-        }
-        __syncwarp(mask);
-        return TotalLoss;
-    }
-
-    __device__ __forceinline__ void gradient(const float *Ininf, float *grad) const {
-        typedef KindTraits<KIND> T;
-        enum { P = T::P, NE = 2 * P, NC = (NE + G - 1) / G, PIX = R * R };
-        float v[NC][P] = {};
-        {
-            float t[P];
-#pragma unroll
-            for (int k = 0; k < P; k++) t[k] = Ininf[k];
-#pragma unroll
-            for (int k = 0; k < P; k++) {
-                t[k] = t[k] - 0.002f;
-#pragma unroll
-                for (int c = 0; c < P; c++) {
-                    if (T::CLAMP001) { if (t[c] < 0.01f) t[c] = 0.01f; } else { if (t[c] < 0.0f) t[c] = 0.0f; }
-                }
-#pragma unroll
-                for (int j = 0; j < NC; j++)
-                    if (lane + j * G == 2 * k)
-#pragma unroll
-                        for (int c = 0; c < P; c++) v[j][c] = t[c];
-                t[k] = t[k] + 0.004f;
-#pragma unroll
-                for (int c = 0; c < P; c++) {
-                    if (T::CLAMP001) { if (t[c] < 0.01f) t[c] = 0.01f; } else { if (t[c] < 0.0f) t[c] = 0.0f; }
-                }
-#pragma unroll
-                for (int j = 0; j < NC; j++)
-                    if (lane + j * G == 2 * k + 1)
-#pragma unroll
-                        for (int c = 0; c < P; c++) v[j][c] = t[c];
-                t[k] = t[k] - 0.002f;
-            }
-        }
-        float tot[NC];
-#pragma unroll
-        for (int j = 0; j < NC; j++) tot[j] = 0;
-#pragma unroll 1
-        for (int row = 0; row < R; row++) {
-#pragma unroll(R <= kUnrollMaxR ? R : 1)
-            for (int col = 0; col < R; col++) {
-                const float2 pl = img[row * R + col];
-                const float wk = T::WEIGHTED ? w[row * R + col] : 1.0f;
-#pragma unroll
-                for (int j = 0; j < NC; j++) {
-                    if (lane + j * G < NE) {
-                        const float Lt = multi_term<KIND, DIST, SUM2>(col + 0.5f, row + 0.5f, v[j], pl.x, pl.y);
-                        tot[j] = T::WEIGHTED ? __fmaf_rn(wk, Lt, tot[j]) : __fadd_rn(tot[j], Lt);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < P; k++) {
-            const float tn = __shfl_sync(mask, tot[(2 * k) / G], (2 * k) % G, G);
-            const float tp = __shfl_sync(mask, tot[(2 * k + 1) / G], (2 * k + 1) % G, G);
-            grad[k] = (tp - tn) * 250.0f;
-        }
-    }
-};
-
 // Expected photoelectrons of pixel (colpos, rowpos) under the model at the
 // parameters v (fit units): the model value of loss(), expression for
 // expression.
@@ -982,6 +727,12 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+// (not for a product: see above)
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
     f32x2 d;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -1037,6 +788,404 @@ __device__ __forceinline__ bool flush_safe(const float *v) {
     }
     return ok;
 }
+
+// ------------------------------------------------------- lane-group fits ---
+// Emitters of a kind, and the parameter indices of emitter m's amplitude, x,
+// y and widths (Sx = Sy where the kind has one).
+template <int KIND>
+struct Emitters {
+    enum { AS = KIND == kAS3D || KIND == kAS3D2E, M = KIND == k3E ? 3 : ((KIND == k2E || KIND == kAS3D2E) ? 2 : 1) };
+    __host__ __device__ static constexpr int a(int m) { return m * (AS ? 5 : 3); }
+    __host__ __device__ static constexpr int x(int m) { return a(m) + 1; }
+    __host__ __device__ static constexpr int y(int m) { return a(m) + 2; }
+    __host__ __device__ static constexpr int sx(int m) { return AS ? a(m) + 3 : KindTraits<KIND>::P - 2; }
+    __host__ __device__ static constexpr int sy(int m) { return AS ? a(m) + 4 : KindTraits<KIND>::P - 2; }
+    // whether parameter k enters emitter m's exponent
+    __host__ __device__ static constexpr bool in(int m, int k) { return k == x(m) || k == y(m) || k == sx(m) || k == sy(m); }
+};
+
+// Shared memory of one ROI of a lane group (floats): the pixels' values, then
+// their logs, mask (weighted kinds), loss terms [point][pixel], inverse
+// Hessian, its update's left product and two parameter vectors.  Pixel rows
+// are padded to 4 floats.
+template <int R, int KIND>
+struct LaneLayout {
+    enum {
+        P = KindTraits<KIND>::P,
+        PIX = R * R,
+        PIXP = (PIX + 3) / 4 * 4,
+        VAL = 0,
+        LOG = VAL + PIXP,
+        W = LOG + PIXP,
+        PART = W + (KindTraits<KIND>::WEIGHTED ? PIXP : 0),
+        H = PART + 2 * P * PIXP,
+        T = H + P * P,
+        VEC = T + P * P,
+        TOTAL = (VEC + 2 * P + 3) / 4 * 4,
+    };
+};
+
+// One ROI's fit by a group of G consecutive lanes of a warp, the rows of the
+// one-thread kernels bit for bit: every term, every sum's order and every
+// rounding is theirs; the lanes only divide the work.
+//  - Line search: the next midpoint and the one after it do not depend on the
+//    comparison between them, and the third has two candidates, so one round
+//    evaluates three steps: 4 points on G / 4 lanes each (first the ends and
+//    the first midpoint), then the lanes 0..3 sum one point's terms each, in
+//    pixel order.  The 12 evaluations one after the other take 4 rounds.
+//  - Gradient: a lane computes its pixels' terms at all 2P difference points,
+//    each distinct exponential once (a parameter's two points differ only in
+//    that parameter, and after it is moved back its rounded value stays: 26
+//    exponentials instead of 66 for three emitters), then lane j sums point j.
+//  - The inverse Hessian's update: one element per lane and round.
+// A line-search term takes two pixels at a time in packed instructions.
+// Only for roundings fixed in the source (DIST, SUM2 != kCompiler).  pos: the
+// pixels' centres, col + 0.5 of PIXP pixels, then row + 0.5.
+template <int R, int KIND, int DIST, int G>
+struct LaneFit {
+    typedef KindTraits<KIND> T;
+    typedef Emitters<KIND> E;
+    typedef LaneLayout<R, KIND> L;
+    enum { P = T::P, NE = 2 * P, PIX = R * R, PIXP = L::PIXP, KPTS = 4, LP = G / KPTS, LOW = T::CLAMP001 };
+    const float *pos;
+    float *s;  // the ROI's LaneLayout
+    int lane;
+    unsigned mask;
+
+    __device__ __forceinline__ static float bound(float v) {
+        if (LOW) return v < 0.01f ? 0.01f : v;
+        return v < 0.0f ? 0.0f : v;
+    }
+    // The flushing forms change nothing at clamped parameters with this
+    // background and sum of amplitudes: an exp below 2^-126 times its amplitude
+    // is lost under the background also in the partial sums of the model
+    // (flush_safe).
+    __device__ __forceinline__ static bool safe(float B, float sumA) {
+        return B * QCS_BSCALE >= fmaxf(1e-30f, sumA * QCS_ASCALE * 0x1p-45f);
+    }
+    __device__ __forceinline__ static float exponent(float cp, float rp, float x, float y, float sx, float sy) {
+        const float dx = cp - x, dy = rp - y;
+        if (E::AS) return -sum_of_products<DIST>(__fmul_rn(__fmul_rn(dx, dx), sx), QCS_SSCALE,
+                                                 __fmul_rn(__fmul_rn(dy, dy), sy), QCS_SSCALE);
+        return __fmul_rn(__fmul_rn(-sum_of_products<DIST>(dx, dx, dy, dy), sx), QCS_SSCALE);
+    }
+    __device__ __forceinline__ static float expo(float cp, float rp, float x, float y, float sx, float sy) {
+        return ex2_flush(__fmul_rn(exponent(cp, rp, x, y, sx, sy), kLog2E));
+    }
+    // deviance term from the emitters' exponentials e and amplitudes A, and the background B (fit units)
+    __device__ __forceinline__ static float term(const float (&e)[E::M], const float (&A)[E::M], float B, float2 pl) {
+        float I;
+        if (E::M == 1) {
+            I = __fmaf_rn(A[0] * QCS_ASCALE, e[0], B * QCS_BSCALE);
+        } else {
+            I = __fmaf_rn(A[0] * QCS_ASCALE, e[0], __fmul_rn(A[E::M > 1 ? 1 : 0] * QCS_ASCALE, e[E::M > 1 ? 1 : 0]));
+            if (E::M > 2) I = __fmaf_rn(A[E::M - 1] * QCS_ASCALE, e[E::M - 1], I);
+            I = __fadd_rn(I, B * QCS_BSCALE);
+        }
+        return __fmaf_rn(pl.x, __fmaf_rn(lg2_flush(I), -kLn2, pl.y), __fsub_rn(I, pl.x));
+    }
+    // pixel k's term as the one-thread kernels form it, with __expf and __logf
+    __device__ __forceinline__ float term_general(int k, const float *v) const {
+        const float cp = pos[k], rp = pos[PIXP + k], pix = s[L::VAL + k], lg = s[L::LOG + k];
+        if constexpr (E::M == 1)
+            return single_term<KIND>(single_expo<KIND, DIST>(cp, rp, v), v, pix, lg);
+        else
+            return multi_term<KIND, DIST, kFuseFirst>(cp, rp, v, pix, lg);
+    }
+    __device__ __forceinline__ static f32x2 pair_at(const float *p) { return *reinterpret_cast<const f32x2 *>(p); }
+    // expo and term of two pixels
+    __device__ __forceinline__ static f32x2 expo2(f32x2 cp, f32x2 rp, f32x2 x, f32x2 y, f32x2 sx, f32x2 sy) {
+        const f32x2 s01 = pack2(QCS_SSCALE, QCS_SSCALE), dx = sub2(cp, x), dy = sub2(rp, y);
+        f32x2 t;
+        if (E::AS) {
+            t = mul2(fma2(mul2(mul2(dx, dx), sx), s01, mul2(mul2(mul2(dy, dy), sy), s01)), pack2(-kLog2E, -kLog2E));
+        } else {
+            // -d S: sx is -S
+            const f32x2 d = DIST == kFuseFirst ? fma2(dx, dx, mul2(dy, dy)) : fma2(dy, dy, mul2(dx, dx));
+            t = mul2(mul2(mul2(d, sx), s01), pack2(kLog2E, kLog2E));
+        }
+        return ex2_flush2(t);
+    }
+    __device__ __forceinline__ static f32x2 term2(const f32x2 (&e)[E::M], const f32x2 (&A)[E::M], f32x2 B, f32x2 pix,
+                                                  f32x2 lg) {
+        f32x2 I;
+        if (E::M == 1) {
+            I = fma2(A[0], e[0], B);
+        } else {
+            I = fma2(A[0], e[0], mul2(A[E::M > 1 ? 1 : 0], e[E::M > 1 ? 1 : 0]));
+            if (E::M > 2) I = fma2(A[E::M - 1], e[E::M - 1], I);
+            I = add2(I, B);
+        }
+        return fma2(pix, fma2(lg2_flush2(I), pack2(-kLn2, -kLn2), lg), sub2(I, pix));
+    }
+
+    // Sum of term row j (PIX terms in pixel order, with the mask where the kind is weighted).
+    __device__ __forceinline__ float row_sum(int j) const {
+        const float4 *p4 = reinterpret_cast<const float4 *>(s + L::PART + j * PIXP);
+        const float4 *w4 = reinterpret_cast<const float4 *>(s + L::W);
+        float total = 0.0f;
+#pragma unroll(PIX <= 49 ? PIX / 4 : 8)
+        for (int q = 0; q < PIX / 4; q++) {
+            const float4 t = p4[q];
+            if (T::WEIGHTED) {
+                const float4 a = w4[q];
+                total = __fmaf_rn(a.x, t.x, total);
+                total = __fmaf_rn(a.y, t.y, total);
+                total = __fmaf_rn(a.z, t.z, total);
+                total = __fmaf_rn(a.w, t.w, total);
+            } else {
+                total = __fadd_rn(total, t.x);
+                total = __fadd_rn(total, t.y);
+                total = __fadd_rn(total, t.z);
+                total = __fadd_rn(total, t.w);
+            }
+        }
+#pragma unroll
+        for (int k = PIX / 4 * 4; k < PIX; k++) {
+            const float t = s[L::PART + j * PIXP + k];
+            total = T::WEIGHTED ? __fmaf_rn(s[L::W + k], t, total) : __fadd_rn(total, t);
+        }
+        return total;
+    }
+
+    // Losses at x + d * step[j], j < KPTS, in every lane.
+    __device__ __forceinline__ void losses(const float *x, const float *d, const float (&step)[KPTS],
+                                           float (&f)[KPTS]) const {
+        const int j = lane / LP, k0 = lane - j * LP;
+        float st = step[0];
+#pragma unroll
+        for (int i = 1; i < KPTS; i++) st = j == i ? step[i] : st;
+        float v[P], A[E::M], sumA = 0.0f;
+#pragma unroll
+        for (int k = 0; k < P; k++) v[k] = bound(__fmaf_rn(d[k], st, x[k]));
+#pragma unroll
+        for (int m = 0; m < E::M; m++) {
+            A[m] = v[E::a(m)];
+            sumA += A[m];
+        }
+        float *part = s + L::PART + j * PIXP;
+        if (__all_sync(mask, safe(v[P - 1], sumA))) {
+            f32x2 A2[E::M], x2[E::M], y2[E::M], sx2[E::M], sy2[E::M];
+            const f32x2 B2 = pack2(v[P - 1] * QCS_BSCALE, v[P - 1] * QCS_BSCALE);
+#pragma unroll
+            for (int m = 0; m < E::M; m++) {
+                const float sx = E::AS ? v[E::sx(m)] : -v[E::sx(m)], sy = v[E::sy(m)];
+                A2[m] = pack2(A[m] * QCS_ASCALE, A[m] * QCS_ASCALE);
+                x2[m] = pack2(v[E::x(m)], v[E::x(m)]);
+                y2[m] = pack2(v[E::y(m)], v[E::y(m)]);
+                sx2[m] = pack2(sx, sx);
+                sy2[m] = pack2(sy, sy);
+            }
+// (unrolled rounds are slower: the loop is short and the kernel is bound by instruction fetch as well)
+#pragma unroll 1
+            for (int k = 2 * k0; k < PIX; k += 2 * LP) {
+                const f32x2 cp = pair_at(pos + k), rp = pair_at(pos + PIXP + k);
+                f32x2 e[E::M];
+#pragma unroll
+                for (int m = 0; m < E::M; m++) e[m] = expo2(cp, rp, x2[m], y2[m], sx2[m], sy2[m]);
+                *reinterpret_cast<f32x2 *>(part + k) = term2(e, A2, B2, pair_at(s + L::VAL + k), pair_at(s + L::LOG + k));
+            }
+        } else {
+#pragma unroll 1
+            for (int k = k0; k < PIX; k += LP) part[k] = term_general(k, v);
+        }
+        __syncwarp(mask);
+        const float total = row_sum(lane & (KPTS - 1));
+#pragma unroll
+        for (int i = 0; i < KPTS; i++) f[i] = __shfl_sync(mask, total, i, G);
+        __syncwarp(mask);
+    }
+
+    __device__ __forceinline__ void gradient(const float *x, float *grad) const {
+        // parameter k: b before it is moved, lo / hi its two points, r after it is moved back
+        float b[P], lo[P], hi[P], r[P], sumA = 0.0f;
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            // (the first loss call, at parameter 0's lower point, clamps all the others)
+            b[k] = bound(x[k]);
+            lo[k] = bound((k == 0 ? x[k] : b[k]) - 0.002f);
+            hi[k] = bound(lo[k] + 0.004f);
+            r[k] = bound(hi[k] - 0.002f);
+        }
+#pragma unroll
+        for (int m = 0; m < E::M; m++) sumA += fmaxf(b[E::a(m)], fmaxf(hi[E::a(m)], r[E::a(m)]));
+        float *part = s + L::PART;
+        if (safe(lo[P - 1], sumA) && safe(b[P - 1], sumA)) {
+#pragma unroll 1
+            for (int k = lane; k < PIX; k += G) {
+                const float2 c = make_float2(pos[k], pos[PIXP + k]), pl = make_float2(s[L::VAL + k], s[L::LOG + k]);
+                float v[P], e[E::M];
+#pragma unroll
+                for (int i = 0; i < P; i++) v[i] = b[i];
+#pragma unroll
+                for (int m = 0; m < E::M; m++) e[m] = 0.0f;
+#pragma unroll
+                for (int i = 0; i < P; i++) {
+                    float A[E::M], en[E::M];
+                    // emitters whose exponent the parameter before this one moved, or none is known yet
+#pragma unroll
+                    for (int m = 0; m < E::M; m++)
+                        if (!E::in(m, i) && (i == 0 || E::in(m, i - 1)))
+                            e[m] = expo(c.x, c.y, v[E::x(m)], v[E::y(m)], v[E::sx(m)], v[E::sy(m)]);
+#pragma unroll
+                    for (int side = 0; side < 2; side++) {
+                        v[i] = side ? hi[i] : lo[i];
+#pragma unroll
+                        for (int m = 0; m < E::M; m++) {
+                            A[m] = v[E::a(m)];
+                            en[m] = E::in(m, i) ? expo(c.x, c.y, v[E::x(m)], v[E::y(m)], v[E::sx(m)], v[E::sy(m)]) : e[m];
+                        }
+                        part[(2 * i + side) * PIXP + k] = term(en, A, v[P - 1], pl);
+                    }
+                    v[i] = r[i];
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < NE; j++) {
+                float v[P];
+#pragma unroll
+                for (int i = 0; i < P; i++) v[i] = i == j / 2 ? ((j & 1) ? hi[i] : lo[i]) : (i < j / 2 ? r[i] : b[i]);
+#pragma unroll 1
+                for (int k = lane; k < PIX; k += G) part[j * PIXP + k] = term_general(k, v);
+            }
+        }
+        __syncwarp(mask);
+        enum { PASSES = (NE + G - 1) / G };
+        float tot[PASSES];
+#pragma unroll
+        for (int p = 0; p < PASSES; p++) tot[p] = row_sum(min(lane + p * G, NE - 1));
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            const float tn = __shfl_sync(mask, tot[(2 * k) / G], (2 * k) % G, G);
+            const float tp = __shfl_sync(mask, tot[(2 * k + 1) / G], (2 * k + 1) % G, G);
+            grad[k] = (tp - tn) * 250.0f;
+        }
+        __syncwarp(mask);
+    }
+
+    // bfgs_update and the new direction -D grad, operation for operation (its
+    // temporaries recomputed with the roundings nvcc gives their expressions:
+    // one fused multiply-add or separate product each, the final s s'/(y's)
+    // fused into the sum).
+    __device__ __forceinline__ void update(const float *sk, const float *yk, const float *grad, float *d) const {
+        float *D = s + L::H, *Tm = s + L::T, *vec = s + L::VEC;
+        float divdat = 0.0f;
+#pragma unroll
+        for (int c = 0; c < P; c++) divdat = __fmaf_rn(sk[c], yk[c], divdat);
+        divdat = 1.0f / divdat;
+        float t10[P];
+#pragma unroll
+        for (int c = 0; c < P; c++) t10[c] = __fmul_rn(yk[c], divdat);
+        if (lane == 0) {
+#pragma unroll
+            for (int c = 0; c < P; c++) {
+                vec[c] = sk[c];
+                vec[P + c] = __fmul_rn(sk[c], divdat);
+            }
+        }
+        __syncwarp(mask);
+#pragma unroll 1
+        for (int e = lane; e < P * P; e += G) {
+            const int row = e / P, col = e - (e / P) * P;
+            const float sr = -vec[row];
+            float acc = 0.0f;
+#pragma unroll
+            for (int c = 0; c < P; c++) acc = __fmaf_rn(__fmaf_rn(sr, t10[c], row == c ? 1.0f : 0.0f), D[c * P + col], acc);
+            Tm[e] = acc;
+        }
+        __syncwarp(mask);
+#pragma unroll 1
+        for (int e = lane; e < P * P; e += G) {
+            const int row = e / P, col = e - (e / P) * P;
+            const float sc = -vec[col];
+            float acc = 0.0f;
+#pragma unroll
+            for (int c = 0; c < P; c++) acc = __fmaf_rn(Tm[row * P + c], __fmaf_rn(sc, t10[c], col == c ? 1.0f : 0.0f), acc);
+            D[e] = __fmaf_rn(vec[row], vec[P + col], acc);
+        }
+        __syncwarp(mask);
+        const int row = min(lane, P - 1);
+        float acc = 0.0f;
+#pragma unroll
+        for (int c = 0; c < P; c++) acc = __fmaf_rn(-D[row * P + c], grad[c], acc);
+#pragma unroll
+        for (int c = 0; c < P; c++) d[c] = __shfl_sync(mask, acc, c, G);
+    }
+
+    // bfgs_fit's schedule
+    __device__ __forceinline__ void fit(float *x) const {
+        static_assert(kBisections == 11 && P <= G, "one evaluation, then three rounds of three; one direction per lane");
+        float grad[P], d[P];
+        for (int e = lane; e < P * P; e += G) s[L::H + e] = e % (P + 1) == 0 ? 1.0f : 0.0f;
+        gradient(x, grad);
+#pragma unroll
+        for (int k = 0; k < P; k++) d[k] = -grad[k];
+#pragma unroll 1
+        for (int it = 0; it < T::IT; it++) {
+            float total = 0.0f;
+#pragma unroll
+            for (int k = 0; k < P; k++) total += fabsf(d[k]);
+            total = ((float)P) / total;
+#pragma unroll
+            for (int k = 0; k < P; k++) d[k] = d[k] * total;
+            float p0 = 0.00001f, p1 = 1.0f, f0 = 0.0f, f1 = 0.0f, f[KPTS];
+            // one bisection step: the moved end takes the midpoint and its loss
+            auto move = [&](float fm) {
+                const bool down = f0 < f1;
+                const float mid = (p0 + p1) * 0.5f;
+                p0 = down ? p0 : mid;
+                p1 = down ? mid : p1;
+                f0 = down ? f0 : fm;
+                f1 = down ? fm : f1;
+            };
+            {
+                const float st[KPTS] = {0.0001f, 1.0f, (p0 + p1) * 0.5f, 0.0001f};
+                losses(x, d, st, f);
+                f0 = f[0];
+                f1 = f[1];
+                move(f[2]);
+            }
+#pragma unroll 1
+            for (int round = 0; round < 3; round++) {
+                const bool down = f0 < f1;
+                const float m1 = (p0 + p1) * 0.5f;
+                const float q0 = down ? p0 : m1, q1 = down ? m1 : p1;
+                const float m2 = (q0 + q1) * 0.5f;
+                // the third midpoint: the lower half kept (upper end moved to m2), or the upper
+                const float st[KPTS] = {m1, m2, (q0 + m2) * 0.5f, (m2 + q1) * 0.5f};
+                losses(x, d, st, f);
+                move(f[0]);
+                const bool lower = f0 < f1;
+                move(f[1]);
+                move(lower ? f[2] : f[3]);
+            }
+            const bool down = f0 < f1;  // the last step moves an end without an evaluation
+            const float mid = (p0 + p1) * 0.5f;
+            p0 = down ? p0 : mid;
+            p1 = down ? mid : p1;
+            const float scale = (p0 + p1) * 0.5f;
+            float sk[P];
+#pragma unroll
+            for (int k = 0; k < P; k++) {
+                sk[k] = d[k] * scale;
+                x[k] = x[k] + sk[k];
+            }
+#pragma unroll
+            for (int k = 0; k < P; k++)
+                if (x[k] < 0.01f) x[k] = 0.01f;
+            if (it < T::IT - 1) {
+                float yk[P];
+#pragma unroll
+                for (int k = 0; k < P; k++) yk[k] = grad[k];
+                gradient(x, grad);
+#pragma unroll
+                for (int k = 0; k < P; k++) yk[k] = grad[k] - yk[k];
+                update(sk, yk, grad, d);
+            }
+        }
+    }
+};
 
 // ------------------------------------------ staged single-emitter eval ---
 // The weighted-MLE mask of an R x R ROI depends on |col - R/2| and
@@ -1837,6 +1986,18 @@ template <int R, int KIND, int DIST = ArithSpec<KIND, R>::DIST, int SUM2 = Arith
           int ITERS = KindTraits<KIND>::IT>
 __device__ __forceinline__ void mle_fit(const RoiRef &roi, float *Ininf, float *D, int ld) {
     bfgs_fit<KindTraits<KIND>::P, ITERS>(ThreadEval<R, KIND, DIST, SUM2>{roi}, Ininf, D, ld);
+}
+
+// One pixel's weight of the mask below, for the sizes whose contraction is fixed in the source.
+template <int R, int MASK>
+__device__ __forceinline__ float wle_weight(float colpos, float rowpos, float WLE_SigmaX, float WLE_SigmaY,
+                                            int MoleculeType) {
+    const float ROICenter = R / 2.0f;
+    const float WLE_SigmaX1 = 1.0f / (2.0f * WLE_SigmaX * WLE_SigmaX);
+    const float WLE_SigmaY1 = 1.0f / (2.0f * WLE_SigmaY * WLE_SigmaY);
+    if (MoleculeType == 0) return 1.0f;
+    return __expf(-sum_of_products<MASK>((colpos - ROICenter) * (colpos - ROICenter), WLE_SigmaX1,
+                                         (rowpos - ROICenter) * (rowpos - ROICenter), WLE_SigmaY1));
 }
 
 // Weighted-MLE mask (bfgsMLE_core.h:206-238).

@@ -33,8 +33,10 @@ struct FitLaunch {
     // latency, sets the time)
     int thread_per_roi = 0;
     // multi-emitter kinds: the longest queue the lane-group kernel fits (0: the
-    // default, about three of its waves; the autotuner measures it)
+    // default; the autotuner measures it)
     int group_limit = 0;
+    // the queue's length is max_count (known on the host)
+    int exact = 0;
 };
 
 // kind: FitKind (qcs_fit_math.cuh); R: ROI size.
@@ -44,9 +46,11 @@ cudaError_t launch_fit(int kind, int R, const FitLaunch &a);
 bool multi_group_available(int kind, int R);
 int multi_group_default_limit(int kind, int R);
 
-// Single-emitter kinds with `lanes` lanes per ROI (8; also 4 and 16 for GS2D
-// 7x7): the rows of launch_fit bit for bit, lower latency.  Sizes: GS2D 7, 9,
-// 11, 13 and AS3D 7, 9, 11 (group_fit_supported).
+// Single-emitter kinds with several lanes per ROI: the rows of launch_fit bit
+// for bit, lower latency.  lanes: 4, 8 or 16 (at least that many where a size
+// is compiled for more), or 0: by the queue's length, with one thread per ROI
+// for long ones.  Sizes: GS2D 7, 9, 11, 13 and AS3D 7, 9, 11
+// (group_fit_supported).
 bool group_fit_supported(int kind, int R);
 cudaError_t launch_fit_group(int kind, int R, int lanes, const FitLaunch &a);
 
