@@ -46,87 +46,89 @@ __device__ __forceinline__ float psf_value(const PsfPara &p, float dx, float dy)
     return __fmaf_rn(p.peak, e, p.bkg);
 }
 
+// x / 0.02f correctly rounded without a division: with C the double-length
+// reciprocal ch + cl of 0.02f, RN(ch x + RN(cl x)) (Brisebarre and Muller,
+// "Correctly rounded multiplication by arbitrary precision constants", IEEE
+// Trans. Comput. 57, 2008).  Compared with the division for every float in the
+// range it is used for (a zero may lose its sign, which no sum shows).
+__device__ __forceinline__ float div_dh(float x) {
+    constexpr double inv = 1.0 / (double)0.02f;
+    constexpr float ch = (float)inv, cl = (float)(inv - (double)ch);
+    const float q = __fmaf_rn(ch, x, __fmul_rn(cl, x));
+    const float a = fabsf(x);
+    if (a < 1e30f && (a > 1e-30f || a == 0.0f)) return q;
+    return __fdiv_rn(x, 0.02f);
+}
+
 // (f(+h) - 2 f(0) + f(-h)) / h / h with the reference's rounding
 // (LocPrecCalc_GaussianCRLB.h:188-196; 2 f(0) is exact, so fusing it changes nothing).
 __device__ __forceinline__ float second_diff(float fp, float f0, float fn) {
-    const float dh = 0.02f;
-    return __fdiv_rn(__fdiv_rn(__fadd_rn(__fmaf_rn(-2.0f, f0, fp), fn), dh), dh);
+    return div_dh(div_dh(__fadd_rn(__fmaf_rn(-2.0f, f0, fp), fn)));
 }
 
-// Two lanes per row.  The reference evaluates the PSF on the full grid
-// seven times per row (model, then base, +dh, -dh for each derivative) and
-// sums d2 - model * d2log over every pixel.  The same values come from far
+// One thread per row and axis.  The reference evaluates the PSF on the full
+// grid seven times per row (model, then base, +dh, -dh for each derivative)
+// and sums d2 - model * d2log over every pixel.  The same values come from far
 // fewer evaluations, exactly: the base points equal the model (same
 // parameters, same rounding), the model is symmetric in x and y, the -dh
 // evaluation is the +dh one mirrored (x - (-h) = -((-x) - h) exactly), and
-// each derivative's terms are symmetric across the other axis.  So the
-// model is evaluated on one quadrant, each +dh grid on half the rows
-// (columns), each term on half the grid, and the Fisher sums still add every
-// pixel's term in the reference's pixel order.  A 32-thread block takes 16
-// rows: lane r (r < 16) computes row r's x-derivative terms and Fisher sum,
-// lane r + 16 its y-derivative terms and sum, after the two have filled the
-// row's model table together.  The y terms are the x terms' code with the
-// axes exchanged (the reference's two sites contract mirror-image products),
-// so the warp does not diverge; each sum still runs in pixel order.  Tables
-// live in shared memory, [entry][row].
+// each derivative's terms are symmetric across the other axis.  So a thread
+// takes the half grid line by line: the line's model values (half a line) and
+// +dh values, then its terms, kept in shared memory ([term][thread]); the
+// Fisher sum adds every pixel's term in the reference's pixel order.  The y
+// terms are the x terms with the axes exchanged (the reference's two sites
+// contract mirror-image products); warp 0 of a block takes 32 rows' x terms,
+// warp 1 their y terms.  Nothing is shared between threads, so the terms are
+// the only shared memory: 14 warps an SM at 15 x 15.  100,000 rows at 9 x 9: 66
+// -> 43 us, 60,013 at 15 x 15: 221 -> 93 us, 300 rows: 24 -> 14 us (before: a
+// model table per row, 9 warps an SM at 15 x 15, and four divisions per term).
+// Bound by the instructions of logf, 2 (Q + G) a line.
 template <int G>
-__global__ void __launch_bounds__(32) crlb_kernel(float *__restrict__ loc, const int *__restrict__ n_dev, int n,
+__global__ void __launch_bounds__(64) crlb_kernel(float *__restrict__ loc, const int *__restrict__ n_dev, int n,
                                                   const int *__restrict__ ids, const uint8_t *__restrict__ skip,
                                                   float ReadNoise_e, float QE, float PixelSize) {
-    enum { H = G / 2, Q = H + 1, ROWS = 16, TT = Q * G * ROWS, TSTRIDE = TT + ((TT % 32) == 0 ? 16 : 0) };
+    enum { H = G / 2, Q = H + 1 };
     using S = CrlbSites<G>;
-    // the x-derivative lane uses fma(dx^2, six, dy^2 siy), the y-derivative lane
+    // the x-derivative thread uses fma(dx^2, six, dy^2 siy), the y-derivative thread
     // fma(dy^2, siy, dx^2 six): one expression with its operands exchanged
     static_assert(S::SHIFT_X == kFuseFirst && S::SHIFT_Y == kFuseSecond, "mirrored derivative sites");
-    // per row: model and its log on one quadrant (shared by the row's two
-    // lanes); per lane: its derivative's terms T[l][k] (line l, position k)
-    __shared__ float sM[Q * Q][ROWS], sLM[Q * Q][ROWS];
-    __shared__ float sT[2 * TSTRIDE];
-    const int lane = threadIdx.x, slot = lane & (ROWS - 1), role = lane >> 4;  // role 0: x, 1: y
+    __shared__ float sT[Q * G][64];
+    const int role = threadIdx.x >> 5;  // 0: x, 1: y
     const int rows = n_dev ? *n_dev : n;
-    const int k_slot = blockIdx.x * ROWS + slot;
-    bool have = k_slot < rows;
-    const int gid = have ? (ids ? ids[k_slot] : k_slot) : 0;
-    if (have && skip && skip[gid]) have = false;
+    const int k_slot = blockIdx.x * 32 + (threadIdx.x & 31);
+    if (k_slot >= rows) return;
+    const int gid = ids ? ids[k_slot] : k_slot;
+    if (skip && skip[gid]) return;
     float *r = loc + (size_t)gid * 12;
-    bool valid = false;
-    PsfPara p = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (have) {
-        const float TotalPhoton_e = __fmul_rn(r[QCS_POS_TPHO], QE);
-        float Background_e = __fmul_rn(r[QCS_POS_BAKG], QE);
-        const float sx = r[QCS_POS_SIGX], sy = r[QCS_POS_SIGY];
-        valid = (TotalPhoton_e > 1) && (Background_e > 1) && (sx > 0.1) && (sy > 0.1) && (sx < 10) && (sy < 10);
-        if (valid) {
-            // read noise counted into the background (LocPrecCalc_GaussianCRLB.h:89-92)
-            Background_e = __fdiv_rn(__fmaf_rn(ReadNoise_e, ReadNoise_e, __fmul_rn(Background_e, QE)), QE);
-            const float pi = 3.141592654f;
-            p.peak = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(__fmul_rn(__fmul_rn(2.0f, pi), sx), sy)), TotalPhoton_e);
-            p.six = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, sx), sx));
-            p.siy = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, sy), sy));
-            p.bkg = Background_e;
-            // model on one quadrant, sM[a][b] at |CurY| = a, |CurX| = b: the two
-            // lanes of the row take alternate entries
-            for (int e = role; e < Q * Q; e += 2) {
-                const int a = e / Q, b = e - (e / Q) * Q;
-                const float v = psf_value<S::CENTRE>(p, (float)b, (float)a);
-                sM[e][slot] = v;
-                sLM[e][slot] = logf(v);
-            }
-        }
-    }
-    __syncwarp();
+    const float TotalPhoton_e = __fmul_rn(r[QCS_POS_TPHO], QE);
+    float Background_e = __fmul_rn(r[QCS_POS_BAKG], QE);
+    const float sx = r[QCS_POS_SIGX], sy = r[QCS_POS_SIGY];
     float std_dev = 100.0f;
-    if (valid) {
+    if ((TotalPhoton_e > 1) && (Background_e > 1) && (sx > 0.1) && (sy > 0.1) && (sx < 10) && (sy < 10)) {
+        // read noise counted into the background (LocPrecCalc_GaussianCRLB.h:89-92)
+        Background_e = __fdiv_rn(__fmaf_rn(ReadNoise_e, ReadNoise_e, __fmul_rn(Background_e, QE)), QE);
+        const float pi = 3.141592654f;
+        PsfPara p;
+        p.peak = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(__fmul_rn(__fmul_rn(2.0f, pi), sx), sy)), TotalPhoton_e);
+        p.six = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, sx), sx));
+        p.siy = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, sy), sy));
+        p.bkg = Background_e;
         const float h = 0.02f;
-        float *T = sT + role * TSTRIDE;
         const float su = role ? p.siy : p.six, sv = role ? p.six : p.siy;
-        // x lane: the +dh row at |CurY| = l, every column k; y lane: the +dh
-        // column at |CurX| = l, every row k
+        float *T = &sT[0][threadIdx.x];
+        // x thread: the +dh row at |CurY| = l, every column k; y thread: the
+        // +dh column at |CurX| = l, every row k
 #pragma unroll 1
         for (int l = 0; l < Q; ++l) {
-            float tp[G], lp[G];
             const float fl = (float)l;
             const float ll = __fmul_rn(__fmul_rn(fl, fl), sv);
+            float m[Q], lm[Q], tp[G], lp[G];
+#pragma unroll
+            for (int o = 0; o < Q; ++o) {
+                const float dx = role ? fl : (float)o, dy = role ? (float)o : fl;
+                m[o] = psf_value<S::CENTRE>(p, dx, dy);
+                lm[o] = logf(m[o]);
+            }
 #pragma unroll
             for (int k = 0; k < G; ++k) {
                 const float sh = __fsub_rn((float)(k - H), h);
@@ -136,11 +138,9 @@ __global__ void __launch_bounds__(32) crlb_kernel(float *__restrict__ loc, const
 #pragma unroll
             for (int k = 0; k < G; ++k) {
                 const int o = k < H ? H - k : k - H;  // |k - H|
-                const int e = role ? o * Q + l : l * Q + o;
-                const float m = sM[e][slot];
-                const float d2 = second_diff(tp[k], m, tp[G - 1 - k]);
-                const float dl = second_diff(lp[k], sLM[e][slot], lp[G - 1 - k]);
-                T[(l * G + k) * ROWS + slot] = __fmaf_rn(-m, dl, d2);
+                const float d2 = second_diff(tp[k], m[o], tp[G - 1 - k]);
+                const float dl = second_diff(lp[k], lm[o], lp[G - 1 - k]);
+                T[(l * G + k) * 64] = __fmaf_rn(-m[o], dl, d2);
             }
         }
         // Fisher information, pixel order (LocPrecCalc_GaussianCRLB.h:226-243)
@@ -151,14 +151,13 @@ __global__ void __launch_bounds__(32) crlb_kernel(float *__restrict__ loc, const
 #pragma unroll
             for (int x = 0; x < G; ++x) {
                 const int bx = x < H ? H - x : x - H;
-                const int tl = role ? bx : ay, tk = role ? y : x;
-                F = __fadd_rn(F, T[(tl * G + tk) * ROWS + slot]);
+                F = __fadd_rn(F, T[(role ? bx * G + y : ay * G + x) * 64]);
             }
         }
         if (F == 0.0f) F = 1;
         std_dev = __fmul_rn(__fsqrt_rn(__fdiv_rn(1.0f, F)), PixelSize);
     }
-    if (have) r[role ? QCS_POS_CRBY : QCS_POS_CRBX] = std_dev;
+    r[role ? QCS_POS_CRBY : QCS_POS_CRBX] = std_dev;
 }
 
 }  // namespace
@@ -166,11 +165,11 @@ __global__ void __launch_bounds__(32) crlb_kernel(float *__restrict__ loc, const
 cudaError_t launch_crlb(float *loc, const int *n_dev, int n, int max_rows, int loc_type, float ReadNoise_e, float QE,
                         float PixelSize, cudaStream_t s, const int *ids, const uint8_t *skip) {
     if (max_rows <= 0) return cudaSuccess;
-    const int blocks = (max_rows + 15) / 16;  // 16 rows per 32-thread block
+    const int blocks = (max_rows + 31) / 32;  // 32 rows per 64-thread block
     if (loc_type != QCS_LOCTYPE_AS3D)
-        crlb_kernel<9><<<blocks, 32, 0, s>>>(loc, n_dev, n, ids, skip, ReadNoise_e, QE, PixelSize);
+        crlb_kernel<9><<<blocks, 64, 0, s>>>(loc, n_dev, n, ids, skip, ReadNoise_e, QE, PixelSize);
     else
-        crlb_kernel<15><<<blocks, 32, 0, s>>>(loc, n_dev, n, ids, skip, ReadNoise_e, QE, PixelSize);
+        crlb_kernel<15><<<blocks, 64, 0, s>>>(loc, n_dev, n, ids, skip, ReadNoise_e, QE, PixelSize);
     return cudaGetLastError();
 }
 
