@@ -1,11 +1,11 @@
 // WLE pre-pass (weighted-MLE parameters) over a batch of ROI records:
-//   psf_width_kernel   row/column means -> natural cubic spline x10 -> peak ->
-//                      two-sided widths sigma L/R/U/D
+//   widths_keys_kernel row/column means -> natural cubic spline x10 -> peak ->
+//                      two-sided widths sigma L/R/U/D, neighbour keys
 //                      (WLEParaEstimation_core.h:44-156, SplineInterpolation.h:40-202,
 //                      WLEParaEstimation_core.cu:21-28, 91-136)
 //   nearest neighbour  same-frame minimum centre distance
 //                      (WLEParaEstimation_core.cu:140-183)
-//   classify_kernel    molecule type MLEFit / WLEFit / MultiFit
+//   molecule type      MLEFit / WLEFit / MultiFit
 //                      (WLEParaEstimation_core.cu:197-264)
 // The floating-point code keeps the reference's expression shapes (bit-equal
 // results).  The nearest-neighbour search replaces the reference's O(N^2)
@@ -29,107 +29,6 @@ constexpr int kInterp = 10;                    // InterpolationRatio
 #define QCS_PEAK_FIND_RATIO 0.8f               // PeakFindRangeRatio
 #define QCS_MAX_WIDTH_DIFF 0.40f               // MaxTolerablePSFWidthDiff
 
-template <int N>
-__device__ __forceinline__ void spline_system(float *A, float *b, const float *x_i, const float *y_i) {
-    for (int r = 0; r < N; r++)
-        for (int c = 0; c < N; c++) A[r * N + c] = 0;
-    A[0] = 1;
-    A[(N - 1) * N + N - 1] = 1;
-    for (int i = 1; i < N - 1; i++) {
-        const float h0 = x_i[i] - x_i[i - 1];
-        const float h1 = x_i[i + 1] - x_i[i];
-        A[i * N + i - 1] = h0;
-        A[i * N + i] = 2 * (h0 + h1);
-        A[i * N + i + 1] = h1;
-    }
-    b[0] = 0;
-    b[N - 1] = 0;
-    for (int i = 1; i < N - 1; i++) {
-        const float h0 = x_i[i] - x_i[i - 1];
-        const float h1 = x_i[i + 1] - x_i[i];
-        const float a0 = y_i[i - 1];
-        const float a1 = y_i[i];
-        const float a2 = y_i[i + 1];
-        b[i] = 3 / h1 * (a2 - a1) - 3 / h0 * (a1 - a0);
-    }
-}
-
-template <int N>
-__device__ __forceinline__ void spline_solve(const float *A, const float *b, float *x) {
-    float y[N], Beta[N];
-    for (int i = 0; i < N - 1; i++) {
-        const float ci = A[i * N + i + 1];
-        const float bi = A[i * N + i];
-        if (i == 0) {
-            Beta[i] = ci / bi;
-        } else {
-            const float ai = A[i * N + i - 1];
-            Beta[i] = ci / (bi - ai * Beta[i - 1]);
-        }
-    }
-    for (int i = 0; i < N; i++) {
-        const float bi = A[i * N + i];
-        if (i == 0) {
-            y[i] = b[i] / bi;
-        } else {
-            const float ai = A[i * N + i - 1];
-            y[i] = (b[i] - ai * y[i - 1]) / (bi - ai * Beta[i - 1]);
-        }
-    }
-    for (int i = N - 1; i >= 0; i--) {
-        if (i == N - 1)
-            x[i] = y[i];
-        else
-            x[i] = y[i] - Beta[i] * x[i + 1];
-    }
-}
-
-template <int N, int M>
-__device__ __forceinline__ void spline_interpolate(const float *x_i, const float *y_i, const float *x_o, float *y_o) {
-    float An[N], Bn[N], Cn[N], Dn[N];
-    for (int i = 0; i < N; i++) An[i] = y_i[i];
-    float A[N * N], b[N];
-    spline_system<N>(A, b, x_i, y_i);
-    spline_solve<N>(A, b, Cn);
-    for (int i = 0; i < N - 1; i++) {
-        const float hi = x_i[i + 1] - x_i[i];
-        Bn[i] = 1 / hi * (An[i + 1] - An[i]) - hi / 3 * (2 * Cn[i] + Cn[i + 1]);
-        Dn[i] = (Cn[i + 1] - Cn[i]) / (3 * hi);
-    }
-    for (int i = 0; i < M; i++) {
-        const float xn = x_o[i];
-        int ParaSet = xn - 0.0f;  // sample positions start at pixel 0, unit spacing
-        if (ParaSet < 0) ParaSet = 0;
-        if (ParaSet >= N - 1) ParaSet = N - 2;
-        const float xi = x_i[ParaSet];
-        y_o[i] = An[ParaSet] + Bn[ParaSet] * (xn - xi) + Cn[ParaSet] * (xn - xi) * (xn - xi) +
-                 Dn[ParaSet] * (xn - xi) * (xn - xi) * (xn - xi);
-    }
-}
-
-__device__ __forceinline__ int find_max_pos(const float *iData, int DataLen, int LSel, int RSel) {
-    LSel = max(LSel, 0);
-    RSel = min(RSel, DataLen - 1);
-    int MaxIdx = DataLen / 2;
-    for (int cnt = LSel; cnt <= RSel; cnt++)
-        if (iData[cnt] > iData[MaxIdx]) MaxIdx = cnt;
-    return MaxIdx;
-}
-
-__device__ __forceinline__ void two_sided_width(float *SigmaL, float *SigmaR, const float *MeanData_Intp, int DataLen,
-                                                int MaxPos) {
-    const float MaxValue = MeanData_Intp[MaxPos];
-    const int LLen = MaxPos;
-    const int RLen = DataLen - MaxPos - 1;
-    const int CmpLen = min(LLen, RLen);
-    float SDat_L = 0;
-    for (int i = MaxPos - CmpLen; i <= MaxPos; i++) SDat_L = SDat_L + MeanData_Intp[i];
-    float SDat_R = 0;
-    for (int i = MaxPos; i <= MaxPos + CmpLen; i++) SDat_R = SDat_R + MeanData_Intp[i];
-    *SigmaL = SDat_L * QCS_INTERP_GAP / MaxValue / 1.2533f;
-    *SigmaR = SDat_R * QCS_INTERP_GAP / MaxValue / 1.2533f;
-}
-
 // Records [begin, begin + n): from the arguments, or from span[0], span[1]
 // in device memory when span is set (grid-stride loops cover any n).
 struct Span {
@@ -146,66 +45,144 @@ struct Span {
     }
 };
 
+// Two-sided widths of one profile (a record's column or row sums, integers).
+// The natural cubic spline through the R means has unit knots, so its system
+// has constant coefficients (elimination factors beta, folded at compile
+// time); the 10 R - 9 samples at 0.1 px are evaluated where they are used
+// instead of being kept: first those near the centre for the peak, then all of
+// them for the two sums, each sum adding its samples in ascending order.
+// Every rounding is that of the straightforward code (arrays of samples,
+// general tridiagonal solve) as nvcc contracts it, found by comparing each
+// choice with it on a GPU: the same widths bit for bit.
 template <int R>
-__device__ __forceinline__ void psf_width_one(const uint16_t *__restrict__ rois, float *__restrict__ wle, int gid) {
-    enum { Len = R, ILen = (R - 1) * kInterp + 1, WHOLE = R * (R + 1) };
-    const uint16_t *pROI = rois + (size_t)gid * WHOLE;
-    float MeanX[Len], MeanY[Len], x0[Len], xn[ILen], yn_MeanX[ILen], yn_MeanY[ILen];
-    for (int cnt = 0; cnt < Len; cnt++) {
-        MeanX[cnt] = 0;
-        MeanY[cnt] = 0;
+struct Spline {
+    enum { S = R - 1, LEN = S * kInterp + 1, MID = LEN / 2, FIND = (int)(kInterp * QCS_PEAK_FIND_RATIO) };
+    float A[S], B[S], C[S], D[S];
+    static __device__ __forceinline__ int seg(int i) { return i / kInterp < S ? i / kInterp : S - 1; }
+    // sample i (a constant after unrolling)
+    __device__ __forceinline__ float at(int i) const {
+        const int g = seg(i);
+        const float t = i * QCS_INTERP_GAP - (float)g;
+        return __fmaf_rn(__fmul_rn(__fmul_rn(D[g], t), t), t, __fmaf_rn(__fmul_rn(C[g], t), t, __fmaf_rn(B[g], t, A[g])));
     }
-    for (int r = 0; r < Len; r++) {
-        for (int c = 0; c < Len; c++) {
-            MeanX[c] = MeanX[c] + pROI[r * R + c];
-            MeanY[r] = MeanY[r] + pROI[r * R + c];
+};
+
+template <int R>
+__device__ __forceinline__ void profile_widths(const int (&sum)[R], float &left, float &right) {
+    typedef Spline<R> Sp;
+    Spline<R> sp;
+    int low = sum[0];
+#pragma unroll
+    for (int i = 1; i < R; i++) low = min(low, sum[i]);
+    float a[R], y[R], c[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) a[i] = __fdiv_rn((float)(sum[i] - low), (float)R);
+    // beta[i] of the elimination: 0, then 1 / (4 - beta[i - 1])
+    float beta = 0.0f, betas[R];
+    y[0] = 0.0f;
+    betas[0] = 0.0f;
+#pragma unroll
+    for (int i = 1; i < R - 1; i++) {
+        const float d1 = __fsub_rn(a[i + 1], a[i]), d0 = __fsub_rn(a[i], a[i - 1]);
+        // 3 d1 - 3 d0: nvcc fuses the first product, at i = 1 and R - 3 the second (5x5: at 2 neither)
+        const float b = (R == 5 && i == 2)        ? __fsub_rn(__fmul_rn(3.0f, d1), __fmul_rn(3.0f, d0))
+                        : (i == 1 || i == R - 3) ? __fmaf_rn(-3.0f, d0, __fmul_rn(3.0f, d1))
+                                                 : __fmaf_rn(3.0f, d1, -__fmul_rn(3.0f, d0));
+        y[i] = __fdiv_rn(__fsub_rn(b, y[i - 1]), 4.0f - beta);
+        beta = 1.0f / (4.0f - beta);
+        betas[i] = beta;
+    }
+    c[R - 1] = 0.0f;
+#pragma unroll
+    for (int i = R - 2; i >= 0; i--) c[i] = __fmaf_rn(-betas[i], c[i + 1], y[i]);
+#pragma unroll
+    for (int i = 0; i < R - 1; i++) {
+        sp.A[i] = a[i];
+        sp.B[i] = __fmaf_rn(-(1.0f / 3.0f), __fmaf_rn(2.0f, c[i], c[i + 1]), __fsub_rn(a[i + 1], a[i]));
+        sp.C[i] = c[i];
+        sp.D[i] = __fdiv_rn(__fsub_rn(c[i + 1], c[i]), 3.0f);
+    }
+    int pos = Sp::MID;
+    float peak = sp.at(Sp::MID);
+#pragma unroll
+    for (int i = Sp::MID - Sp::FIND; i <= Sp::MID + Sp::FIND; i++) {
+        const float v = sp.at(i);
+        if (v > peak) {
+            peak = v;
+            pos = i;
         }
     }
-    float MinX = MeanX[0];
-    float MinY = MeanY[0];
-    for (int cnt = 0; cnt < Len; cnt++) {
-        MinX = fminf(MinX, MeanX[cnt]);
-        MinY = fminf(MinY, MeanY[cnt]);
+    const int half = min(pos, (int)Sp::LEN - pos - 1);
+    const int lo = pos - half, hi = pos + half;
+    float sl = 0.0f, sr = 0.0f;
+#pragma unroll
+    for (int i = 0; i < Sp::LEN; i++) {
+        const float v = sp.at(i);
+        if (i <= Sp::MID + Sp::FIND) sl = (i >= lo && i <= pos) ? __fadd_rn(sl, v) : sl;
+        if (i >= Sp::MID - Sp::FIND) sr = (i >= pos && i <= hi) ? __fadd_rn(sr, v) : sr;
     }
-    for (int cnt = 0; cnt < Len; cnt++) {
-        MeanX[cnt] = (MeanX[cnt] - MinX) / Len;
-        MeanY[cnt] = (MeanY[cnt] - MinY) / Len;
-    }
-    for (int cnt = 0; cnt < Len; cnt++) x0[cnt] = cnt;
-    for (int cnt = 0; cnt < ILen; cnt++) xn[cnt] = cnt * QCS_INTERP_GAP;
-    spline_interpolate<Len, ILen>(x0, MeanX, xn, yn_MeanX);
-    spline_interpolate<Len, ILen>(x0, MeanY, xn, yn_MeanY);
-    const int FindRegionlen = kInterp * QCS_PEAK_FIND_RATIO;
-    const int InterpCenter = ILen / 2;
-    const int MaxPos_X = find_max_pos(yn_MeanX, ILen, InterpCenter - FindRegionlen, InterpCenter + FindRegionlen);
-    const int MaxPos_Y = find_max_pos(yn_MeanY, ILen, InterpCenter - FindRegionlen, InterpCenter + FindRegionlen);
-    float SigmaL, SigmaR, SigmaU, SigmaD;
-    two_sided_width(&SigmaL, &SigmaR, yn_MeanX, ILen, MaxPos_X);
-    two_sided_width(&SigmaU, &SigmaD, yn_MeanY, ILen, MaxPos_Y);
-    float *o = wle + (size_t)gid * QCS_WLE_PARA_NUM;
-    o[1] = SigmaL;
-    o[2] = SigmaR;
-    o[3] = SigmaU;
-    o[4] = SigmaD;
+    left = __fdiv_rn(__fdiv_rn(__fmul_rn(sl, QCS_INTERP_GAP), peak), 1.2533f);
+    right = __fdiv_rn(__fdiv_rn(__fmul_rn(sr, QCS_INTERP_GAP), peak), 1.2533f);
 }
+
+// The PSF widths of a tile of kTile records, two threads a record: the tile is
+// copied into shared memory (coalesced; an odd word pitch), warps 0 and 1 take
+// the column sums, 2 and 3 the row sums.  Called by every thread of the block;
+// the rows are complete after the next block barrier.  One thread per record with
+// sample arrays in local memory took 23 / 79 / 152 us for 100,000 7x7 / 60,013
+// 9x9 / 100,000 11x11 records (and 13 us for keys and types in kernels of their
+// own); this takes 15 / 14 / 25 us with the keys.
+constexpr int kTile = 64, kTileThreads = 2 * kTile;
+template <int R>
+struct Tile {
+    enum { WHOLE = R * (R + 1), WORDS = WHOLE / 2, PITCH = WORDS | 1 };
+    uint32_t px[kTile * PITCH];
+};
 
 template <int R>
-__global__ void psf_width_kernel(const uint16_t *__restrict__ rois, float *__restrict__ wle, Span sp) {
-    int b, n;
-    sp.get(b, n);
-    for (int k = threadIdx.x + blockDim.x * blockIdx.x; k < n; k += gridDim.x * blockDim.x)
-        psf_width_one<R>(rois, wle, b + k);
+__device__ __forceinline__ void tile_widths(Tile<R> &tile, const uint16_t *__restrict__ rois, float *__restrict__ wle,
+                                            int first, int cnt) {
+    typedef Tile<R> T;
+    const uint16_t *src = rois + (size_t)first * T::WHOLE;
+    uint16_t *dst = reinterpret_cast<uint16_t *>(tile.px);
+    if ((reinterpret_cast<uintptr_t>(src) & 3) == 0) {
+        const uint32_t *s4 = reinterpret_cast<const uint32_t *>(src);
+        for (int i = threadIdx.x; i < cnt * T::WORDS; i += kTileThreads)
+            tile.px[i / T::WORDS * T::PITCH + i % T::WORDS] = __ldg(s4 + i);
+    } else {
+        for (int i = threadIdx.x; i < cnt * T::WHOLE; i += kTileThreads)
+            dst[i / T::WHOLE * (2 * T::PITCH) + i % T::WHOLE] = __ldg(src + i);
+    }
+    __syncthreads();
+    const int rec = threadIdx.x % kTile, rows = threadIdx.x / kTile;
+    if (rec < cnt) {
+        const uint16_t *p = dst + rec * (2 * T::PITCH);
+        int sum[R];
+#pragma unroll
+        for (int i = 0; i < R; i++) sum[i] = 0;
+        // sums of at most 17 x 65,535 are exact as floats, so the integers' order does not matter
+        if (rows) {
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int c = 0; c < R; c++) sum[r] += p[r * R + c];
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; r++)
+#pragma unroll
+                for (int c = 0; c < R; c++) sum[c] += p[r * R + c];
+        }
+        float left, right;
+        profile_widths<R>(sum, left, right);
+        float *o = wle + (size_t)(first + rec) * QCS_WLE_PARA_NUM + 1 + 2 * rows;
+        o[0] = left;
+        o[1] = right;
+    }
 }
 
-// Sort key: frame (32 bits) | y (16) | x (16) of the ROI centre.
-__global__ void nn_keys_kernel(const uint16_t *__restrict__ rois, int n, int whole, int pix,
-                               unsigned long long *keys, int *vals) {
-    const int i = threadIdx.x + blockDim.x * blockIdx.x;
-    if (i >= n) return;
-    const uint16_t *h = rois + (size_t)i * whole + pix;
-    const unsigned long long frame = (unsigned long long)h[2] + 65536ull * h[3];
-    keys[i] = (frame << 32) | ((unsigned long long)h[1] << 16) | h[0];
-    vals[i] = i;
+// Sort key of a record's header h: frame (32 bits) | y (16) | x (16) of the ROI centre.
+__device__ __forceinline__ unsigned long long record_key(const uint16_t *h) {
+    return (((unsigned long long)h[2] + 65536ull * h[3]) << 32) | ((unsigned long long)h[1] << 16) | h[0];
 }
 
 // Distance to the nearest other ROI centre of the same frame: scans the
@@ -261,14 +238,6 @@ __device__ __forceinline__ float nn_sorted(const unsigned long long *__restrict_
     return sqrtf(best);
 }
 
-// Minimum distance for each record, over the radix-sorted keys.
-__global__ void nn_scan_kernel(const unsigned long long *__restrict__ keys, const int *__restrict__ vals, int n,
-                               float *__restrict__ wle) {
-    const int a = threadIdx.x + blockDim.x * blockIdx.x;
-    if (a >= n) return;
-    wle[(size_t)vals[a] * QCS_WLE_PARA_NUM + 0] = nn_sorted(keys, a, n);
-}
-
 __device__ __forceinline__ void classify_one(const uint16_t *__restrict__ rois, float *__restrict__ wle, int gid, int R,
                                              int whole, int LocType) {
     float MaxMeanSigmaTh;
@@ -296,46 +265,80 @@ __device__ __forceinline__ void classify_one(const uint16_t *__restrict__ rois, 
     w[5] = MoleculeType;
 }
 
-__global__ void classify_kernel(const uint16_t *__restrict__ rois, float *__restrict__ wle, Span sp, int R, int whole,
-                                int LocType) {
-    int b, n;
-    sp.get(b, n);
-    for (int k = threadIdx.x + blockDim.x * blockIdx.x; k < n; k += gridDim.x * blockDim.x)
-        classify_one(rois, wle, b + k, R, whole, LocType);
+// Nearest neighbour, then molecule type, of each record, over the radix-sorted keys.
+__global__ void nn_scan_kernel(const unsigned long long *__restrict__ keys, const int *__restrict__ vals, int n,
+                               const uint16_t *__restrict__ rois, float *__restrict__ wle, int R, int LocType) {
+    const int a = threadIdx.x + blockDim.x * blockIdx.x;
+    if (a >= n) return;
+    const int id = vals[a];
+    wle[(size_t)id * QCS_WLE_PARA_NUM + 0] = nn_sorted(keys, a, n);
+    classify_one(rois, wle, id, R, R * (R + 1), LocType);
 }
 
 // Records already in ascending (frame, y, x) order with their keys in a
 // compact array: PSF widths, nearest neighbour and molecule type of each
 // record in one pass (one thread per record).
 template <int R>
-__global__ void wle_sorted_kernel(const uint16_t *__restrict__ rois, const unsigned long long *__restrict__ keys,
-                                  Span sp, float *__restrict__ wle, int LocType) {
+__global__ void __launch_bounds__(kTileThreads) wle_sorted_kernel(const uint16_t *__restrict__ rois,
+                                                                  const unsigned long long *__restrict__ keys, Span sp,
+                                                                  float *__restrict__ wle, int LocType) {
+    __shared__ Tile<R> tile;
     int b0, n;
     sp.get(b0, n);
-    for (int a = threadIdx.x + blockDim.x * blockIdx.x; a < n; a += gridDim.x * blockDim.x) {
-        psf_width_one<R>(rois, wle, b0 + a);
-        wle[(size_t)(b0 + a) * QCS_WLE_PARA_NUM + 0] = nn_sorted(keys + b0, a, n);
-        classify_one(rois, wle, b0 + a, R, R * (R + 1), LocType);
+    for (int a0 = blockIdx.x * kTile; a0 < n; a0 += gridDim.x * kTile) {
+        const int cnt = min(kTile, n - a0);
+        tile_widths<R>(tile, rois, wle, b0 + a0, cnt);
+        __syncthreads();  // the tile's widths are written, its pixels free
+        if (threadIdx.x < cnt) {
+            const int a = a0 + threadIdx.x;
+            wle[(size_t)(b0 + a) * QCS_WLE_PARA_NUM + 0] = nn_sorted(keys + b0, a, n);
+            classify_one(rois, wle, b0 + a, R, R * (R + 1), LocType);
+        }
     }
 }
 
+// PSF widths of the records, and their neighbour keys: keys[i], vals[i] = i;
+// unsorted[0] = 1 (zero at launch) when some record's key is below its
+// predecessor's, unsorted[1] = n (unsorted may be null).
 template <int R>
-void psf_width_launch(const uint16_t *rois, float *wle, Span sp, int grid, int tpb, cudaStream_t s) {
-    psf_width_kernel<R><<<grid, tpb, 0, s>>>(rois, wle, sp);
+__global__ void __launch_bounds__(kTileThreads) widths_keys_kernel(const uint16_t *__restrict__ rois, int n,
+                                                                   float *__restrict__ wle,
+                                                                   unsigned long long *__restrict__ keys,
+                                                                   int *__restrict__ vals, int *__restrict__ unsorted) {
+    __shared__ Tile<R> tile;
+    if (unsorted && blockIdx.x == 0 && threadIdx.x == 0) unsorted[1] = n;
+    const int first = blockIdx.x * kTile, cnt = min(kTile, n - first);
+    tile_widths<R>(tile, rois, wle, first, cnt);
+    if (threadIdx.x < kTile) {  // two whole warps
+        bool bad = false;
+        if (threadIdx.x < cnt) {
+            const int i = first + threadIdx.x;
+            const unsigned long long k = record_key(rois + (size_t)i * Tile<R>::WHOLE + R * R);
+            bad = i > 0 && record_key(rois + (size_t)(i - 1) * Tile<R>::WHOLE + R * R) > k;
+            keys[i] = k;
+            vals[i] = i;
+        }
+        if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0 && unsorted) atomicOr(unsorted, 1);
+    }
 }
 
-cudaError_t launch_psf_width(int R, const uint16_t *rois, float *wle, Span sp, int grid, int tpb, cudaStream_t s) {
+cudaError_t launch_widths_keys(int R, const uint16_t *rois, int n, float *wle, unsigned long long *keys, int *vals,
+                               int *unsorted, cudaStream_t s) {
+    const int grid = (n + kTile - 1) / kTile;
+#define QCS_WIDTHS(RR) \
+    case RR: widths_keys_kernel<RR><<<grid, kTileThreads, 0, s>>>(rois, n, wle, keys, vals, unsorted); break;
     switch (R) {
-    case 5: psf_width_launch<5>(rois, wle, sp, grid, tpb, s); break;
-    case 7: psf_width_launch<7>(rois, wle, sp, grid, tpb, s); break;
-    case 9: psf_width_launch<9>(rois, wle, sp, grid, tpb, s); break;
-    case 11: psf_width_launch<11>(rois, wle, sp, grid, tpb, s); break;
-    case 13: psf_width_launch<13>(rois, wle, sp, grid, tpb, s); break;
-    case 15: psf_width_launch<15>(rois, wle, sp, grid, tpb, s); break;
-    case 17: psf_width_launch<17>(rois, wle, sp, grid, tpb, s); break;
+        QCS_WIDTHS(5)
+        QCS_WIDTHS(7)
+        QCS_WIDTHS(9)
+        QCS_WIDTHS(11)
+        QCS_WIDTHS(13)
+        QCS_WIDTHS(15)
+        QCS_WIDTHS(17)
     default: return cudaErrorInvalidValue;
     }
-    return cudaSuccess;
+#undef QCS_WIDTHS
+    return cudaGetLastError();
 }
 
 size_t sort_temp_bytes(int n) {
@@ -351,16 +354,11 @@ inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 size_t wle_scratch_bytes(int n) {
     const size_t nn = (size_t)(n > 0 ? n : 1);
-    return 2 * align256(nn * 8) + 2 * align256(nn * 4) + align256(sort_temp_bytes((int)nn)) + align256(sizeof(int));
+    return 2 * align256(nn * 8) + 2 * align256(nn * 4) + align256(sort_temp_bytes((int)nn)) + align256(2 * sizeof(int));
 }
 
 cudaError_t launch_wle(const uint16_t *rois, int n, int R, int loc_type, float *wle, void *scratch, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    const int tpb = 64;
-    const int grid = (n + tpb - 1) / tpb;
-    const Span sp{0, n, nullptr};
-    cudaError_t e = launch_psf_width(R, rois, wle, sp, grid, tpb, s);
-    if (e != cudaSuccess) return e;
     const size_t nn = (size_t)n;
     char *p = static_cast<char *>(scratch);
     unsigned long long *k_in = reinterpret_cast<unsigned long long *>(p);
@@ -372,43 +370,27 @@ cudaError_t launch_wle(const uint16_t *rois, int n, int R, int loc_type, float *
     int *v_out = reinterpret_cast<int *>(p);
     p += align256(nn * 4);
     size_t temp = sort_temp_bytes(n);
-    const int whole = R * (R + 1);
-    nn_keys_kernel<<<grid, tpb, 0, s>>>(rois, n, whole, R * R, k_in, v_in);
+    cudaError_t e = launch_widths_keys(R, rois, n, wle, k_in, v_in, nullptr, s);
+    if (e != cudaSuccess) return e;
     e = cub::DeviceRadixSort::SortPairs(p, temp, k_in, k_out, v_in, v_out, n, 0, 64, s);
     if (e != cudaSuccess) return e;
-    nn_scan_kernel<<<grid, tpb, 0, s>>>(k_out, v_out, n, wle);
-    classify_kernel<<<grid, tpb, 0, s>>>(rois, wle, sp, R, whole, loc_type);
+    const int tpb = 64;
+    nn_scan_kernel<<<(n + tpb - 1) / tpb, tpb, 0, s>>>(k_out, v_out, n, rois, wle, R, loc_type);
     return cudaGetLastError();
 }
 
 namespace {
 
-// Keys of records [0, n) and padding (all ones, after every real key) up to
-// cap; *unsorted = 1 when some record's key is below its predecessor's.
-__global__ void nn_keys_flag_kernel(const uint16_t *__restrict__ rois, int n, int cap, int whole, int pix,
-                                    unsigned long long *__restrict__ keys, int *__restrict__ vals,
-                                    int *__restrict__ unsorted) {
+// Fills keys[*count .. cap) with padding (all ones, after every real key).
+__global__ void pad_keys_kernel(unsigned long long *__restrict__ keys, int *__restrict__ vals,
+                                const int *__restrict__ count, int cap) {
     const int i = threadIdx.x + blockDim.x * blockIdx.x;
-    bool bad = false;
-    if (i < cap) {
-        unsigned long long k = ~0ull;
-        if (i < n) {
-            const uint16_t *h = rois + (size_t)i * whole + pix;
-            k = (((unsigned long long)h[2] + 65536ull * h[3]) << 32) | ((unsigned long long)h[1] << 16) | h[0];
-            if (i > 0) {
-                const uint16_t *g = h - whole;
-                const unsigned long long kp =
-                    (((unsigned long long)g[2] + 65536ull * g[3]) << 32) | ((unsigned long long)g[1] << 16) | g[0];
-                bad = kp > k;
-            }
-        }
-        keys[i] = k;
-        vals[i] = i;
-    }
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(unsorted, 1);
+    if (i < *count || i >= cap) return;
+    keys[i] = ~0ull;
+    vals[i] = i;
 }
 
-// Sets the sort's IF condition from the flag of nn_keys_flag_kernel.
+// Sets the sort's IF condition from the flag of widths_keys_kernel.
 __global__ void wle_sort_cond_kernel(cudaGraphConditionalHandle h, const int *__restrict__ unsorted) {
     cudaGraphSetConditional(h, *unsorted ? 1u : 0u);
 }
@@ -417,13 +399,13 @@ __global__ void wle_sort_cond_kernel(cudaGraphConditionalHandle h, const int *__
 // else over the records' own keys (already sorted, identity order).
 __global__ void nn_scan_select_kernel(const unsigned long long *__restrict__ k_in, const unsigned long long *__restrict__ k_out,
                                       const int *__restrict__ v_out, const int *__restrict__ unsorted, int n,
-                                      float *__restrict__ wle) {
+                                      const uint16_t *__restrict__ rois, float *__restrict__ wle, int R, int LocType) {
     const int a = threadIdx.x + blockDim.x * blockIdx.x;
     if (a >= n) return;
-    if (*unsorted)
-        wle[(size_t)v_out[a] * QCS_WLE_PARA_NUM + 0] = nn_sorted(k_out, a, n);
-    else
-        wle[(size_t)a * QCS_WLE_PARA_NUM + 0] = nn_sorted(k_in, a, n);
+    const bool sorted = *unsorted == 0;
+    const int id = sorted ? a : v_out[a];
+    wle[(size_t)id * QCS_WLE_PARA_NUM + 0] = nn_sorted(sorted ? k_in : k_out, a, n);
+    classify_one(rois, wle, id, R, R * (R + 1), LocType);
 }
 
 }  // namespace
@@ -431,10 +413,10 @@ __global__ void nn_scan_select_kernel(const unsigned long long *__restrict__ k_i
 // The WLE pre-pass of a localization context.  Records produced by ROI
 // extraction (and most callers' batches) are already in (frame, y, x)
 // order; then the radix sort of the nearest-neighbour keys is the identity
-// and only costs time.  Here the keys kernel flags out-of-order records and
+// and only costs time.  Here widths_keys_kernel flags out-of-order records and
 // a CUDA graph holds the sort inside an IF node whose condition a one-thread
 // kernel sets from that flag, so the sort runs only when needed and the host
-// never waits.  The sort covers `capacity` keys (padding sorts last).
+// never waits.  The sort covers `capacity` keys (padded inside the node).
 struct WleSorter {
     int capacity = 0;
     void *scratch = nullptr;  // wle_scratch_bytes(capacity), owned by the caller
@@ -502,6 +484,7 @@ cudaError_t wle_sorter_create(int capacity, void *scratch, WleSorter **out) {
     if (e == cudaSuccess)
         e = cudaStreamBeginCaptureToGraph(w->cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed);
     if (e == cudaSuccess) {
+        pad_keys_kernel<<<(capacity + 255) / 256, 256, 0, w->cap>>>(w->k_in, w->v_in, w->flag + 1, capacity);
         cudaError_t es = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, w->k_in, w->k_out, w->v_in, w->v_out,
                                                          capacity, 0, 64, w->cap);
         cudaGraph_t captured = nullptr;
@@ -526,38 +509,32 @@ cudaError_t launch_wle_ctx(WleSorter *w, const uint16_t *rois, int n, int R, int
     if (e != cudaSuccess) return e;
     if (n > w->capacity || cs != cudaStreamCaptureStatusNone)
         return launch_wle(rois, n, R, loc_type, wle, w->scratch, s);
-    const int tpb = 64;
-    const int grid = (n + tpb - 1) / tpb;
-    const Span sp{0, n, nullptr};
-    e = launch_psf_width(R, rois, wle, sp, grid, tpb, s);
-    if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(w->flag, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
-    const int whole = R * (R + 1);
-    nn_keys_flag_kernel<<<(w->capacity + tpb - 1) / tpb, tpb, 0, s>>>(rois, n, w->capacity, whole, R * R, w->k_in,
-                                                                      w->v_in, w->flag);
+    e = launch_widths_keys(R, rois, n, wle, w->k_in, w->v_in, w->flag, s);
+    if (e != cudaSuccess) return e;
     e = cudaGraphLaunch(w->exec, s);
     if (e != cudaSuccess) return e;
-    nn_scan_select_kernel<<<grid, tpb, 0, s>>>(w->k_in, w->k_out, w->v_out, w->flag, n, wle);
-    classify_kernel<<<grid, tpb, 0, s>>>(rois, wle, sp, R, whole, loc_type);
+    const int tpb = 64;
+    nn_scan_select_kernel<<<(n + tpb - 1) / tpb, tpb, 0, s>>>(w->k_in, w->k_out, w->v_out, w->flag, n, rois, wle, R,
+                                                              loc_type);
     return cudaGetLastError();
 }
 
 cudaError_t launch_wle_presorted(const uint16_t *rois, const unsigned long long *keys, const int *d_span, int max_n,
                                  int R, int loc_type, float *wle, cudaStream_t s) {
     if (max_n <= 0) return cudaSuccess;
-    const int tpb = 64;
-    int grid = (max_n + tpb - 1) / tpb;
+    int grid = (max_n + kTile - 1) / kTile;
     if (grid > 148 * 8) grid = 148 * 8;
     const Span sp{0, 0, d_span};
     switch (R) {
-    case 5: wle_sorted_kernel<5><<<grid, tpb, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 7: wle_sorted_kernel<7><<<grid, tpb, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 9: wle_sorted_kernel<9><<<grid, tpb, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 11: wle_sorted_kernel<11><<<grid, tpb, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 13: wle_sorted_kernel<13><<<grid, tpb, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 15: wle_sorted_kernel<15><<<grid, tpb, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 17: wle_sorted_kernel<17><<<grid, tpb, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 5: wle_sorted_kernel<5><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 7: wle_sorted_kernel<7><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 9: wle_sorted_kernel<9><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 11: wle_sorted_kernel<11><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 13: wle_sorted_kernel<13><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 15: wle_sorted_kernel<15><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 17: wle_sorted_kernel<17><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
