@@ -139,7 +139,7 @@ struct Tile {
     uint32_t px[kTile * PITCH];
 };
 
-template <int R>
+template <int R, int THREADS = kTileThreads>
 __device__ __forceinline__ void tile_widths(Tile<R> &tile, const uint16_t *__restrict__ rois, float *__restrict__ wle,
                                             int first, int cnt) {
     typedef Tile<R> T;
@@ -147,15 +147,15 @@ __device__ __forceinline__ void tile_widths(Tile<R> &tile, const uint16_t *__res
     uint16_t *dst = reinterpret_cast<uint16_t *>(tile.px);
     if ((reinterpret_cast<uintptr_t>(src) & 3) == 0) {
         const uint32_t *s4 = reinterpret_cast<const uint32_t *>(src);
-        for (int i = threadIdx.x; i < cnt * T::WORDS; i += kTileThreads)
+        for (int i = threadIdx.x; i < cnt * T::WORDS; i += THREADS)
             tile.px[i / T::WORDS * T::PITCH + i % T::WORDS] = __ldg(s4 + i);
     } else {
-        for (int i = threadIdx.x; i < cnt * T::WHOLE; i += kTileThreads)
+        for (int i = threadIdx.x; i < cnt * T::WHOLE; i += THREADS)
             dst[i / T::WHOLE * (2 * T::PITCH) + i % T::WHOLE] = __ldg(src + i);
     }
     __syncthreads();
     const int rec = threadIdx.x % kTile, rows = threadIdx.x / kTile;
-    if (rec < cnt) {
+    if (rec < cnt && rows < 2) {
         const uint16_t *p = dst + rec * (2 * T::PITCH);
         int sum[R];
 #pragma unroll
@@ -278,22 +278,23 @@ __global__ void nn_scan_kernel(const unsigned long long *__restrict__ keys, cons
 // Records already in ascending (frame, y, x) order with their keys in a
 // compact array: PSF widths, nearest neighbour and molecule type of each
 // record in one pass (one thread per record).
+// One thread more per record looks for the neighbour while the other two take
+// the widths: a batch of frames has few tiles, so a tile's chain sets the time.
+constexpr int kSortedThreads = 3 * kTile;
 template <int R>
-__global__ void __launch_bounds__(kTileThreads) wle_sorted_kernel(const uint16_t *__restrict__ rois,
-                                                                  const unsigned long long *__restrict__ keys, Span sp,
-                                                                  float *__restrict__ wle, int LocType) {
+__global__ void __launch_bounds__(kSortedThreads) wle_sorted_kernel(const uint16_t *__restrict__ rois,
+                                                                    const unsigned long long *__restrict__ keys, Span sp,
+                                                                    float *__restrict__ wle, int LocType) {
     __shared__ Tile<R> tile;
     int b0, n;
     sp.get(b0, n);
     for (int a0 = blockIdx.x * kTile; a0 < n; a0 += gridDim.x * kTile) {
         const int cnt = min(kTile, n - a0);
-        tile_widths<R>(tile, rois, wle, b0 + a0, cnt);
-        __syncthreads();  // the tile's widths are written, its pixels free
-        if (threadIdx.x < cnt) {
-            const int a = a0 + threadIdx.x;
-            wle[(size_t)(b0 + a) * QCS_WLE_PARA_NUM + 0] = nn_sorted(keys + b0, a, n);
-            classify_one(rois, wle, b0 + a, R, R * (R + 1), LocType);
-        }
+        tile_widths<R, kSortedThreads>(tile, rois, wle, b0 + a0, cnt);
+        const int k = (int)threadIdx.x - 2 * kTile;
+        if (k >= 0 && k < cnt) wle[(size_t)(b0 + a0 + k) * QCS_WLE_PARA_NUM + 0] = nn_sorted(keys + b0, a0 + k, n);
+        __syncthreads();  // the tile's widths and distances are written, its pixels free
+        if (threadIdx.x < cnt) classify_one(rois, wle, b0 + a0 + threadIdx.x, R, R * (R + 1), LocType);
     }
 }
 
@@ -528,13 +529,13 @@ cudaError_t launch_wle_presorted(const uint16_t *rois, const unsigned long long 
     if (grid > 148 * 8) grid = 148 * 8;
     const Span sp{0, 0, d_span};
     switch (R) {
-    case 5: wle_sorted_kernel<5><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 7: wle_sorted_kernel<7><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 9: wle_sorted_kernel<9><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 11: wle_sorted_kernel<11><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 13: wle_sorted_kernel<13><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 15: wle_sorted_kernel<15><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
-    case 17: wle_sorted_kernel<17><<<grid, kTileThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 5: wle_sorted_kernel<5><<<grid, kSortedThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 7: wle_sorted_kernel<7><<<grid, kSortedThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 9: wle_sorted_kernel<9><<<grid, kSortedThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 11: wle_sorted_kernel<11><<<grid, kSortedThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 13: wle_sorted_kernel<13><<<grid, kSortedThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 15: wle_sorted_kernel<15><<<grid, kSortedThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
+    case 17: wle_sorted_kernel<17><<<grid, kSortedThreads, 0, s>>>(rois, keys, sp, wle, loc_type); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
