@@ -37,19 +37,62 @@ namespace {
 constexpr int kTPB = 256;
 constexpr int kBlockRows = 32;  // the reference's ThreadsPerBlock: the link scan starts at its block's first row
 
-__device__ __forceinline__ uint64_t link_key(int frame, int y) {
-    return ((uint64_t)(uint32_t)frame << 32) | (uint64_t)((uint32_t)y ^ 0x80000000u);
+// Frame and integer y ranges of the rows: [fmin, fmax, ymin, ymax].
+struct Ranges {
+    int v[4];
+};
+
+// Sort key of (frame, integer y): both counted from the rows' lowest, y in the
+// low `bits` bits, so that the sort takes only the digits the rows span (32
+// frames of a 512-pixel image: 2 passes of 8 bits instead of 8).
+struct LinkKey {
+    int f0, y0, bits;
+    __device__ __forceinline__ uint64_t operator()(int frame, int y) const {
+        return ((uint64_t)((uint32_t)frame - (uint32_t)f0) << bits) | (uint64_t)((uint32_t)y - (uint32_t)y0);
+    }
+};
+
+// Float-to-int as the reference's implicit conversions (truncation; NaN -> 0;
+// saturation).
+__global__ void __launch_bounds__(kTPB) ranges_kernel(const float *__restrict__ rows, int T, Ranges *__restrict__ out) {
+    int f0 = 0x7fffffff, f1 = -0x7fffffff - 1, y0 = f0, y1 = f1;
+    for (int i = blockIdx.x * kTPB + threadIdx.x; i < T; i += gridDim.x * kTPB) {
+        const float *r = rows + (size_t)i * 12;
+        const int f = (int)r[QCS_POS_FRME], y = (int)r[QCS_POS_YPOS];
+        f0 = min(f0, f);
+        f1 = max(f1, f);
+        y0 = min(y0, y);
+        y1 = max(y1, y);
+    }
+    f0 = __reduce_min_sync(0xffffffffu, f0);
+    f1 = __reduce_max_sync(0xffffffffu, f1);
+    y0 = __reduce_min_sync(0xffffffffu, y0);
+    y1 = __reduce_max_sync(0xffffffffu, y1);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(out->v, f0);
+        atomicMax(out->v + 1, f1);
+        atomicMin(out->v + 2, y0);
+        atomicMax(out->v + 3, y1);
+    }
 }
 
-// (frame, integer y) sort keys of the rows; float-to-int as the reference's
-// implicit conversions (truncation; NaN -> 0; saturation)
-__global__ void keys_kernel(const float *__restrict__ rows, int T, uint64_t *__restrict__ keys,
+__global__ void keys_kernel(const float *__restrict__ rows, int T, LinkKey key, uint64_t *__restrict__ keys,
                             int *__restrict__ vals) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= T) return;
     const float *r = rows + (size_t)i * 12;
-    keys[i] = link_key((int)r[QCS_POS_FRME], (int)r[QCS_POS_YPOS]);
+    keys[i] = key((int)r[QCS_POS_FRME], (int)r[QCS_POS_YPOS]);
     vals[i] = i;
+}
+
+// Integer x, y of the sorted rows side by side, so that the link search reads
+// its candidates from consecutive addresses.
+__global__ void sorted_xy_kernel(const float *__restrict__ rows, int T, const int *__restrict__ svals,
+                                 int2 *__restrict__ sxy) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= T) return;
+    const float *r = rows + (size_t)svals[j] * 12;
+    sxy[j] = make_int2((int)r[QCS_POS_XPOS], (int)r[QCS_POS_YPOS]);
 }
 
 // first index in [0, n) whose key is >= k
@@ -63,36 +106,51 @@ __device__ __forceinline__ int lower_bound(const uint64_t *__restrict__ a, int n
 }
 
 // gpuFindConsecutiveMolecules: bwd[i] = the closest row of the next frame
-// within the threshold (-2: none), fwd[that row] = 1.
-__global__ void link_kernel(const float *__restrict__ rows, int T, const uint64_t *__restrict__ skeys,
-                            const int *__restrict__ svals, float th_px, int *__restrict__ fwd, int *__restrict__ bwd) {
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= T) return;
-    const float *r1 = rows + (size_t)gid * 12;
-    const int X1 = (int)r1[QCS_POS_XPOS], Y1 = (int)r1[QCS_POS_YPOS], F1 = (int)r1[QCS_POS_FRME];
+// within the threshold (-2: none), fwd[that row] = 1.  Threads take the rows in
+// sorted order, so that neighbouring threads search and read the same lines,
+// and load four candidates at a time.
+__global__ void link_kernel(int T, LinkKey key, Ranges range, const uint64_t *__restrict__ skeys,
+                            const int *__restrict__ svals, const int2 *__restrict__ sxy, float th_px,
+                            int *__restrict__ fwd, int *__restrict__ bwd) {
+    const int me = blockIdx.x * blockDim.x + threadIdx.x;
+    if (me >= T) return;
+    const int gid = svals[me];
+    const int2 at = sxy[me];
+    const int X1 = at.x, Y1 = at.y, F1 = (int)((uint32_t)(skeys[me] >> key.bits) + (uint32_t)key.f0);
     float th2 = th_px;
     th2 = th2 * th2;
     int best = -1;
-    if (F1 < 0x7fffffff && th2 > 0.0f) {
+    if (F1 < range.v[1] && th2 > 0.0f) {  // no later frame: no link
         const int gid0 = gid - gid % kBlockRows;
         // every dy with dy * dy < th2, and one more
         const long long r = (long long)ceilf(sqrtf(th2));
         long long ylo = (long long)Y1 - r, yhi = (long long)Y1 + r;
-        if (ylo < -2147483648LL) ylo = -2147483648LL;
-        if (yhi > 2147483647LL) yhi = 2147483647LL;
-        const uint64_t klo = link_key(F1 + 1, (int)ylo), khi = link_key(F1 + 1, (int)yhi);
+        if (ylo < range.v[2]) ylo = range.v[2];
+        if (yhi > range.v[3]) yhi = range.v[3];
+        const uint64_t klo = key(F1 + 1, (int)ylo), khi = key(F1 + 1, (int)yhi);
         int bd = 0;
-        for (int j = lower_bound(skeys, T, klo); j < T && skeys[j] <= khi; ++j) {
-            const int c = svals[j];
-            if (c < gid0) continue;
-            const float *r2 = rows + (size_t)c * 12;
-            const unsigned dx = (unsigned)X1 - (unsigned)(int)r2[QCS_POS_XPOS];
-            const unsigned dy = (unsigned)Y1 - (unsigned)(int)r2[QCS_POS_YPOS];
-            const int d2 = (int)(dx * dx + dy * dy);
-            if (!((float)d2 < th2)) continue;
-            if (best < 0 || d2 < bd || (d2 == bd && c < best)) {
-                best = c;
-                bd = d2;
+        for (int j = lower_bound(skeys, T, klo); j < T && skeys[j] <= khi; j += 4) {
+            uint64_t k[4];
+            int c[4];
+            int2 q[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = min(j + u, T - 1);
+                k[u] = j + u < T ? skeys[i] : ~0ull;
+                c[u] = svals[i];
+                q[u] = sxy[i];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (k[u] > khi || c[u] < gid0) continue;
+                const unsigned dx = (unsigned)X1 - (unsigned)q[u].x;
+                const unsigned dy = (unsigned)Y1 - (unsigned)q[u].y;
+                const int d2 = (int)(dx * dx + dy * dy);
+                if (!((float)d2 < th2)) continue;
+                if (best < 0 || d2 < bd || (d2 == bd && c[u] < best)) {
+                    best = c[u];
+                    bd = d2;
+                }
             }
         }
     }
@@ -104,12 +162,9 @@ __global__ void link_kernel(const float *__restrict__ rows, int T, const uint64_
     }
 }
 
-// gpuConsecutiveFit: every row without a forward link takes its chain's sums
-// and precision-weighted averages; chains starting in the new group are counted.
-__global__ void merge_kernel(float *__restrict__ rows, int T, int last_n, const int *__restrict__ fwd,
-                             const int *__restrict__ bwd, float QE, int *__restrict__ stat) {
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= T || fwd[gid] != 0) return;
+// The chain that starts at row gid (gpuConsecutiveFit).
+__device__ __forceinline__ void merge_chain(float *__restrict__ rows, int gid, int last_n, const int *__restrict__ bwd,
+                                            float QE, int *on_time) {
     float wx = 0, wy = 0, wz = 0, wsx = 0, wsy = 0, sp = 0, st = 0, sb = 0, sprec = 0;
     int id = gid, num = 0;
     for (;;) {
@@ -140,8 +195,25 @@ __global__ void merge_kernel(float *__restrict__ rows, int T, int last_n, const 
     h[QCS_POS_PSNR] = __fdiv_rn(__fmul_rn(__fsqrt_rn(QE), sp), __fsqrt_rn(__fadd_rn(sp, sb)));
     if (gid >= last_n) {
         const int on = min(max(num - 1, 0), QCS_ONTIME_BINS - 1);
-        atomicAdd(stat + QCS_ONTIME_BINS, 1);
-        atomicAdd(stat + on, 1);
+        atomicAdd(on_time + on, 1);
+    }
+}
+
+// gpuConsecutiveFit: every row without a forward link takes its chain's sums
+// and precision-weighted averages; chains starting in the new group are counted.
+__global__ void merge_kernel(float *__restrict__ rows, int T, int last_n, const int *__restrict__ fwd,
+                             const int *__restrict__ bwd, float QE, int *__restrict__ stat) {
+    // the block's on-time histogram, added to the total once per block (every
+    // chain adding to the same eleven words took most of the kernel's time)
+    __shared__ int on_time[QCS_ONTIME_BINS];
+    for (int k = threadIdx.x; k < QCS_ONTIME_BINS; k += blockDim.x) on_time[k] = 0;
+    __syncthreads();
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gid < T && fwd[gid] == 0) merge_chain(rows, gid, last_n, bwd, QE, on_time);
+    __syncthreads();
+    if (threadIdx.x < QCS_ONTIME_BINS && on_time[threadIdx.x]) {
+        atomicAdd(stat + threadIdx.x, on_time[threadIdx.x]);
+        atomicAdd(stat + QCS_ONTIME_BINS, on_time[threadIdx.x]);
     }
 }
 
@@ -158,6 +230,14 @@ __global__ void remove_kernel(float *__restrict__ rows, int T, const int *__rest
 
 inline int blocks(int n) { return (n + kTPB - 1) / kTPB; }
 
+// bits (at least 1) that hold lo .. hi counted from lo
+inline int span_bits(int lo, int hi) {
+    const uint32_t span = (uint32_t)hi - (uint32_t)lo;
+    int bits = 1;
+    while (bits < 32 && (span >> bits)) ++bits;
+    return bits;
+}
+
 }  // namespace
 
 struct qcs_consec {
@@ -169,6 +249,7 @@ struct qcs_consec {
     int *d_fwd = nullptr, *d_bwd = nullptr;
     uint64_t *d_keys = nullptr, *d_skeys = nullptr;
     int *d_vals = nullptr, *d_svals = nullptr;
+    Ranges *d_range = nullptr, *h_range = nullptr;  // h_range pinned: [0] the empty range, [1] the rows'
     void *d_sort = nullptr;
     size_t sort_bytes = 0;
     int *d_stat = nullptr;    // on-time histogram, then the chain count
@@ -194,13 +275,22 @@ int consec_run(qcs_consec *c, const float *rows, bool device_rows, int n, int is
     QCS_CUDA(cudaMemsetAsync(c->d_fwd, 0, (size_t)(T > 0 ? T : 1) * sizeof(int), s), "links");
     QCS_CUDA(cudaMemsetAsync(c->d_stat, 0, (QCS_ONTIME_BINS + 1) * sizeof(int), s), "on-time histogram");
     if (T > 0) {
-        keys_kernel<<<blocks(T), kTPB, 0, s>>>(c->d_work, T, c->d_keys, c->d_vals);
+        QCS_CUDA(cudaMemcpyAsync(c->d_range, c->h_range, sizeof(Ranges), cudaMemcpyHostToDevice, s), "row ranges");
+        ranges_kernel<<<blocks(T) < 148 ? blocks(T) : 148, kTPB, 0, s>>>(c->d_work, T, c->d_range);
+        QCS_CUDA(cudaMemcpyAsync(c->h_range + 1, c->d_range, sizeof(Ranges), cudaMemcpyDeviceToHost, s), "row ranges");
+        QCS_CUDA(cudaStreamSynchronize(s), "row ranges");
+        const Ranges range = c->h_range[1];
+        const LinkKey key{range.v[0], range.v[2], span_bits(range.v[2], range.v[3])};
+        const int end_bit = key.bits + span_bits(range.v[0], range.v[1]);
+        keys_kernel<<<blocks(T), kTPB, 0, s>>>(c->d_work, T, key, c->d_keys, c->d_vals);
         size_t tb = c->sort_bytes;
-        QCS_CUDA(cub::DeviceRadixSort::SortPairs(c->d_sort, tb, c->d_keys, c->d_skeys, c->d_vals, c->d_svals, T, 0, 64,
-                                                 s),
+        QCS_CUDA(cub::DeviceRadixSort::SortPairs(c->d_sort, tb, c->d_keys, c->d_skeys, c->d_vals, c->d_svals, T, 0,
+                                                 end_bit, s),
                  "sort rows by frame and y");
+        int2 *sxy = reinterpret_cast<int2 *>(c->d_keys);  // the unsorted keys are done with
+        sorted_xy_kernel<<<blocks(T), kTPB, 0, s>>>(c->d_work, T, c->d_svals, sxy);
         const float th_px = p->ConsecFit_DistanceTh_nm / p->PixelSize;
-        link_kernel<<<blocks(T), kTPB, 0, s>>>(c->d_work, T, c->d_skeys, c->d_svals, th_px, c->d_fwd, c->d_bwd);
+        link_kernel<<<blocks(T), kTPB, 0, s>>>(T, key, range, c->d_skeys, c->d_svals, sxy, th_px, c->d_fwd, c->d_bwd);
         merge_kernel<<<blocks(T), kTPB, 0, s>>>(c->d_work, T, c->last_n, c->d_fwd, c->d_bwd, p->QE, c->d_stat);
         remove_kernel<<<blocks(T), kTPB, 0, s>>>(c->d_work, T, c->d_fwd, c->d_bwd);
         QCS_CUDA(cudaGetLastError(), "consecutive-frame kernels");
@@ -248,6 +338,8 @@ int qcs_consec_deinit(qcs_consec *c) {
     cudaFree(c->d_keys);
     cudaFree(c->d_sort);
     cudaFree(c->d_stat);
+    cudaFree(c->d_range);
+    cudaFreeHost(c->h_range);
     cudaFreeHost(c->h_out);
     cudaFreeHost(c->h_stat);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -282,6 +374,9 @@ int qcs_consec_init(int capacity, qcs_consec **out) {
     }
     if (e == cudaSuccess) e = cudaMalloc(&c->d_sort, c->sort_bytes > 0 ? c->sort_bytes : 1);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_stat, (QCS_ONTIME_BINS + 1) * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_range, sizeof(Ranges));
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&c->h_range, 2 * sizeof(Ranges));
+    if (e == cudaSuccess) c->h_range[0] = Ranges{{0x7fffffff, -0x7fffffff - 1, 0x7fffffff, -0x7fffffff - 1}};
     if (e == cudaSuccess) e = cudaMallocHost((void **)&c->h_out, T * 12 * sizeof(float));
     if (e == cudaSuccess) e = cudaMallocHost((void **)&c->h_stat, (QCS_ONTIME_BINS + 1) * sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);

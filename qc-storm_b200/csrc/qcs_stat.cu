@@ -37,7 +37,6 @@ constexpr float kGapPhoton = 10000.0f / kLen;
 constexpr float kGapPrec = 60.0f / kLen;
 constexpr float kGapSNR = 50.0f / kLen;
 constexpr float kGapPSF = 5.0f / kLen;
-constexpr uint64_t kKeyNone = ~0ull;
 
 __device__ __forceinline__ int bin(float v, float gap) {
     int b = (int)__fdiv_rn(v, gap);
@@ -85,39 +84,58 @@ __global__ void __launch_bounds__(kTPB) hist_kernel(const float *__restrict__ ro
     }
 }
 
-// block partial sums -> sums[5], in block order
-__global__ void sum_kernel(const float *__restrict__ part, int nblocks, float *__restrict__ sums) {
-    if (threadIdx.x >= 5) return;
+// block partial sums -> sums[5], in block order (one chain of additions per
+// sum, fed from shared memory)
+__global__ void __launch_bounds__(kTPB) sum_kernel(const float *__restrict__ part, int nblocks,
+                                                   float *__restrict__ sums) {
+    __shared__ float p[kTPB * 5];
     float s = 0;
-    for (int b = 0; b < nblocks; ++b) s += part[(size_t)b * 5 + threadIdx.x];
-    sums[threadIdx.x] = s;
-}
-
-// GetFirstFrame / GetLastFrame (bfgsMLE_Loc_top/bfgs_top.cu:345-381): index of
-// the first row with a nonzero frame, and of the last such row after row 0.
-__global__ void frame_ends_kernel(const float *__restrict__ rows, int n, int *__restrict__ ends) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if ((int)rows[(size_t)i * 12 + QCS_POS_FRME] != 0) {
-        atomicMin(ends, i);
-        if (i > 0) atomicMax(ends + 1, i);
+    for (int b0 = 0; b0 < nblocks; b0 += kTPB) {
+        const int nb = min(kTPB, nblocks - b0);
+        for (int i = threadIdx.x; i < nb * 5; i += kTPB) p[i] = part[(size_t)b0 * 5 + i];
+        __syncthreads();
+        if (threadIdx.x < 5)
+#pragma unroll 8
+            for (int b = 0; b < nb; ++b) s += p[b * 5 + threadIdx.x];
+        __syncthreads();
     }
+    if (threadIdx.x < 5) sums[threadIdx.x] = s;
 }
 
-__device__ __forceinline__ uint64_t cell_key(int frame, int cell) {
-    return ((uint64_t)(uint32_t)frame << 32) | (uint64_t)((uint32_t)cell ^ 0x80000000u);
+// GetFirstFrame / GetLastFrame (bfgsMLE_Loc_top/bfgs_top.cu:345-381): the
+// first row with a nonzero frame, and the last such row after row 0, each as
+// row index << 32 | the frame's bits (the index decides).
+__global__ void frame_ends_kernel(const float *__restrict__ rows, int n, unsigned long long *__restrict__ ends) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const float f = i < n ? rows[(size_t)i * 12 + QCS_POS_FRME] : 0.0f;
+    const unsigned set = __ballot_sync(0xffffffffu, (int)f != 0);
+    const int lane = threadIdx.x & 31;
+    const unsigned long long v = ((unsigned long long)(unsigned)i << 32) | __float_as_uint(f);
+    if (set && lane == __ffs(set) - 1) atomicMin(ends, v);
+    if (set && lane == 31 - __clz(set) && i > 0) atomicMax(ends + 1, v);
 }
+
+// Sort key of (frame, cell row): the frame from the first selected one, the
+// cell (-1 .. cells) plus one in the low `bits` bits, so that the sort takes
+// only the digits that occur; none: one above every key.
+struct CellKey {
+    int f0, bits;
+    uint64_t none;
+    __device__ __forceinline__ uint64_t operator()(int frame, int cell) const {
+        return ((uint64_t)((uint32_t)frame - (uint32_t)f0) << bits) | (uint64_t)(uint32_t)(cell + 1);
+    }
+};
 
 // FillerMoleculesInCurFrame's selection for every frame of [fs, fe] at once:
 // rows at least 5 px inside the image get a (frame, cell row) key, others none.
 __global__ void density_keys_kernel(const float *__restrict__ rows, int n, int fs, int fe, int W, int H, float rad,
-                                    uint64_t *__restrict__ keys, int *__restrict__ vals) {
+                                    CellKey key, uint64_t *__restrict__ keys, int *__restrict__ vals) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float *q = rows + (size_t)i * 12;
     const int xp = (int)q[QCS_POS_XPOS], yp = (int)q[QCS_POS_YPOS], f = (int)q[QCS_POS_FRME];
     const bool sel = xp >= 5 && xp < W - 5 && yp >= 5 && yp < H - 5 && f >= fs && f <= fe;
-    keys[i] = sel ? cell_key(f, (int)floorf(__fdiv_rn(q[QCS_POS_YPOS], rad))) : kKeyNone;
+    keys[i] = sel ? key(f, (int)floorf(__fdiv_rn(q[QCS_POS_YPOS], rad))) : key.none;
     vals[i] = i;
 }
 
@@ -132,30 +150,53 @@ __device__ __forceinline__ int lower_bound(const uint64_t *__restrict__ a, int n
 
 // CalcOverlapFluoNum: rows with no / one other selected row of their frame
 // within the radius (squared distance with separate roundings, <= rad^2).
-__global__ void density_count_kernel(const float *__restrict__ rows, int n, const uint64_t *__restrict__ skeys,
-                                     const int *__restrict__ svals, float rad, int *__restrict__ cnt) {
+__global__ void density_count_kernel(int n, CellKey ck, const uint64_t *__restrict__ skeys,
+                                     const float2 *__restrict__ sxy, float rad, int *__restrict__ cnt) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    int nb = -1;  // not a selected row
+    if (j < n && skeys[j] < ck.none) {
+        const uint64_t key = skeys[j];
+        const float2 me = sxy[j];
+        const float th2 = __fmul_rn(rad, rad);
+        nb = 0;
+        const uint64_t khi = key + 1;
+        // four candidates at a time: their loads overlap
+        for (int k = lower_bound(skeys, n, key - 1); k < n && skeys[k] <= khi && nb < 2; k += 4) {
+            uint64_t kk[4];
+            float2 o[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = min(k + u, n - 1);
+                kk[u] = k + u < n ? skeys[i] : ~0ull;
+                o[u] = sxy[i];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (kk[u] > khi || k + u == j) continue;
+                const float dx = __fsub_rn(o[u].x, me.x);
+                const float dy = __fsub_rn(o[u].y, me.y);
+                const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), 0.0f);
+                nb += (d2 <= th2);
+            }
+        }
+        nb = min(nb, 2);
+    }
+    const int c0 = __syncthreads_count(nb == 0), c1 = __syncthreads_count(nb == 1), c2 = __syncthreads_count(nb >= 0);
+    if (threadIdx.x == 0) {
+        if (c0) atomicAdd(cnt, c0);
+        if (c1) atomicAdd(cnt + 1, c1);
+        if (c2) atomicAdd(cnt + 2, c2);
+    }
+}
+
+// Positions of the sorted rows side by side, so that the count reads its
+// candidates from consecutive addresses.
+__global__ void sorted_xy_kernel(const float *__restrict__ rows, int n, const int *__restrict__ svals,
+                                 float2 *__restrict__ sxy) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
-    const uint64_t key = skeys[j];
-    if (key == kKeyNone) return;
-    const int me = svals[j];
-    const int frame = (int)(key >> 32);
-    const int cell = (int)((uint32_t)key ^ 0x80000000u);
-    const float cx = rows[(size_t)me * 12 + QCS_POS_XPOS], cy = rows[(size_t)me * 12 + QCS_POS_YPOS];
-    const float th2 = __fmul_rn(rad, rad);
-    int nb = 0;
-    const uint64_t khi = cell_key(frame, cell + 1);
-    for (int k = lower_bound(skeys, n, cell_key(frame, cell - 1)); k < n && skeys[k] <= khi && nb < 2; ++k) {
-        const int o = svals[k];
-        if (o == me) continue;
-        const float dx = __fsub_rn(rows[(size_t)o * 12 + QCS_POS_XPOS], cx);
-        const float dy = __fsub_rn(rows[(size_t)o * 12 + QCS_POS_YPOS], cy);
-        const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), 0.0f);
-        nb += (d2 <= th2);
-    }
-    if (nb == 0) atomicAdd(cnt, 1);
-    if (nb == 1) atomicAdd(cnt + 1, 1);
-    atomicAdd(cnt + 2, 1);
+    const float *r = rows + (size_t)svals[j] * 12;
+    sxy[j] = make_float2(r[QCS_POS_XPOS], r[QCS_POS_YPOS]);
 }
 
 inline int blocks(int n) { return (n + kTPB - 1) / kTPB; }
@@ -332,14 +373,14 @@ struct qcs_stat {
     int *d_hist = nullptr;    // 4 x 1600
     float *d_part = nullptr;  // per-block sums
     float *d_sums = nullptr;  // 5
-    int *d_ints = nullptr;    // frame ends (2), neighbour counts (3)
+    int *d_ints = nullptr;    // frame ends (two 64-bit words), neighbour counts (3)
     uint64_t *d_keys = nullptr, *d_skeys = nullptr;
     int *d_vals = nullptr, *d_svals = nullptr;
     void *d_sort = nullptr;
     size_t sort_bytes = 0;
     int *h_hist = nullptr;    // pinned, 4 x 1600: the last call's histograms
     float *h_sums = nullptr;  // pinned, 5
-    int *h_ints = nullptr;    // pinned, 5
+    int *h_ints = nullptr;    // pinned, 7
     float means[QCS_STAT_MEANS] = {0};
     float mean_ontime = 0;
     float ontime[QCS_ONTIME_BINS] = {0};
@@ -353,28 +394,29 @@ int stat_run(qcs_stat *st, const float *d_rows, int n, const qcs_loc_para *p, cu
     // CalcLocResultStatInf, then the histograms to the host and cleared
     const int nb = blocks(n);
     hist_kernel<<<nb, kTPB, 0, s>>>(d_rows, n, st->d_hist, st->d_part);
-    sum_kernel<<<1, 32, 0, s>>>(st->d_part, nb, st->d_sums);
-    const int init[2] = {0x7fffffff, -1};
-    QCS_CUDA(cudaMemcpyAsync(st->d_ints, init, sizeof(init), cudaMemcpyHostToDevice, s), "frame ends");
-    frame_ends_kernel<<<blocks(n), kTPB, 0, s>>>(d_rows, n, st->d_ints);
+    sum_kernel<<<1, kTPB, 0, s>>>(st->d_part, nb, st->d_sums);
+    unsigned long long *d_ends = reinterpret_cast<unsigned long long *>(st->d_ints);
+    const unsigned long long init[2] = {~0ull, 0ull};
+    QCS_CUDA(cudaMemcpyAsync(d_ends, init, sizeof(init), cudaMemcpyHostToDevice, s), "frame ends");
+    frame_ends_kernel<<<blocks(n), kTPB, 0, s>>>(d_rows, n, d_ends);
     QCS_CUDA(cudaGetLastError(), "statistics kernels");
-    QCS_CUDA(cudaMemcpyAsync(st->h_hist, st->d_hist, 4 * kLenMax * sizeof(int), cudaMemcpyDeviceToHost, s), "histograms");
+    // the histograms and, after them, the frame ends
+    QCS_CUDA(cudaMemcpyAsync(st->h_hist, st->d_hist, (4 * kLenMax + 4) * sizeof(int), cudaMemcpyDeviceToHost, s),
+             "histograms");
     QCS_CUDA(cudaMemcpyAsync(st->h_sums, st->d_sums, 5 * sizeof(float), cudaMemcpyDeviceToHost, s), "sums");
-    QCS_CUDA(cudaMemcpyAsync(st->h_ints, st->d_ints, 2 * sizeof(int), cudaMemcpyDeviceToHost, s), "frame ends");
     QCS_CUDA(cudaMemsetAsync(st->d_hist, 0, 4 * kLenMax * sizeof(int), s), "clear histograms");
     QCS_CUDA(cudaStreamSynchronize(s), "statistics");
     float vnum = st->h_sums[0];
     if (vnum <= 0) vnum = 1;
-    // GetFirstFrame / GetLastFrame from the row indices found on the device
+    // GetFirstFrame / GetLastFrame: the rows found on the device
     float fr[2] = {0, 0};
-    if (st->h_ints[0] < n)
-        QCS_CUDA(cudaMemcpy(&fr[0], d_rows + (size_t)st->h_ints[0] * 12 + QCS_POS_FRME, sizeof(float),
-                            cudaMemcpyDeviceToHost),
-                 "first frame");
-    if (st->h_ints[1] > 0)
-        QCS_CUDA(cudaMemcpy(&fr[1], d_rows + (size_t)st->h_ints[1] * 12 + QCS_POS_FRME, sizeof(float),
-                            cudaMemcpyDeviceToHost),
-                 "last frame");
+    unsigned long long ends[2];
+    memcpy(ends, st->h_ints, sizeof(ends));
+    for (int k = 0; k < 2; ++k) {
+        const bool found = k == 0 ? ends[0] != ~0ull : (ends[1] >> 32) > 0;
+        const uint32_t bits = (uint32_t)ends[k];
+        if (found) memcpy(&fr[k], &bits, sizeof(float));
+    }
     const int sf = (int)fr[0], ef = (int)fr[1];
     // CalcLocalizationDensity2D
     const float rad = (p->LocType == QCS_LOCTYPE_GS2D) ? 10.0f : 20.0f;
@@ -386,21 +428,29 @@ int stat_run(qcs_stat *st, const float *d_rows, int n, const qcs_loc_para *p, cu
     }
     int total = 0, c0 = 0, c1 = 0;
     if (fs <= fe) {
-        density_keys_kernel<<<blocks(n), kTPB, 0, s>>>(d_rows, n, fs, fe, p->ImageWidth, p->ImageHigh, rad, st->d_keys,
-                                                       st->d_vals);
+        // cells 0 .. H / rad, one more on either side, and `none` above every frame
+        CellKey key{fs, 1, 0};
+        while (key.bits < 32 && ((long long)(p->ImageHigh / rad) + 3) >> key.bits) ++key.bits;
+        key.none = ((uint64_t)((uint32_t)fe - (uint32_t)fs) + 1) << key.bits;
+        int end_bit = key.bits;
+        while (key.none >> end_bit) ++end_bit;
+        density_keys_kernel<<<blocks(n), kTPB, 0, s>>>(d_rows, n, fs, fe, p->ImageWidth, p->ImageHigh, rad, key,
+                                                       st->d_keys, st->d_vals);
         size_t tb = st->sort_bytes;
         QCS_CUDA(cub::DeviceRadixSort::SortPairs(st->d_sort, tb, st->d_keys, st->d_skeys, st->d_vals, st->d_svals, n, 0,
-                                                 64, s),
+                                                 end_bit, s),
                  "sort rows by frame and cell");
-        QCS_CUDA(cudaMemsetAsync(st->d_ints + 2, 0, 3 * sizeof(int), s), "neighbour counts");
-        density_count_kernel<<<blocks(n), kTPB, 0, s>>>(d_rows, n, st->d_skeys, st->d_svals, rad, st->d_ints + 2);
+        float2 *sxy = reinterpret_cast<float2 *>(st->d_keys);  // the unsorted keys are done with
+        sorted_xy_kernel<<<blocks(n), kTPB, 0, s>>>(d_rows, n, st->d_svals, sxy);
+        QCS_CUDA(cudaMemsetAsync(st->d_ints + 4, 0, 3 * sizeof(int), s), "neighbour counts");
+        density_count_kernel<<<blocks(n), kTPB, 0, s>>>(n, key, st->d_skeys, sxy, rad, st->d_ints + 4);
         QCS_CUDA(cudaGetLastError(), "density kernels");
-        QCS_CUDA(cudaMemcpyAsync(st->h_ints + 2, st->d_ints + 2, 3 * sizeof(int), cudaMemcpyDeviceToHost, s),
+        QCS_CUDA(cudaMemcpyAsync(st->h_ints + 4, st->d_ints + 4, 3 * sizeof(int), cudaMemcpyDeviceToHost, s),
                  "neighbour counts");
         QCS_CUDA(cudaStreamSynchronize(s), "density");
-        c0 = st->h_ints[2];
-        c1 = st->h_ints[3];
-        total = st->h_ints[4];
+        c0 = st->h_ints[4];
+        c1 = st->h_ints[5];
+        total = st->h_ints[6];
     }
     float *m = st->means;
     if (total > 50) {
