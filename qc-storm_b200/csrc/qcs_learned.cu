@@ -30,7 +30,7 @@
 namespace qcs {
 namespace learned {
 
-constexpr int kGemmThreads = 128;  // 4 warps: one tcgen05 GEMM tile of 128 rows
+constexpr int kGemmThreads = 256;  // 8 warps: one tcgen05 GEMM tile of 128 rows, two warps per 32 rows
 
 // One feature of record r (R x R pixels then header words): feature k of
 // in_width(R), given the record's photoelectron min lo, 1 / range inv and the
@@ -111,20 +111,78 @@ __global__ void targets_kernel(const uint16_t *__restrict__ rois, const float *_
 // C(m, n) = beta * C(m, n) + sum_k A(m, k) B(k, n), M x N x K, with
 // A(m, k) = A[m * sam + k * sak], B(k, n) = B[k * sbk + n * sbn] (FP32 in
 // memory, rounded to BF16 for the tensor cores), C row-major with ldc.
-// One CTA of 128 threads per 128 x bn tile (bn <= 256, a multiple of 16) and
-// K range: the threads stage 64-deep K chunks of both operands into shared
-// memory in the UMMA layout (double-buffered), one thread issues four
-// tcgen05.mma (M = 128, K = 16) per chunk into an FP32 accumulator in tensor
-// memory, and each warp reads its 32 rows back with tcgen05.ld.  With split-K
+// One CTA of 256 threads per 128 x bn tile (bn <= 256, a multiple of 16) and
+// K range: the threads stage 128-deep K chunks of both operands into shared
+// memory in the UMMA layout (double-buffered), one thread issues a
+// tcgen05.mma (M = 128) per 16 of K into an FP32 accumulator in tensor
+// memory, and two warps read each 32 rows back with tcgen05.ld.  With split-K
 // (gridDim.z > 1) CTA z sums K range [z kper, (z + 1) kper) into
 // part[z][M][N] and gemm_reduce_kernel adds the splits in order, so results
-// do not depend on scheduling.
-constexpr int kGemmM = 128, kGemmK = 64;
+// do not depend on scheduling.  The training products (K of 8 to 128 per CTA)
+// are bound by that chain of latencies, load, staging, MMA, read-back, not by
+// the tensor cores: the 128-deep chunk leaves most of them one trip (64 deep:
+// two, 6 us more over the eight of a gradient), 256 threads keep twice the
+// loads in flight, and bias, ReLU and mask go with the store instead of a
+// launch and a pass over the matrix each.  Gradient of 4,096 records: 303 ->
+// 182 us.
+constexpr int kGemmM = 128, kGemmK = 128;
+
+// What a GEMM's result goes through before it is stored (only unsplit, beta
+// 0): C += bias per column, act = relu(C); or C = 0 where mask <= 0 (the
+// gradient through a ReLU whose input was mask).  Null: nothing.
+struct GemmEpilogue {
+    const float *bias = nullptr;
+    float *act = nullptr;
+    const float *mask = nullptr;
+};
+
+// One chunk (kc deep, a multiple of 16) of an operand whose K elements are
+// adjacent in memory (element (r, k) at src[r * ld + k], 16-byte aligned rows)
+// into its UMMA image of `rows` rows: a warp takes 8 rows x 16 K at a time, 64 bytes of each row,
+// and stores 8-byte halves of core-matrix rows, so the loads use whole sectors
+// and the stores all banks.  (One thread per row, as for an operand with
+// adjacent rows, touches 32 sectors a load: 25 us for a 4096 x 128 x 128
+// product.)
+__device__ __forceinline__ void stage_k_rows(uint8_t *img, int rows, const float *__restrict__ src, long long ld, int r0,
+                                             int limit, int k0, int ke, int kc) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k4 = lane & 3;
+    const int groups = rows / 8;  // of 8 rows
+    int r8 = warp, k16 = 0;       // this step's rows and K
+    while (r8 >= groups) {
+        r8 -= groups;
+        k16 += 16;
+    }
+#pragma unroll 16
+    for (int u = warp; u < groups * (kc / 16); u += kGemmThreads / 32) {
+        const int r = r8 * 8 + (lane >> 2), k = k16 + k4 * 4, gr = r0 + r, gk = k0 + k;
+        r8 += kGemmThreads / 32;
+        while (r8 >= groups) {
+            r8 -= groups;
+            k16 += 16;
+        }
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (gr < limit) {
+            const float *s = src + (long long)gr * ld + gk;
+            if (gk + 3 < ke) {
+                v = __ldg(reinterpret_cast<const float4 *>(s));
+            } else {
+                if (gk < ke) v.x = __ldg(s);
+                if (gk + 1 < ke) v.y = __ldg(s + 1);
+                if (gk + 2 < ke) v.z = __ldg(s + 2);
+            }
+        }
+        __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v.x, v.y), __floats2bfloat162_rn(v.z, v.w)};
+        *reinterpret_cast<uint2 *>(img + (size_t)((k >> 3) * rows + r) * 16 + (k4 & 1) * 8) = *reinterpret_cast<uint2 *>(h);
+    }
+}
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_tc_kernel(int M, int N, int K, int bn, const float *__restrict__ A, long long sam, long long sak,
                    const float *__restrict__ B, long long sbk, long long sbn, float *__restrict__ Cm, int ldc,
-                   float beta, int kper, float *__restrict__ part, int *__restrict__ err) {
+                   float beta, int kper, float *__restrict__ part, int *__restrict__ err, GemmEpilogue ep) {
+    // operands with adjacent K elements and 16-byte aligned rows
+    const bool a_rows = sak == 1 && (sam & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    const bool b_rows = sbk == 1 && (sbn & 3) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
     const uint32_t sbase = (raw + 127u) & ~127u;
@@ -156,34 +214,43 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     int issued = 0;  // chunks whose MMAs were issued
     for (int c = 0; c < nchunks; ++c) {
         const int buf = c & 1, k0 = kb + c * kGemmK;
+        const int kc = min(kGemmK, (ke - k0 + 15) & ~15);  // this chunk's depth
         if (c >= 2) {  // the MMAs of chunk c - 2 have read this buffer
             ok = __syncthreads_and(tc::mbar_wait(sBar + 8 * buf, ((c - 2) >> 1) & 1));
             if (!ok) break;
         }
         uint8_t *a_img = base + buf * a_bytes, *b_img = base + 2 * a_bytes + buf * b_bytes;
-        // A: row tid, K groups 0..7 of the chunk
-        const int gm = m0 + tid;
+        if (a_rows) {
+            stage_k_rows(a_img, kGemmM, A, sam, m0, M, k0, ke, kc);
+        } else {
+            // row tid % 128, every other K group of the chunk
+            const int row = tid & (kGemmM - 1), gm = m0 + row;
+#pragma unroll 8
+            for (int kg = tid / kGemmM; kg < kc / 8; kg += kGemmThreads / kGemmM) {
+                float v[8];
 #pragma unroll
-        for (int kg = 0; kg < kGemmK / 8; ++kg) {
-            float v[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int gk = k0 + kg * 8 + e;
-                v[e] = (gm < M && gk < ke) ? __ldg(A + (long long)gm * sam + (long long)gk * sak) : 0.0f;
+                for (int e = 0; e < 8; ++e) {
+                    const int gk = k0 + kg * 8 + e;
+                    v[e] = (gm < M && gk < ke) ? __ldg(A + (long long)gm * sam + (long long)gk * sak) : 0.0f;
+                }
+                *reinterpret_cast<uint4 *>(a_img + (size_t)(kg * kGemmM + row) * 16) = tc::pack8(v);
             }
-            *reinterpret_cast<uint4 *>(a_img + (size_t)(kg * kGemmM + tid) * 16) = tc::pack8(v);
         }
-        // B: bn rows (n) x 8 K groups
+        if (b_rows) {
+            stage_k_rows(b_img, bn, B, sbn, n0, N, k0, ke, kc);
+        } else {
+            // bn rows (n) x 8 K groups
 #pragma unroll 4
-        for (int u = tid; u < bn * (kGemmK / 8); u += kGemmThreads) {
-            const int kg = u / bn, nn = u - kg * bn, gn = n0 + nn;
-            float v[8];
+            for (int u = tid; u < bn * (kc / 8); u += kGemmThreads) {
+                const int kg = u / bn, nn = u - kg * bn, gn = n0 + nn;
+                float v[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int gk = k0 + kg * 8 + e;
-                v[e] = (gn < N && gk < ke) ? __ldg(B + (long long)gk * sbk + (long long)gn * sbn) : 0.0f;
+                for (int e = 0; e < 8; ++e) {
+                    const int gk = k0 + kg * 8 + e;
+                    v[e] = (gn < N && gk < ke) ? __ldg(B + (long long)gk * sbk + (long long)gn * sbn) : 0.0f;
+                }
+                *reinterpret_cast<uint4 *>(b_img + (size_t)(kg * bn + nn) * 16) = tc::pack8(v);
             }
-            *reinterpret_cast<uint4 *>(b_img + (size_t)(kg * bn + nn) * 16) = tc::pack8(v);
         }
         tc::fence_async_smem();
         tc::fence_before();
@@ -191,8 +258,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         tc::fence_after();
         if (tid == 0) {
             const uint32_t a0 = sA + buf * a_bytes, b0 = sB + buf * b_bytes;
-#pragma unroll
-            for (int ks = 0; ks < kGemmK / 16; ++ks)
+            for (int ks = 0; ks < kc / 16; ++ks)
                 tc::mma_bf16(tmem, tc::smem_desc(a0 + ks * 2 * kGemmM * 16, kGemmM * 16, 128),
                              tc::smem_desc(b0 + ks * 2 * bn * 16, bn * 16, 128), idesc, (c > 0 || ks > 0) ? 1u : 0u);
             tc::mma_commit(sBar + 8 * buf);
@@ -208,36 +274,56 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     tc::fence_after();
     if (ok) {
         // 64 columns at a time through shared memory (the operand buffers are
-        // free once the last MMA has ended): each thread stores its row, then
-        // each warp writes whole rows, lanes along the columns (coalesced)
+        // free once the last MMA has ended): a warp of each half stores 32
+        // columns of its 32 rows, then each warp writes 16 whole rows, lanes along
+        // the columns (coalesced), what they read for it loaded ahead
         float *stage = reinterpret_cast<float *>(base);  // [128][65]
         float *out = part ? part + (size_t)blockIdx.z * M * N : Cm;
         const long long ld = part ? N : ldc;
         const float b = part ? 0.0f : beta;
+        const int quarter = warp & 3, half = warp >> 2;
         for (int c0 = 0; c0 < bn; c0 += 64) {
 #pragma unroll
-            for (int q = 0; q < 64; q += 16) {
+            for (int i = 0; i < 2; ++i) {
+                const int q = half * 32 + i * 16;
+                if (c0 + q >= bn) break;
                 float v[16];
                 if (issued > 0) {
-                    tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c0 + q, v);
+                    tc::tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + c0 + q, v);
                 } else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] = 0.0f;
                 }
 #pragma unroll
-                for (int j = 0; j < 16; ++j) stage[tid * 65 + q + j] = v[j];
+                for (int j = 0; j < 16; ++j) stage[(quarter * 32 + lane) * 65 + q + j] = v[j];
             }
             __syncthreads();
-            for (int r = warp * 32; r < warp * 32 + 32; ++r) {
-                const int row = m0 + r;
-                if (row >= M) break;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int c = c0 + h * 32 + lane, col = n0 + c;
-                    if (c < bn && col < N) {
-                        float *dst = out + (size_t)row * ld + col;
-                        const float v = stage[r * 65 + h * 32 + lane];
-                        *dst = (b == 0.0f) ? v : b * (*dst) + v;
+            for (int h = 0; h < 2; ++h) {
+                const int c = c0 + h * 32 + lane, col = n0 + c;
+                if (c < bn && col < N) {
+                    const float bias = ep.bias ? __ldg(ep.bias + col) : 0.0f;
+                    float old[16];
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        const int row = m0 + warp * 16 + r;
+                        const size_t at = (size_t)row * ld + col;
+                        old[r] = row >= M ? 0.0f : (ep.mask ? __ldg(ep.mask + at) : (b != 0.0f ? out[at] : 0.0f));
+                    }
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        const int row = m0 + warp * 16 + r;
+                        if (row >= M) break;
+                        const size_t at = (size_t)row * ld + col;
+                        float v = stage[(warp * 16 + r) * 65 + h * 32 + lane];
+                        if (ep.mask) {
+                            if (!(old[r] > 0.0f)) v = 0.0f;
+                        } else if (b != 0.0f) {
+                            v = b * old[r] + v;
+                        }
+                        if (ep.bias) v += bias;
+                        out[at] = v;
+                        if (ep.act) ep.act[at] = fmaxf(v, 0.0f);
                     }
                 }
             }
@@ -267,23 +353,29 @@ __global__ void gemm_reduce_kernel(const float *__restrict__ part, int splits, i
 size_t gemm_smem_bytes(int bn) { return 2 * (size_t)(kGemmM + bn) * kGemmK * 2 + 32 + 128; }
 
 // Split count for an M x N x K GEMM: enough CTAs to cover the SMs, at least
-// four K chunks per split, and partials within `ws_floats`.
+// 256 of K per split, and partials within `ws_floats`.
 int gemm_splits(int M, int N, int K, int bn, size_t ws_floats) {
     const int tiles = ((M + kGemmM - 1) / kGemmM) * ((N + bn - 1) / bn);
     int s = 148 / tiles;
-    const int by_k = K / (4 * kGemmK);
+    const int by_k = K / 256;
     if (s > by_k) s = by_k;
     if (s > 64) s = 64;
     while (s > 1 && (size_t)s * M * N > ws_floats) --s;
     return s < 1 ? 1 : s;
 }
 
-cudaError_t gemm(int M, int N, int K, const float *A, long long sam, long long sak, const float *B, long long sbk,
-                 long long sbn, float *C, int ldc, float beta, cudaStream_t s, float *ws, size_t ws_floats, int *err) {
+static cudaError_t gemm_epilogue(int M, int N, int K, const float *A, long long sam, long long sak, const float *B,
+                                 long long sbk, long long sbn, float *C, int ldc, float beta, cudaStream_t s, float *ws,
+                                 size_t ws_floats, int *err, const GemmEpilogue &ep) {
     if (M <= 0 || N <= 0) return cudaSuccess;
     int bn = ((N + 15) / 16) * 16;
     if (bn > 256) bn = 256;
-    const int splits = ws ? gemm_splits(M, N, K, bn, ws_floats) : 1;
+    // narrower tiles while they leave SMs without one: a tile's time is a chain
+    // of load latencies, and its B operand and epilogue shrink with it
+    const int m_tiles = (M + kGemmM - 1) / kGemmM;
+    while (bn >= 64 && bn % 32 == 0 && m_tiles * ((N + bn - 1) / bn) < 74) bn /= 2;
+    const bool plain = !ep.bias && !ep.act && !ep.mask;
+    const int splits = ws && plain ? gemm_splits(M, N, K, bn, ws_floats) : 1;
     int kper = (K + splits - 1) / splits;
     kper = ((kper + kGemmK - 1) / kGemmK) * kGemmK;
     const int z = kper > 0 ? (K + kper - 1) / kper : 1;
@@ -298,40 +390,43 @@ cudaError_t gemm(int M, int N, int K, const float *A, long long sam, long long s
     dim3 grid((N + bn - 1) / bn, (M + kGemmM - 1) / kGemmM, z > 1 ? z : 1);
     float *part = z > 1 ? ws : nullptr;
     gemm_tc_kernel<<<grid, kGemmThreads, smem, s>>>(M, N, K, bn, A, sam, sak, B, sbk, sbn, C, ldc, beta,
-                                                    z > 1 ? kper : (K > 0 ? K : 0), part, err);
+                                                    z > 1 ? kper : (K > 0 ? K : 0), part, err, ep);
     if (z > 1)
         gemm_reduce_kernel<<<(int)(((long long)M * N + 255) / 256), 256, 0, s>>>(part, z, M, N, C, ldc, beta);
     return cudaGetLastError();
 }
 
+cudaError_t gemm(int M, int N, int K, const float *A, long long sam, long long sak, const float *B, long long sbk,
+                 long long sbn, float *C, int ldc, float beta, cudaStream_t s, float *ws, size_t ws_floats, int *err) {
+    return gemm_epilogue(M, N, K, A, sam, sak, B, sbk, sbn, C, ldc, beta, s, ws, ws_floats, err, GemmEpilogue{});
+}
+
 // ------------------------------------------------------ elementwise layers
-// Z (rows x cols) += bias; A = relu(Z) (A may alias Z when the caller does not need Z).
-__global__ void bias_relu_kernel(float *__restrict__ Z, const float *__restrict__ bias, int rows, int cols,
-                                 float *__restrict__ A, int relu) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)rows * cols) return;
-    const float z = Z[i] + bias[i % cols];
-    Z[i] = z;
-    A[i] = relu ? fmaxf(z, 0.0f) : z;
-}
+// Column sums of d (rows x cols) into out, for up to three matrices in one
+// launch pair, two passes with a fixed order: block (x, y, z) sums split y's
+// rows of 32 columns of matrix z into part[z][y][cols]; then the second kernel
+// adds the splits in order.
+struct ColumnSums {
+    const float *d;
+    int cols;
+    float *out;
+};
+struct ColumnSums3 {
+    ColumnSums m[3];
+};
+constexpr int kColsumStride = 256;  // columns of a matrix at most (several matrices in one launch)
 
-// dZ = dA * (Z > 0)
-__global__ void relu_back_kernel(float *__restrict__ dA, const float *__restrict__ Z, long long total) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    if (!(Z[i] > 0.0f)) dA[i] = 0.0f;
-}
-
-// Column sums of d (rows x cols), two passes with a fixed order: block
-// (x, z) sums split z's rows of 32 columns into part[z][cols]; then
-// colsum_final adds the splits in order.
-__global__ void colsum_part_kernel(const float *__restrict__ d, long long rows, int cols, float *__restrict__ part) {
+__global__ void colsum_part_kernel(ColumnSums3 a, long long rows, float *__restrict__ part, int stride) {
     __shared__ float acc[8][33];
+    const float *d = a.m[blockIdx.z].d;
+    const int cols = a.m[blockIdx.z].cols;
     const int c = blockIdx.x * 32 + threadIdx.x;
+    if (blockIdx.x * 32 >= cols) return;
     const long long per = (rows + gridDim.y - 1) / gridDim.y;
     const long long r0 = (long long)blockIdx.y * per, r1 = r0 + per < rows ? r0 + per : rows;
     float s = 0.0f;
     if (c < cols)
+#pragma unroll 8
         for (long long r = r0 + threadIdx.y; r < r1; r += 8) s += d[r * cols + c];
     acc[threadIdx.y][threadIdx.x] = s;
     __syncthreads();
@@ -339,36 +434,52 @@ __global__ void colsum_part_kernel(const float *__restrict__ d, long long rows, 
         float t = 0.0f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) t += acc[k][threadIdx.x];
-        part[(size_t)blockIdx.y * cols + c] = t;
+        part[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * stride + c] = t;
     }
 }
 
-__global__ void colsum_final_kernel(const float *__restrict__ part, int splits, int cols, float *__restrict__ g) {
+__global__ void colsum_final_kernel(ColumnSums3 a, const float *__restrict__ part, int splits, int stride) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
+    if (c >= a.m[blockIdx.z].cols) return;
     float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += part[(size_t)z * cols + c];
-    g[c] = s;
+#pragma unroll 16
+    for (int z = 0; z < splits; ++z) s += part[((size_t)blockIdx.z * splits + z) * stride + c];
+    a.m[blockIdx.z].out[c] = s;
+}
+
+static int colsum_splits(long long rows) {
+    int splits = (int)((rows + 255) / 256);
+    if (splits > kColsumSplits) splits = kColsumSplits;
+    return splits < 1 ? 1 : splits;
 }
 
 cudaError_t column_sums(const float *d, long long rows, int cols, float *g, float *part, cudaStream_t s) {
-    int splits = (int)((rows + 255) / 256);
-    if (splits > kColsumSplits) splits = kColsumSplits;
-    if (splits < 1) splits = 1;
-    colsum_part_kernel<<<dim3((cols + 31) / 32, splits), dim3(32, 8), 0, s>>>(d, rows, cols, part);
-    colsum_final_kernel<<<(cols + 127) / 128, 128, 0, s>>>(part, splits, cols, g);
+    const int splits = colsum_splits(rows);
+    const ColumnSums3 a{{{d, cols, g}, {}, {}}};
+    colsum_part_kernel<<<dim3((cols + 31) / 32, splits, 1), dim3(32, 8), 0, s>>>(a, rows, part, cols);
+    colsum_final_kernel<<<dim3((cols + 127) / 128, 1, 1), 128, 0, s>>>(a, part, splits, cols);
     return cudaGetLastError();
 }
 
-// Masked weighted MSE on the first nused outputs plus, where cls is set and
-// cls[i] >= 0 (GS2D networks), kCountWeight x the softmax cross-entropy of
-// the count logits against class cls[i]: loss and dY.
-__global__ void mse_kernel(const float *__restrict__ Y, const float *__restrict__ T, const float *__restrict__ valid,
-                           const float *__restrict__ cls, int rows, int nout, int nused, int wrow, float inv_count,
-                           float *__restrict__ dY,
-                           float *__restrict__ loss) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows) return;
+// Three matrices of at most kColsumStride columns; part holds 3 kColsumSplits kColsumStride floats.
+static cudaError_t column_sums3(const ColumnSums (&m)[3], long long rows, float *part, cudaStream_t s) {
+    const int splits = colsum_splits(rows);
+    const ColumnSums3 a{{m[0], m[1], m[2]}};
+    colsum_part_kernel<<<dim3(kColsumStride / 32, splits, 3), dim3(32, 8), 0, s>>>(a, rows, part, kColsumStride);
+    colsum_final_kernel<<<dim3(kColsumStride / 128, 1, 3), 128, 0, s>>>(a, part, splits, kColsumStride);
+    return cudaGetLastError();
+}
+
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// One record of mse_kernel: its dY, and its loss times the batch size.
+__device__ __forceinline__ float mse_row(const float *__restrict__ Y, const float *__restrict__ T,
+                                         const float *__restrict__ valid, const float *__restrict__ cls, int i, int nout,
+                                         int nused, int wrow, float inv_count, float *__restrict__ dY) {
     const float v = valid[i];
     const float *y = Y + (size_t)i * nout;
     float l = 0.0f;
@@ -392,9 +503,21 @@ __global__ void mse_kernel(const float *__restrict__ Y, const float *__restrict_
         for (int j = 0; j < kClasses; ++j)
             dY[(size_t)i * nout + kCount0 + j] = kCountWeight * (e[j] / sum - (j == label ? 1.0f : 0.0f)) * inv_count;
     }
-    atomicAdd(loss, l * inv_count);
+    return l;
 }
 
+// Masked weighted MSE on the first nused outputs plus, where cls is set and
+// cls[i] >= 0 (GS2D networks), kCountWeight x the softmax cross-entropy of
+// the count logits against class cls[i]: loss and dY.
+__global__ void mse_kernel(const float *__restrict__ Y, const float *__restrict__ T, const float *__restrict__ valid,
+                           const float *__restrict__ cls, int rows, int nout, int nused, int wrow, float inv_count,
+                           float *__restrict__ dY,
+                           float *__restrict__ loss) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const float l = i < rows ? mse_row(Y, T, valid, cls, i, nout, nused, wrow, inv_count, dY) : 0.0f;
+    const float sum = warp_sum(l);
+    if ((threadIdx.x & 31) == 0) atomicAdd(loss, sum * inv_count);  // whole warps: 256-thread blocks
+}
 __global__ void adam_kernel(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
                             float *__restrict__ v, int n, float lr, float b1, float b2, float c1, float c2, float eps) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -799,18 +922,22 @@ cudaError_t forward(qcs_learned_net *net, const float *x, int rows, float *z1, f
         return L::conv::forward(net->conv, net->d_par, x, rows, net->kin, y, s, net->d_ws, net->ws_floats, net->d_err);
     const Views w = views(net->d_par, net->kin, net->nout);
     cudaError_t e;
-    if ((e = L::gemm(rows, L::kHidden, net->kin, x, net->kin, 1, w.W1, L::kHidden, 1, z1, L::kHidden, 0.0f, s, net->d_ws, net->ws_floats, net->d_err)))
+    L::GemmEpilogue ep;
+    ep.bias = w.b1;
+    ep.act = a1;
+    if ((e = L::gemm_epilogue(rows, L::kHidden, net->kin, x, net->kin, 1, w.W1, L::kHidden, 1, z1, L::kHidden, 0.0f, s,
+                              net->d_ws, net->ws_floats, net->d_err, ep)))
         return e;
-    L::bias_relu_kernel<<<blocks((long long)rows * L::kHidden), 256, 0, s>>>(z1, w.b1, rows, L::kHidden, a1, 1);
-    if ((e = L::gemm(rows, L::kHidden, L::kHidden, a1, L::kHidden, 1, w.W2, L::kHidden, 1, z2, L::kHidden, 0.0f, s, net->d_ws, net->ws_floats, net->d_err)))
+    ep.bias = w.b2;
+    ep.act = a2;
+    if ((e = L::gemm_epilogue(rows, L::kHidden, L::kHidden, a1, L::kHidden, 1, w.W2, L::kHidden, 1, z2, L::kHidden, 0.0f,
+                              s, net->d_ws, net->ws_floats, net->d_err, ep)))
         return e;
-    L::bias_relu_kernel<<<blocks((long long)rows * L::kHidden), 256, 0, s>>>(z2, w.b2, rows, L::kHidden, a2, 1);
     const int no = net->nout;
-    if ((e = L::gemm(rows, no, L::kHidden, a2, L::kHidden, 1, w.W3, no, 1, y, no, 0.0f, s, net->d_ws, net->ws_floats,
-                     net->d_err)))
-        return e;
-    L::bias_relu_kernel<<<blocks((long long)rows * no), 256, 0, s>>>(y, w.b3, rows, no, y, 0);
-    return cudaGetLastError();
+    ep.bias = w.b3;
+    ep.act = nullptr;
+    return L::gemm_epilogue(rows, no, L::kHidden, a2, L::kHidden, 1, w.W3, no, 1, y, no, 0.0f, s, net->d_ws,
+                            net->ws_floats, net->d_err, ep);
 }
 
 // Backward of the masked MSE for one batch already forwarded; fills d_grad.
@@ -826,28 +953,27 @@ cudaError_t backward(qcs_learned_net *net, int rows, cudaStream_t s) {
     if ((e = L::gemm(L::kHidden, no, rows, net->d_a2, 1, L::kHidden, net->d_dy, no, 1, g.W3, no, 0.0f,
                      s, net->d_ws, net->ws_floats, net->d_err)))
         return e;
-    if ((e = L::column_sums(net->d_dy, rows, no, g.b3, net->d_ws, s))) return e;
-    if ((e = L::gemm(rows, L::kHidden, no, net->d_dy, no, 1, w.W3, 1, no, net->d_d2, L::kHidden, 0.0f,
-                     s, net->d_ws, net->ws_floats, net->d_err)))
+    // d2 = (dy W3^T) masked by z2 > 0
+    L::GemmEpilogue ep;
+    ep.mask = net->d_z2;
+    if ((e = L::gemm_epilogue(rows, L::kHidden, no, net->d_dy, no, 1, w.W3, 1, no, net->d_d2, L::kHidden, 0.0f, s,
+                              net->d_ws, net->ws_floats, net->d_err, ep)))
         return e;
-    L::relu_back_kernel<<<blocks((long long)rows * L::kHidden), 256, 0, s>>>(net->d_d2, net->d_z2,
-                                                                           (long long)rows * L::kHidden);
     // layer 2
     if ((e = L::gemm(L::kHidden, L::kHidden, rows, net->d_a1, 1, L::kHidden, net->d_d2, L::kHidden, 1, g.W2,
                      L::kHidden, 0.0f, s, net->d_ws, net->ws_floats, net->d_err)))
         return e;
-    if ((e = L::column_sums(net->d_d2, rows, L::kHidden, g.b2, net->d_ws, s))) return e;
-    if ((e = L::gemm(rows, L::kHidden, L::kHidden, net->d_d2, L::kHidden, 1, w.W2, 1, L::kHidden, net->d_d1,
-                     L::kHidden, 0.0f, s, net->d_ws, net->ws_floats, net->d_err)))
+    ep.mask = net->d_z1;
+    if ((e = L::gemm_epilogue(rows, L::kHidden, L::kHidden, net->d_d2, L::kHidden, 1, w.W2, 1, L::kHidden, net->d_d1,
+                              L::kHidden, 0.0f, s, net->d_ws, net->ws_floats, net->d_err, ep)))
         return e;
-    L::relu_back_kernel<<<blocks((long long)rows * L::kHidden), 256, 0, s>>>(net->d_d1, net->d_z1,
-                                                                           (long long)rows * L::kHidden);
     // layer 1
     if ((e = L::gemm(net->kin, L::kHidden, rows, net->d_x, 1, net->kin, net->d_d1, L::kHidden, 1, g.W1, L::kHidden,
                      0.0f, s, net->d_ws, net->ws_floats, net->d_err)))
         return e;
-    if ((e = L::column_sums(net->d_d1, rows, L::kHidden, g.b1, net->d_ws, s))) return e;
-    return cudaGetLastError();
+    // the bias gradients
+    const L::ColumnSums sums[3] = {{net->d_dy, no, g.b3}, {net->d_d2, L::kHidden, g.b2}, {net->d_d1, L::kHidden, g.b1}};
+    return L::column_sums3(sums, rows, net->d_ws, s);
 }
 
 // xorshift-based permutation of [0, n) on the host, copied to the device
