@@ -454,9 +454,18 @@ __device__ __forceinline__ void single_tile(float *smem, int base, int n, const 
     if (to2e) to2e[CurFluoID] = (!accepted && c.MultiEmitterFitEn && IsFittingValid && (CurSNR > 6.0f)) ? 1 : 0;
 }
 
+// Blocks per SM of fit_single_kernel: what the shared memory holds; AS3D at most
+// 6, whose six parameters' difference points spill at 128 registers (7x7,
+// 600,000 fits: 4.07 ms with 7, 3.88 ms with 6).
+template <int R, int KIND, bool FULL>
+constexpr int single_blocks() {
+    constexpr int b = SingleLayout<R, FULL>::BLOCKS;
+    return KIND == kAS3D && b > 6 ? 6 : b;
+}
+
 template <int R, int KIND, bool WORDS, int DIST = ArithSpec<KIND, R>::DIST, int MASK = ArithSpec<KIND, R>::MASK,
           bool FULL = MASK == kCompiler>
-__global__ void __launch_bounds__(kTPB, (SingleLayout<R, FULL>::BLOCKS)) fit_single_kernel(
+__global__ void __launch_bounds__(kTPB, (single_blocks<R, KIND, FULL>())) fit_single_kernel(
     const uint16_t *__restrict__ rois, const float *__restrict__ wle, Queue q, float *__restrict__ loc,
     uint8_t *__restrict__ to2e, CorePara c, double *__restrict__ ll, int min_n) {
     extern __shared__ __align__(16) float smem[];
@@ -970,7 +979,9 @@ struct LaneShape {
         STRIDE = (L::TOTAL + 15) / 32 * 32 + 16,
         FLOATS = 2 * L::PIXP + STRIDE * SLOTS,
         FIT = (228 * 1024) / (FLOATS * 4 + 1024),
-        BLOCKS = FIT < 4 ? FIT : 4,  // per SM: 128 registers a thread
+        // per SM: 102 registers a thread for one emitter, 128 for several
+        MOST = Emitters<KIND>::M == 1 ? 5 : 4,
+        BLOCKS = FIT < MOST ? FIT : MOST,
     };
     static_assert((int)STRIDE >= (int)L::TOTAL, "a slot holds its layout");
 };
@@ -1435,32 +1446,30 @@ cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n) {
 template <int R, int KIND, int G>
 constexpr int kLaneWave = 148 * (int)LaneShape<R, KIND, G>::BLOCKS * (int)LaneShape<R, KIND, G>::SLOTS;
 
-// A single-emitter queue by its length: as many lanes per ROI as fit the
-// whole queue at once (32, 16, at 7x7 also 8), beyond that one thread per ROI.
-// A wave costs one ROI's latency, which more lanes shorten; a second wave
-// costs it again, and past the narrowest wave the one-thread kernel, whose own
-// latency covers 18,944 ROIs, is as fast.  Fits of
-// n ROIs, us (one thread / 8 / 16 / 32 lanes): GS2D 7x7 1,000: 142 / 97 / 58 /
-// 40, 2,500: 142 / 105 / 71 / 79, 7,500: 143 / 132 / 140 / 167, 10,000: 144 /
-// 209 / 195 / 216; AS3D 9x9 1,000: 273 / 175 / 107 / 84, 5,000: 273 / 361 / 247
-// / 261, 7,500: 273 / 377 / 278 / 356.
-// The length is on the device unless a.exact: then every launch whose range
-// the queue can reach is made, and all but one return at once.
+// Longest single-emitter queue that 16 lanes per ROI fit sooner than one thread
+// per ROI: a little over one wave, whose second part costs less than a whole
+// one (the SMs are then half empty); the one-thread kernel's own latency covers
+// 18,944 ROIs.  Fits of 5,000 ROIs, us (16 lanes / one thread): GS2D 7x7 92 /
+// 142, 9x9 136 / 188, 11x11 226 / 268, AS3D 7x7 133 / 235, 9x9 181 / 273, 11x11
+// 290 / 396; of 7,500: about the same, GS2D 9x9 205 / 188; of 10,000: GS2D 7x7
+// 172 / 144, AS3D 9x9 351 / 281.
+template <int R, int KIND>
+constexpr int kLanes16Most = kLaneWave<R, KIND, 16> * (KIND == kAS3D ? 11 : (R == 9 ? 8 : 10)) / 8;
+
+// A single-emitter queue by its length: a warp per ROI while one wave of them
+// holds it (1,000 ROIs: GS2D 7x7 40 us, 16 lanes 51, one thread 142; AS3D 9x9 84,
+// 89, 273), then 16 lanes, then one thread.  The length is on the device unless
+// a.exact: then every launch whose range the queue can reach is made, and all
+// but one return at once.
 template <int R, int KIND>
 cudaError_t launch_by_length(const FitLaunch &a) {
-    int done = 0;
+    constexpr int warp_most = kLaneWave<R, KIND, 32>, half_most = kLanes16Most<R, KIND>;
     cudaError_t e = cudaSuccess;
-    auto step = [&](auto width) {
-        constexpr int G = decltype(width)::value, wave = kLaneWave<R, KIND, G>;
-        if (e != cudaSuccess || a.max_count <= done) return;
-        if (!a.exact || a.max_count <= wave) e = launch_lanes<R, KIND, G>(a, done > 0 ? done : -1, wave);
-        done = wave;
-    };
-    step(std::integral_constant<int, 32>{});
-    step(std::integral_constant<int, 16>{});
-    if (R == 7) step(std::integral_constant<int, 8>{});
-    if (e != cudaSuccess || a.max_count <= done) return e;
-    return launch_single<R, KIND>(a, a.exact ? -1 : done);
+    if (!a.exact || a.max_count <= warp_most) e = launch_lanes<R, KIND, 32>(a, -1, warp_most);
+    if (e != cudaSuccess || a.max_count <= warp_most) return e;
+    if (!a.exact || a.max_count <= half_most) e = launch_lanes<R, KIND, 16>(a, warp_most, half_most);
+    if (e != cudaSuccess || a.max_count <= half_most) return e;
+    return launch_single<R, KIND>(a, a.exact ? -1 : half_most);
 }
 
 // Longest multi-emitter queue that lane groups fit by default: the two- and

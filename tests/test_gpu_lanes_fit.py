@@ -1,6 +1,6 @@
 """Single- and multi-emitter fits by queue length: lane groups against one thread per ROI.
 
-A call without a tuning table fits its queue with 32, 16 or 8 lanes per ROI or
+A call without a tuning table fits its queue with 32 or 16 lanes per ROI or
 with one thread per ROI, by the queue's length (on the host, or on the device
 where only the device knows it).  Every choice must give the one-thread rows
 bit for bit (NaN as NaN), at and around the lengths where the choice changes,
@@ -15,8 +15,9 @@ from test_gpu_flush_fit import edge_records
 
 pytestmark = pytest.mark.gpu
 
-# one wave of 32, 16 and (7x7) 8 lanes per ROI on 148 SMs, 4 blocks of 128 threads each
-WAVES = (2368, 4736, 9472)
+# a wave of warps on 148 SMs (5 or, at 11x11, 4 blocks of 4 ROIs) and the longest queues of 16 lanes (the
+# wave of 3 to 5 blocks of 8 ROIs times 8, 10 or 11 eighths)
+WAVES = (2960, 4440, 4884, 5920, 7400, 8140)
 
 
 def device(rec):
