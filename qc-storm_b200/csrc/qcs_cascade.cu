@@ -215,7 +215,8 @@ cudaError_t launch_compaction(const S &s, int max_count, const CascadeState &st,
     return cudaGetLastError();
 }
 
-__global__ void init_counters_kernel(CascadeState st, int n, const int *__restrict__ n_dev) {
+// Counters of a call without multi-emitter fitting, the valid rows among them.
+__global__ void init_counters_kernel(CascadeState st, int n, const int *__restrict__ n_dev, int max_rows) {
     if (n_dev) n = min(max(*n_dev, 0), n);
     st.counters[kCntSingle] = n;
     st.counters[kCnt2E] = 0;
@@ -225,6 +226,7 @@ __global__ void init_counters_kernel(CascadeState st, int n, const int *__restri
     st.counters[kCntRejected] = 0;
     st.counters[kCntRows] = n;
     st.counters[kCntRefit3E] = 0;
+    st.counters[kCntValid] = n < max_rows ? n : max_rows;
 }
 
 // Likelihood-ratio selection of each record's model (run_cascade_lr); the
@@ -295,7 +297,7 @@ __global__ void finish_kernel(CascadeState st, int max_rows) {
 
 cudaError_t cascade_classify(const CascadeArgs &a, const CascadeState &st) {
     if (a.para.MultiEmitterFitEn) return launch_compaction(ClassifyStage{a.wle, a.n, a.n_dev, a.pred, st}, a.n, st, a.stream);
-    init_counters_kernel<<<1, 1, 0, a.stream>>>(st, a.n, a.n_dev);
+    init_counters_kernel<<<1, 1, 0, a.stream>>>(st, a.n, a.n_dev, a.max_rows);
     return cudaGetLastError();
 }
 
@@ -397,8 +399,10 @@ cudaError_t cascade_tail(const CascadeArgs &a, const CascadeState &st) {
             }
         }
     }
-    finish_kernel<<<1, 1, 0, a.stream>>>(st, a.max_rows);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (multi) {  // else set with the other counters
+        finish_kernel<<<1, 1, 0, a.stream>>>(st, a.max_rows);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     return launch_crlb(a.loc, st.counters + kCntValid, 0, multi ? a.max_rows : n, p.LocType, p.ReadNoise_e, p.QE,
                        p.PixelSize, a.stream);
 }

@@ -66,60 +66,64 @@ __device__ __forceinline__ float second_diff(float fp, float f0, float fn) {
     return div_dh(div_dh(__fadd_rn(__fmaf_rn(-2.0f, f0, fp), fn)));
 }
 
-// One thread per row and axis.  The reference evaluates the PSF on the full
-// grid seven times per row (model, then base, +dh, -dh for each derivative)
-// and sums d2 - model * d2log over every pixel.  The same values come from far
-// fewer evaluations, exactly: the base points equal the model (same
-// parameters, same rounding), the model is symmetric in x and y, the -dh
-// evaluation is the +dh one mirrored (x - (-h) = -((-x) - h) exactly), and
-// each derivative's terms are symmetric across the other axis.  So a thread
-// takes the half grid line by line: the line's model values (half a line) and
-// +dh values, then its terms, kept in shared memory ([term][thread]); the
-// Fisher sum adds every pixel's term in the reference's pixel order.  The y
-// terms are the x terms with the axes exchanged (the reference's two sites
-// contract mirror-image products); warp 0 of a block takes 32 rows' x terms,
-// warp 1 their y terms.  Nothing is shared between threads, so the terms are
-// the only shared memory: 14 warps an SM at 15 x 15.  100,000 rows at 9 x 9: 66
-// -> 43 us, 60,013 at 15 x 15: 221 -> 93 us, 300 rows: 24 -> 14 us (before: a
-// model table per row, 9 warps an SM at 15 x 15, and four divisions per term).
-// Bound by the instructions of logf, 2 (Q + G) a line.
+// Rows per block.
+__host__ __device__ constexpr int crlb_rows(int G) { return G == 9 ? 32 : 16; }
+
+// One thread per row, axis and line of the half grid.  The reference
+// evaluates the PSF on the full grid seven times per row (model, then base,
+// +dh, -dh for each derivative) and sums d2 - model * d2log over every pixel.
+// The same values come from far fewer evaluations, exactly: the base points
+// equal the model (same parameters, same rounding), the model is symmetric in
+// x and y, the -dh evaluation is the +dh one mirrored (x - (-h) = -((-x) - h)
+// exactly), and each derivative's terms are symmetric across the other axis.
+// So a thread takes one line: its model values (half a line) and +dh values,
+// then its terms, kept in shared memory ([term][row and axis]); after a
+// barrier one thread per row and axis adds every pixel's term in the
+// reference's pixel order.  The y terms are the x terms with the axes
+// exchanged (the reference's two sites contract mirror-image products); a
+// warp holds one axis of 32 rows (15 x 15: two axes of 16).  100,000 rows at 9
+// x 9: 41 us, 60,013 at 15 x 15: 67, 300 at 9 x 9: 6 (a thread per row and
+// axis walking the lines: 43, 92, 13; two lanes per row sharing a model table,
+// with divisions: 66, 221, 24).  Bound by the instructions of logf, Q +
+// G a line.
 template <int G>
-__global__ void __launch_bounds__(64) crlb_kernel(float *__restrict__ loc, const int *__restrict__ n_dev, int n,
-                                                  const int *__restrict__ ids, const uint8_t *__restrict__ skip,
-                                                  float ReadNoise_e, float QE, float PixelSize) {
-    enum { H = G / 2, Q = H + 1 };
+__global__ void __launch_bounds__((G / 2 + 1) * (G == 9 ? 64 : 32)) crlb_kernel(
+    float *__restrict__ loc, const int *__restrict__ n_dev, int n, const int *__restrict__ ids,
+    const uint8_t *__restrict__ skip, float ReadNoise_e, float QE, float PixelSize) {
+    enum { H = G / 2, Q = H + 1, ROWS = crlb_rows(G), LANES = 2 * ROWS };
     using S = CrlbSites<G>;
     // the x-derivative thread uses fma(dx^2, six, dy^2 siy), the y-derivative thread
     // fma(dy^2, siy, dx^2 six): one expression with its operands exchanged
     static_assert(S::SHIFT_X == kFuseFirst && S::SHIFT_Y == kFuseSecond, "mirrored derivative sites");
-    __shared__ float sT[Q * G][64];
-    const int role = threadIdx.x >> 5;  // 0: x, 1: y
+    __shared__ float sT[Q * G][LANES];
+    const int slot = threadIdx.x % LANES, l = threadIdx.x / LANES;
+    const int role = slot / ROWS;  // 0: x, 1: y
     const int rows = n_dev ? *n_dev : n;
-    const int k_slot = blockIdx.x * 32 + (threadIdx.x & 31);
-    if (k_slot >= rows) return;
-    const int gid = ids ? ids[k_slot] : k_slot;
-    if (skip && skip[gid]) return;
+    const int k_slot = blockIdx.x * ROWS + slot % ROWS;
+    if (blockIdx.x * ROWS >= rows) return;  // the whole block
+    const int gid = k_slot < rows ? (ids ? ids[k_slot] : k_slot) : 0;
+    const bool have = k_slot < rows && !(skip && skip[gid]);
     float *r = loc + (size_t)gid * 12;
-    const float TotalPhoton_e = __fmul_rn(r[QCS_POS_TPHO], QE);
-    float Background_e = __fmul_rn(r[QCS_POS_BAKG], QE);
-    const float sx = r[QCS_POS_SIGX], sy = r[QCS_POS_SIGY];
-    float std_dev = 100.0f;
-    if ((TotalPhoton_e > 1) && (Background_e > 1) && (sx > 0.1) && (sy > 0.1) && (sx < 10) && (sy < 10)) {
-        // read noise counted into the background (LocPrecCalc_GaussianCRLB.h:89-92)
-        Background_e = __fdiv_rn(__fmaf_rn(ReadNoise_e, ReadNoise_e, __fmul_rn(Background_e, QE)), QE);
-        const float pi = 3.141592654f;
-        PsfPara p;
-        p.peak = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(__fmul_rn(__fmul_rn(2.0f, pi), sx), sy)), TotalPhoton_e);
-        p.six = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, sx), sx));
-        p.siy = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, sy), sy));
-        p.bkg = Background_e;
-        const float h = 0.02f;
-        const float su = role ? p.siy : p.six, sv = role ? p.six : p.siy;
-        float *T = &sT[0][threadIdx.x];
-        // x thread: the +dh row at |CurY| = l, every column k; y thread: the
-        // +dh column at |CurX| = l, every row k
-#pragma unroll 1
-        for (int l = 0; l < Q; ++l) {
+    float *T = &sT[0][slot];
+    bool valid = false;
+    if (have) {
+        const float TotalPhoton_e = __fmul_rn(r[QCS_POS_TPHO], QE);
+        float Background_e = __fmul_rn(r[QCS_POS_BAKG], QE);
+        const float sx = r[QCS_POS_SIGX], sy = r[QCS_POS_SIGY];
+        valid = (TotalPhoton_e > 1) && (Background_e > 1) && (sx > 0.1) && (sy > 0.1) && (sx < 10) && (sy < 10);
+        if (valid) {
+            // read noise counted into the background (LocPrecCalc_GaussianCRLB.h:89-92)
+            Background_e = __fdiv_rn(__fmaf_rn(ReadNoise_e, ReadNoise_e, __fmul_rn(Background_e, QE)), QE);
+            const float pi = 3.141592654f;
+            PsfPara p;
+            p.peak = __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(__fmul_rn(__fmul_rn(2.0f, pi), sx), sy)), TotalPhoton_e);
+            p.six = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, sx), sx));
+            p.siy = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, sy), sy));
+            p.bkg = Background_e;
+            const float h = 0.02f;
+            const float su = role ? p.siy : p.six, sv = role ? p.six : p.siy;
+            // x thread: the +dh row at |CurY| = l, every column k; y thread: the
+            // +dh column at |CurX| = l, every row k
             const float fl = (float)l;
             const float ll = __fmul_rn(__fmul_rn(fl, fl), sv);
             float m[Q], lm[Q], tp[G], lp[G];
@@ -140,9 +144,14 @@ __global__ void __launch_bounds__(64) crlb_kernel(float *__restrict__ loc, const
                 const int o = k < H ? H - k : k - H;  // |k - H|
                 const float d2 = second_diff(tp[k], m[o], tp[G - 1 - k]);
                 const float dl = second_diff(lp[k], lm[o], lp[G - 1 - k]);
-                T[(l * G + k) * 64] = __fmaf_rn(-m[o], dl, d2);
+                T[(l * G + k) * LANES] = __fmaf_rn(-m[o], dl, d2);
             }
         }
+    }
+    __syncthreads();  // the lines' terms; the row is read by all before its CRLB is written
+    if (l != 0 || !have) return;
+    float std_dev = 100.0f;
+    if (valid) {
         // Fisher information, pixel order (LocPrecCalc_GaussianCRLB.h:226-243)
         float F = 0;
 #pragma unroll 1
@@ -151,7 +160,7 @@ __global__ void __launch_bounds__(64) crlb_kernel(float *__restrict__ loc, const
 #pragma unroll
             for (int x = 0; x < G; ++x) {
                 const int bx = x < H ? H - x : x - H;
-                F = __fadd_rn(F, T[(role ? bx * G + y : ay * G + x) * 64]);
+                F = __fadd_rn(F, T[(role ? bx * G + y : ay * G + x) * LANES]);
             }
         }
         if (F == 0.0f) F = 1;
@@ -165,11 +174,12 @@ __global__ void __launch_bounds__(64) crlb_kernel(float *__restrict__ loc, const
 cudaError_t launch_crlb(float *loc, const int *n_dev, int n, int max_rows, int loc_type, float ReadNoise_e, float QE,
                         float PixelSize, cudaStream_t s, const int *ids, const uint8_t *skip) {
     if (max_rows <= 0) return cudaSuccess;
-    const int blocks = (max_rows + 31) / 32;  // 32 rows per 64-thread block
+    const int rows = loc_type != QCS_LOCTYPE_AS3D ? crlb_rows(9) : crlb_rows(15);
+    const int blocks = (max_rows + rows - 1) / rows;
     if (loc_type != QCS_LOCTYPE_AS3D)
-        crlb_kernel<9><<<blocks, 64, 0, s>>>(loc, n_dev, n, ids, skip, ReadNoise_e, QE, PixelSize);
+        crlb_kernel<9><<<blocks, 2 * rows * 5, 0, s>>>(loc, n_dev, n, ids, skip, ReadNoise_e, QE, PixelSize);
     else
-        crlb_kernel<15><<<blocks, 64, 0, s>>>(loc, n_dev, n, ids, skip, ReadNoise_e, QE, PixelSize);
+        crlb_kernel<15><<<blocks, 2 * rows * 8, 0, s>>>(loc, n_dev, n, ids, skip, ReadNoise_e, QE, PixelSize);
     return cudaGetLastError();
 }
 
