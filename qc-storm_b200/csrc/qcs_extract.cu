@@ -18,8 +18,8 @@
 //                      image itself, as the reference does (its sharpen step
 //                      writes into a scratch image nothing reads,
 //                      _ImageFiltering.cu:96-104, 675)
-//   scan_kernel        exclusive scan of detections per 4096-pixel chunk
-//   compact_kernel     ordered compaction of the detections into sorted keys
+//   compact_kernel     ordered compaction of the detections into sorted keys,
+//                      by their counts per 4096-pixel chunk
 //   cut_kernel         single/multi classification, ROI cut and header, one
 //                      warp per record (_ROIExtraction.cu:181-302)
 //   WLE pre-pass       launch_wle_presorted over the batch's records and keys
@@ -53,8 +53,8 @@ constexpr int kBgPairs = 128;        // column pairs per block (two columns per 
 constexpr int kBgThreads = 2 * kBgPairs; // two row halves
 constexpr int kBgCols = 2 * kBgPairs, kBgRows = 32, kBgWords = kBgCols / 2 + 4;
 constexpr int kDetTX = 128, kDetTY = 32, kDetThreads = 256;
-constexpr int kVarBlocks = 64, kVarThreads = 256;
-constexpr int kScanThreads = 1024;
+constexpr int kVarBlocks = 256, kVarThreads = 256;
+constexpr int kSuper = 64;           // chunks per count of the second level
 constexpr int kCutThreads = 256;     // one warp per record
 
 // Device state words of an extraction context.
@@ -68,11 +68,12 @@ struct Taps {
 };
 
 struct DetectPara {
-    int W, H0, Hb, half, low_th;
+    int W, H0, Hb, half, low_th, nchunks;
 };
 
 struct EmitPara {
     int W, H0, R, multi, start_frame, npx;
+    int nchunks, batch_cap, capacity;
 };
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v, lo), hi); }
@@ -87,6 +88,13 @@ __device__ __forceinline__ float u2f(uint32_t u) { return __fsub_rn(__uint_as_fl
 __device__ __forceinline__ uint32_t trunc_u16(float v) {
     return __float_as_uint(__fadd_rz(fminf(v, 65535.0f), 8388608.0f)) - 0x4B000000u;
 }
+// Candidates are counted per chunk, counts[0 .. nchunks), and per kSuper
+// chunks, counts[nchunks ..).
+__device__ __forceinline__ void count_candidate(int *counts, const DetectPara &dp, int chunk) {
+    atomicAdd(&counts[chunk], 1);
+    atomicAdd(&counts[dp.nchunks + chunk / kSuper], 1);
+}
+
 // trunc_u16 as a float (the value a uint16 intermediate image would hold)
 __device__ __forceinline__ float trunc_u16f(float v) { return __fsub_rn(__fadd_rz(fminf(v, 65535.0f), 8388608.0f), 8388608.0f); }
 
@@ -130,7 +138,11 @@ __device__ __forceinline__ void load_tile_clamped_f(float *dst, const uint16_t *
 // registers.  All sums are integers, so the float steps that follow (ring
 // sum / 8, three-neighbour sum, / 3) round exactly as the reference's.
 __global__ void __launch_bounds__(kBgThreads) background_kernel(const uint16_t *__restrict__ raw,
-                                                                uint16_t *__restrict__ bg, int W, int H) {
+                                                                uint16_t *__restrict__ bg, int W, int H,
+                                                                int *__restrict__ counts, int ncounts) {
+    // the detection counts of this batch
+    const int c0 = (blockIdx.y * gridDim.x + blockIdx.x) * kBgThreads + threadIdx.x;
+    if (c0 < ncounts) counts[c0] = 0;
     // t[r][k]: pixels (x0 - 4 + 2k, x0 - 3 + 2k) of row y0 - 4 + r (clamped), low half first
     __shared__ uint32_t t[kBgRows + 8][kBgWords];
     const int x0 = blockIdx.x * kBgCols, y0 = blockIdx.y * kBgRows;
@@ -246,7 +258,7 @@ __global__ void __launch_bounds__(kBgThreads) background_kernel(const uint16_t *
 // var[0] = mean square - mean^2 (at least 100) and clears acc[0..2].
 __global__ void __launch_bounds__(kVarThreads) variance_kernel(const uint16_t *__restrict__ bg, int W, int cx, int cy,
                                                                int S, unsigned long long *__restrict__ acc,
-                                                               float *__restrict__ var) {
+                                                               float *__restrict__ var, int *__restrict__ state) {
     unsigned long long s1 = 0, s2 = 0;
     const int total = S * S;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
@@ -287,6 +299,7 @@ __global__ void __launch_bounds__(kVarThreads) variance_kernel(const uint16_t *_
             float v = __fsub_rn(mx2, __fmul_rn(mx, mx));
             if (v < 100.0f) v = 100.0f;
             var[0] = v;
+            state[kStBase] = state[kStAccum];  // where this batch's records start
             acc[0] = 0;
             acc[1] = 0;
             acc[2] = 0;
@@ -364,7 +377,7 @@ __global__ void __launch_bounds__(kDetThreads) detect_kernel(const uint16_t *__r
                         flag = kMarked;
                         if (jo == 4) {
                             flag |= kCandidate;
-                            atomicAdd(&chunk_count[(y * W + x) / kChunk], 1);
+                            count_candidate(chunk_count, dp, (y * W + x) / kChunk);
                         }
                     }
                 }
@@ -420,7 +433,7 @@ __global__ void __launch_bounds__(kWideX * kWideY) detect_wide_kernel(const uint
                 uint32_t flag = kMarked;
                 if (jo == 4) {
                     flag |= kCandidate;
-                    atomicAdd(&chunk_count[(y * W + x) / kChunk], 1);
+                    count_candidate(chunk_count, dp, (y * W + x) / kChunk);
                 }
                 flags[j / 4] |= flag << (8 * (j & 3));
             }
@@ -458,39 +471,15 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *total) {
     return before + x - v;
 }
 
-// Chunk counts -> exclusive chunk offsets (in place); decides how many of the
-// batch's detections are kept and where they start in the record buffer.
-__global__ void __launch_bounds__(kScanThreads) scan_kernel(int *__restrict__ chunk, int nchunks,
-                                                            int *__restrict__ state, int batch_cap, int capacity) {
-    const int per = (nchunks + kScanThreads - 1) / kScanThreads;
-    const int b = threadIdx.x * per, e = min(b + per, nchunks);
-    int sum = 0;
-    for (int i = b; i < e; ++i) sum += chunk[i];
-    int total = 0;
-    int run = block_exclusive_scan<kScanThreads>(sum, &total);
-    for (int i = b; i < e; ++i) {
-        const int c = chunk[i];
-        chunk[i] = run;
-        run += c;
-    }
-    if (threadIdx.x == 0) {
-        const int acc = state[kStAccum];
-        int n = min(total, batch_cap);
-        n = min(n, capacity - acc);
-        if (n < 0) n = 0;
-        state[kStBase] = acc;
-        state[kStBatchN] = n;
-        state[kStAccum] = acc + n;
-        state[kStDropped] += total - n;
-        state[kStDetected] = total;
-    }
-}
-
 // Ordered compaction: the k-th detection of the batch in pixel order gets
 // record base + k; its key frame << 32 | y << 16 | x goes to keys[base + k].
+// Each block adds the counts before its chunk, at most kSuper of them and one
+// per kSuper chunks, so that no launch is needed to scan them (one block's scan
+// of 1,024 counts took 3.7 us a frame); they also say how many of the batch's
+// detections are kept, which block 0 writes down.
 __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const uint8_t *__restrict__ pos,
-                                                                  const int *__restrict__ chunk_off,
-                                                                  const int *__restrict__ state,
+                                                                  const int *__restrict__ counts,
+                                                                  int *__restrict__ state,
                                                                   unsigned long long *__restrict__ keys, EmitPara ep) {
     const int p0 = blockIdx.x * kChunk + threadIdx.x * 16;
     uint8_t f[16];
@@ -501,13 +490,39 @@ __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const uint8_t 
 #pragma unroll
         for (int j = 0; j < 16; ++j) f[j] = (p0 + j < ep.npx) ? pos[p0 + j] : 0;
     }
+    const int base = state[kStBase];
+    const int super = blockIdx.x / kSuper, supers = (ep.nchunks + kSuper - 1) / kSuper;
+    int before = 0, all = 0;
+    for (int i = threadIdx.x; i < supers; i += kCompactThreads) {
+        const int v = counts[ep.nchunks + i];
+        all += v;
+        if (i < super) before += v;
+    }
+    const int c = super * kSuper + threadIdx.x;
+    if (threadIdx.x < kSuper && c < blockIdx.x) before += counts[c];
     int cnt = 0;
 #pragma unroll
     for (int j = 0; j < 16; ++j) cnt += (f[j] & kCandidate) ? 1 : 0;
+    __shared__ int sum[2];
+    if (threadIdx.x < 2) sum[threadIdx.x] = 0;
     int total;
-    int k = chunk_off[blockIdx.x] + block_exclusive_scan<kCompactThreads>(cnt, &total);
+    int k = block_exclusive_scan<kCompactThreads>(cnt, &total);  // synchronises the block
+    before = __reduce_add_sync(0xffffffffu, before);
+    all = __reduce_add_sync(0xffffffffu, all);
+    if ((threadIdx.x & 31) == 0) {
+        if (before) atomicAdd(&sum[0], before);
+        if (all) atomicAdd(&sum[1], all);
+    }
+    __syncthreads();
+    k += sum[0];
+    const int n = max(min(min(sum[1], ep.batch_cap), ep.capacity - base), 0);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        state[kStBatchN] = n;
+        state[kStAccum] = base + n;
+        state[kStDropped] += sum[1] - n;
+        state[kStDetected] = sum[1];
+    }
     if (cnt == 0) return;
-    const int base = state[kStBase], n = state[kStBatchN];
     for (int j = 0; j < 16; ++j) {
         if (!(f[j] & kCandidate)) continue;
         if (k < n) {
@@ -716,7 +731,7 @@ int qcs_extract_init_ex(const qcs_loc_para *p, int max_batched_num, int capacity
     cudaError_t e = cudaMalloc((void **)&c->d_raw, px * sizeof(uint16_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_bg, px * sizeof(uint16_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_pos, px_pad);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_chunk, (size_t)c->nchunks_max * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_chunk, (c->nchunks_max + (size_t)(c->nchunks_max + qcs::kSuper - 1) / qcs::kSuper) * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_state, qcs::kStNum * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_var, 4 * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_var_acc, 4 * sizeof(unsigned long long));
@@ -799,9 +814,10 @@ int qcs_extract_molecules(qcs_extract_data *c, const uint16_t *img, int image_so
     }
     const int Hb = H0 * batched_num;
     const int nchunks = (int)((npx + qcs::kChunk - 1) / qcs::kChunk);
-    QCS_CUDA(cudaMemsetAsync(c->d_chunk, 0, (size_t)nchunks * sizeof(int), s), "clear chunk counts");
+    const int nsupers = (nchunks + qcs::kSuper - 1) / qcs::kSuper;
     dim3 gbg((W + qcs::kBgCols - 1) / qcs::kBgCols, (Hb + qcs::kBgRows - 1) / qcs::kBgRows);
-    qcs::background_kernel<<<gbg, qcs::kBgThreads, 0, s>>>(raw, c->d_bg, W, Hb);
+    // (W/256 x Hb/32 blocks of 256 threads: more threads than counts)
+    qcs::background_kernel<<<gbg, qcs::kBgThreads, 0, s>>>(raw, c->d_bg, W, Hb, c->d_chunk, nchunks + nsupers);
     // central patch of the stacked batch (LDROIExtraction.cu:142-157)
     int sw = W / 2 - 5, sh = Hb / 2 - 5;
     sw = sw > 256 ? 256 : sw;
@@ -809,12 +825,13 @@ int qcs_extract_molecules(qcs_extract_data *c, const uint16_t *img, int image_so
     sw = sw < 1 ? 1 : sw;
     sh = sh < 1 ? 1 : sh;
     const int S = sw < sh ? sw : sh;
-    int vblocks = (S * S + qcs::kVarThreads * 4 - 1) / (qcs::kVarThreads * 4);
+    int vblocks = (S * S + qcs::kVarThreads - 1) / qcs::kVarThreads;
     vblocks = vblocks < 1 ? 1 : (vblocks > qcs::kVarBlocks ? qcs::kVarBlocks : vblocks);
-    qcs::variance_kernel<<<vblocks, qcs::kVarThreads, 0, s>>>(c->d_bg, W, W / 2, Hb / 2, S, c->d_var_acc, c->d_var);
+    qcs::variance_kernel<<<vblocks, qcs::kVarThreads, 0, s>>>(c->d_bg, W, W / 2, Hb / 2, S, c->d_var_acc, c->d_var, c->d_state);
     const int multi = p->MultiEmitterFitEn;
     qcs::DetectPara dp{W, H0, Hb, c->R / 2,
-                       (p->LocType == QCS_LOCTYPE_AS3D || (multi == 0 && p->LocType == QCS_LOCTYPE_GS2D)) ? 1 : 0};
+                       (p->LocType == QCS_LOCTYPE_AS3D || (multi == 0 && p->LocType == QCS_LOCTYPE_GS2D)) ? 1 : 0,
+                       nchunks};
     dim3 gdet((W + qcs::kDetTX - 1) / qcs::kDetTX, (Hb + qcs::kDetTY - 1) / qcs::kDetTY);
     if (p->LocType == QCS_LOCTYPE_GS2D && multi > 0 && W % 8 == 0)
         qcs::detect_wide_kernel<<<dim3((Hb + qcs::kWideY - 1) / qcs::kWideY, (W / 8 + qcs::kWideX - 1) / qcs::kWideX),
@@ -823,8 +840,7 @@ int qcs_extract_molecules(qcs_extract_data *c, const uint16_t *img, int image_so
         qcs::detect_kernel<false><<<gdet, qcs::kDetThreads, 0, s>>>(c->d_bg, c->d_pos, c->d_chunk, c->d_var, c->taps, dp);
     else
         qcs::detect_kernel<true><<<gdet, qcs::kDetThreads, 0, s>>>(c->d_bg, c->d_pos, c->d_chunk, c->d_var, c->taps, dp);
-    qcs::scan_kernel<<<1, qcs::kScanThreads, 0, s>>>(c->d_chunk, nchunks, c->d_state, QCS_MAX_POINT_NUM, c->capacity);
-    qcs::EmitPara ep{W, H0, c->R, multi, start_frame, (int)npx};
+    qcs::EmitPara ep{W, H0, c->R, multi, start_frame, (int)npx, nchunks, QCS_MAX_POINT_NUM, c->capacity};
     qcs::compact_kernel<<<nchunks, qcs::kCompactThreads, 0, s>>>(c->d_pos, c->d_chunk, c->d_state, c->d_keys, ep);
     const int batch_max = QCS_MAX_POINT_NUM < c->capacity ? QCS_MAX_POINT_NUM : c->capacity;
     int cut_blocks = (batch_max + qcs::kCutThreads / 32 - 1) / (qcs::kCutThreads / 32);
