@@ -454,6 +454,25 @@ __device__ __forceinline__ void single_tile(float *smem, int base, int n, const 
     if (to2e) to2e[CurFluoID] = (!accepted && c.MultiEmitterFitEn && IsFittingValid && (CurSNR > 6.0f)) ? 1 : 0;
 }
 
+// ROIs of one warp on every scheduler: fit_single_kernel takes the same time
+// for any number of them up to here, and half as long again for one more.
+constexpr int kThreadWave = 148 * 4 * 32;
+
+// The last entries of a queue that lane groups fit beside fit_single_kernel:
+// what it holds past whole waves, where that is at most `most` (0: none).  One
+// wave of warps takes 2,960, and costs less than the schedulers' next warp:
+// records end to end, us (without / with): 11x11 18,945: 457 / 313, 20,000: 459
+// / 328, 40,848: 698 / 654; AS3D 9x9 38,944: 735 / 527, 116,624: 1,589 / 1,504;
+// GS2D 7x7 20,000: 233 / 191, 40,848: 321 / 274.  4,440 of them lose up to a
+// tenth past the first wave, and at GS2D 7x7, whose warps cost least, any number
+// past four (154,512: 844 / 872).
+template <int R, int KIND>
+__device__ __host__ __forceinline__ int queue_rest(int n, int most) {
+    if (n <= kThreadWave || (R == 7 && KIND == kGS2D && n >= 5 * kThreadWave)) return 0;
+    const int r = n % kThreadWave;
+    return r <= most ? r : 0;
+}
+
 // Blocks per SM of fit_single_kernel: what the shared memory holds; AS3D at most
 // 6, whose six parameters' difference points spill at 128 registers (7x7,
 // 600,000 fits: 4.07 ms with 7, 3.88 ms with 6).
@@ -467,11 +486,14 @@ template <int R, int KIND, bool WORDS, int DIST = ArithSpec<KIND, R>::DIST, int 
           bool FULL = MASK == kCompiler>
 __global__ void __launch_bounds__(kTPB, (single_blocks<R, KIND, FULL>())) fit_single_kernel(
     const uint16_t *__restrict__ rois, const float *__restrict__ wle, Queue q, float *__restrict__ loc,
-    uint8_t *__restrict__ to2e, CorePara c, double *__restrict__ ll, int min_n) {
+    uint8_t *__restrict__ to2e, CorePara c, double *__restrict__ ll, int min_n, int rest_most) {
     extern __shared__ __align__(16) float smem[];
+    // once every block has started, the lane groups that fit the rest may
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int n = queue_len(q);
-    if (n <= min_n) return;  // a queue this short is the lane-group kernel's
-    single_tile<R, KIND, WORDS, DIST, MASK, FULL, kTPB>(smem, blockIdx.x * kTPB, n, rois, wle, q, loc, to2e, c, ll);
+    if (n > min_n)  // a queue this short is the lane-group kernel's
+        single_tile<R, KIND, WORDS, DIST, MASK, FULL, kTPB>(smem, blockIdx.x * kTPB, n - queue_rest<R, KIND>(n, rest_most), rois,
+                                                            wle, q, loc, to2e, c, ll);
 }
 
 // ------------------------------------------------ mixed-size single fits ---
@@ -990,7 +1012,7 @@ template <int R, int KIND, int G, int DIST = ArithSpec<KIND, R>::DIST, int MASK 
           int SUM2 = ArithSpec<KIND, R>::SUM2>
 __global__ void __launch_bounds__(kGroupTPB, (LaneShape<R, KIND, G>::BLOCKS)) fit_lanes_kernel(
     const uint16_t *__restrict__ rois, const float *__restrict__ wle, Queue q, float *__restrict__ loc,
-    uint8_t *__restrict__ to2e, MultiOut mo, CorePara c, double *__restrict__ ll, int min_n, int max_n) {
+    uint8_t *__restrict__ to2e, MultiOut mo, CorePara c, double *__restrict__ ll, int min_n, int max_n, int rest_most) {
     typedef LaneLayout<R, KIND> L;
     typedef LaneShape<R, KIND, G> S;
     constexpr bool MULTI = Emitters<KIND>::M > 1;
@@ -998,7 +1020,15 @@ __global__ void __launch_bounds__(kGroupTPB, (LaneShape<R, KIND, G>::BLOCKS)) fi
     static_assert(DIST != kCompiler && (!MULTI || SUM2 == kFuseFirst), "roundings fixed in the source");
     extern __shared__ __align__(16) float smem[];
     const int n = queue_len(q);
-    if (n <= min_n || (max_n >= 0 && n > max_n)) return;
+    const bool whole = n > min_n && (max_n < 0 || n <= max_n);
+    const int rest = whole ? n : queue_rest<R, KIND>(n, rest_most);
+    // beside the one-thread kernel of the queue's other entries: ends after it
+    // does, so that what follows on the stream finds its rows
+    const bool last = rest_most > 0 && blockIdx.x == 0;
+    if (rest == 0) {
+        if (last) asm volatile("griddepcontrol.wait;" ::: "memory");
+        return;
+    }
     float *pos = smem;
     for (int k = threadIdx.x; k < L::PIXP; k += kGroupTPB) {
         pos[k] = k % R + 0.5f;
@@ -1008,7 +1038,7 @@ __global__ void __launch_bounds__(kGroupTPB, (LaneShape<R, KIND, G>::BLOCKS)) fi
     const int lane = threadIdx.x % G;
     const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G % 32)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
     float *s = smem + 2 * L::PIXP + threadIdx.x / G * S::STRIDE;
-    for (int slot = blockIdx.x * S::SLOTS + threadIdx.x / G; slot < n; slot += gridDim.x * S::SLOTS) {
+    for (int slot = n - rest + blockIdx.x * S::SLOTS + threadIdx.x / G; slot < n; slot += gridDim.x * S::SLOTS) {
         const int CurFluoID = queue_at(q, slot);
         const uint16_t *rec = rois + (size_t)CurFluoID * WHOLE;
         for (int k = lane; k < L::PIXP; k += G) {
@@ -1074,6 +1104,7 @@ __global__ void __launch_bounds__(kGroupTPB, (LaneShape<R, KIND, G>::BLOCKS)) fi
         }
         __syncwarp(mask);  // the slot's shared memory is free again
     }
+    if (last) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Shared memory per slot of fit_learned_3e_warp_kernel: pixels, and one
@@ -1412,34 +1443,49 @@ cudaError_t launch_learned_3e(const FitLaunch &a, const float *start, float dev_
     return cudaGetLastError();
 }
 
+// rest_most > 0: all but the queue's rest (queue_rest).
 template <int R, int KIND>
-cudaError_t launch_single(const FitLaunch &a, int min_n = -1) {
+cudaError_t launch_single(const FitLaunch &a, int min_n = -1, int rest_most = 0) {
     const size_t smem = SingleLayout<R, ArithSpec<KIND, R>::MASK == kCompiler>::BYTES;
     // two pixels per load when every record starts on a 4-byte boundary
     auto k = (reinterpret_cast<uintptr_t>(a.rois) & 3) == 0 ? fit_single_kernel<R, KIND, true>
                                                              : fit_single_kernel<R, KIND, false>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int grid = (a.max_count + kTPB - 1) / kTPB;
+    // no empty blocks where the length is known: the blocks of a grid that is a
+    // multiple of the SMs are spread evenly, those of a larger one are not
+    const int grid = (a.max_count - (a.exact ? queue_rest<R, KIND>(a.max_count, rest_most) : 0) + kTPB - 1) / kTPB;
     if (grid == 0) return cudaSuccess;
-    k<<<grid, kTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.to2e, a.para, a.ll, min_n);
+    k<<<grid, kTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.to2e, a.para, a.ll, min_n, rest_most);
     return cudaGetLastError();
 }
 
-// Queues of min_n < n <= max_n (< 0: any length) entries with G lanes per ROI.
+// Queues of min_n < n <= max_n (< 0: any length) entries with G lanes per ROI,
+// and the rest of longer ones (queue_rest; rest_most > 0: launched right after
+// the one-thread kernel, and runs beside it).
 template <int R, int KIND, int G>
-cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n) {
+cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n, int rest_most = 0) {
     typedef LaneShape<R, KIND, G> S;
     const size_t smem = S::FLOATS * sizeof(float);
     auto k = fit_lanes_kernel<R, KIND, G>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const long long most = max_n >= 0 && max_n < a.max_count ? max_n : a.max_count;
+    const int longest = max_n >= 0 && max_n < rest_most ? rest_most : max_n;
+    const long long most = longest >= 0 && longest < a.max_count ? longest : a.max_count;
     const long long need = (most + S::SLOTS - 1) / S::SLOTS;
     const int grid = (int)(need < 148 * S::BLOCKS ? need : 148 * S::BLOCKS);
     if (grid <= 0) return cudaSuccess;
-    k<<<grid, kGroupTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.to2e, a.mo, a.para, a.ll, min_n, max_n);
-    return cudaGetLastError();
+    cudaLaunchAttribute beside{};
+    beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    beside.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kGroupTPB);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = a.stream;
+    cfg.attrs = &beside;
+    cfg.numAttrs = rest_most > 0 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k, a.rois, a.wle, a.q, a.loc, a.to2e, a.mo, a.para, a.ll, min_n, max_n, rest_most);
 }
 
 // The ROIs that G lanes each fit at once on the whole GPU.
@@ -1458,18 +1504,27 @@ constexpr int kLanes16Most = kLaneWave<R, KIND, 16> * (KIND == kAS3D ? 11 : (R =
 
 // A single-emitter queue by its length: a warp per ROI while one wave of them
 // holds it (1,000 ROIs: GS2D 7x7 40 us, 16 lanes 51, one thread 142; AS3D 9x9 84,
-// 89, 273), then 16 lanes, then one thread.  The length is on the device unless
-// a.exact: then every launch whose range the queue can reach is made, and all
-// but one return at once.
+// 89, 273), then 16 lanes, then one thread, beside a warp per ROI for a short
+// rest past whole waves (queue_rest).  The length is on the device unless
+// a.exact: then every launch whose range the queue can reach is made, and those
+// that it does not reach return at once.
 template <int R, int KIND>
 cudaError_t launch_by_length(const FitLaunch &a) {
-    constexpr int warp_most = kLaneWave<R, KIND, 32>, half_most = kLanes16Most<R, KIND>;
+    constexpr int warp_most = kLaneWave<R, KIND, 32>, half_most = kLanes16Most<R, KIND>, rest_most = kLaneWave<R, KIND, 32>;
+    const bool may_be_long = a.max_count > half_most;
     cudaError_t e = cudaSuccess;
-    if (!a.exact || a.max_count <= warp_most) e = launch_lanes<R, KIND, 32>(a, -1, warp_most);
-    if (e != cudaSuccess || a.max_count <= warp_most) return e;
-    if (!a.exact || a.max_count <= half_most) e = launch_lanes<R, KIND, 16>(a, warp_most, half_most);
-    if (e != cudaSuccess || a.max_count <= half_most) return e;
-    return launch_single<R, KIND>(a, a.exact ? -1 : half_most);
+    if (a.max_count > warp_most && (!a.exact || !may_be_long)) e = launch_lanes<R, KIND, 16>(a, warp_most, half_most);
+    if (e != cudaSuccess) return e;
+    if (a.exact && may_be_long) {
+        const int rest = queue_rest<R, KIND>(a.max_count, rest_most);
+        e = launch_single<R, KIND>(a, -1, rest);
+        if (e == cudaSuccess && rest > 0) e = launch_lanes<R, KIND, 32>(a, -1, 0, rest);
+        return e;
+    }
+    const int rest = a.max_count > kThreadWave ? rest_most : 0;
+    if (may_be_long) e = launch_single<R, KIND>(a, half_most, rest);
+    if (e == cudaSuccess && (!a.exact || a.max_count <= warp_most)) e = launch_lanes<R, KIND, 32>(a, -1, warp_most, rest);
+    return e;
 }
 
 // Longest multi-emitter queue that lane groups fit by default: the two- and

@@ -28,8 +28,20 @@ def device(rec):
 @pytest.mark.parametrize("loc_type,R", [(0, 7), (1, 7), (0, 9), (1, 9), (0, 11), (1, 11), (0, 13)])
 @pytest.mark.parametrize("n", [1, 3, 5] + [w + d for w in WAVES for d in (0, 1)])
 def test_single_by_length(cuda_ok, loc_type, R, n):
-    import torch
     rec, para = edge_records(max(n, 2051), R, loc_type)
+    check_single(rec, para, n)
+
+
+# whole waves of one warp per scheduler (18,944 ROIs), and a rest beside them
+@pytest.mark.parametrize("loc_type,R", [(0, 7), (1, 7), (0, 9), (1, 9), (0, 11), (1, 11), (0, 13)])
+@pytest.mark.parametrize("n", [18944, 18945, 18946, 21312, 21313, 21904, 21906, 40000, 94721])
+def test_single_rest(cuda_ok, loc_type, R, n):
+    rec, para = edge_records(2051, R, loc_type)
+    check_single(np.resize(rec, (n, rec.shape[1])), para, n)
+
+
+def check_single(rec, para, n):
+    import torch
     d = device(rec[:n])
     ctx = qlib.LocContext(para, n)
     rows = []
