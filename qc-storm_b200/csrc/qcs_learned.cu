@@ -16,6 +16,7 @@
 // Training and inference GEMMs run on the tensor cores (tcgen05) in BF16 with
 // FP32 accumulation; master weights and Adam moments are FP32.
 // Labels are the converged plain MLEbfgs fits of the same ROIs.
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <cuda_bf16.h>
@@ -124,7 +125,7 @@ __global__ void targets_kernel(const uint16_t *__restrict__ rois, const float *_
 // two, 6 us more over the eight of a gradient), 256 threads keep twice the
 // loads in flight, and bias, ReLU and mask go with the store instead of a
 // launch and a pass over the matrix each.  Gradient of 4,096 records: 303 ->
-// 182 us.
+// 182 us, then 143 with the weight gradients in one launch (layer_gradients).
 constexpr int kGemmM = 128, kGemmK = 128;
 
 // What a GEMM's result goes through before it is stored (only unsplit, beta
@@ -176,10 +177,31 @@ __device__ __forceinline__ void stage_k_rows(uint8_t *img, int rows, const float
     }
 }
 
-__global__ void __launch_bounds__(kGemmThreads, 1)
-    gemm_tc_kernel(int M, int N, int K, int bn, const float *__restrict__ A, long long sam, long long sak,
-                   const float *__restrict__ B, long long sbk, long long sbn, float *__restrict__ Cm, int ldc,
-                   float beta, int kper, float *__restrict__ part, int *__restrict__ err, GemmEpilogue ep) {
+// One product, its tiles and its share of K per split (z = 1: unsplit).
+struct GemmArgs {
+    int M, N, K, bn, kper, z;
+    const float *A, *B;
+    long long sam, sak, sbk, sbn;
+    float *C;
+    int ldc;
+    float beta;
+    float *part;   // z > 1: part[z][M][N]
+    // where set: B's column sums over K, unrounded, of split z at bsum[z][N]
+    // (bn divides kGemmThreads, B's K elements not adjacent)
+    float *bsum;
+    GemmEpilogue ep;
+
+    __host__ __device__ int n_tiles() const { return (N + bn - 1) / bn; }
+    __host__ __device__ int m_tiles() const { return (M + kGemmM - 1) / kGemmM; }
+};
+
+// Tile (tn, tm) of split tz; every thread of the CTA calls it.
+__device__ __forceinline__ void gemm_tile(const GemmArgs &g, int tn, int tm, int tz, int *__restrict__ err) {
+    const int M = g.M, N = g.N, bn = g.bn;
+    const float *__restrict__ A = g.A, *__restrict__ B = g.B;
+    const long long sam = g.sam, sak = g.sak, sbk = g.sbk, sbn = g.sbn;
+    float *__restrict__ part = g.part;
+    const GemmEpilogue &ep = g.ep;
     // operands with adjacent K elements and 16-byte aligned rows
     const bool a_rows = sak == 1 && (sam & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
     const bool b_rows = sbk == 1 && (sbn & 3) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0;
@@ -190,8 +212,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const uint32_t a_bytes = kGemmM * kGemmK * 2, b_bytes = (uint32_t)bn * kGemmK * 2;
     const uint32_t sA = sbase, sB = sbase + 2 * a_bytes, sBar = sB + 2 * b_bytes, sTmem = sBar + 16;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.y * kGemmM, n0 = blockIdx.x * bn;
-    const int kb = blockIdx.z * kper, ke = min(K, kb + kper);
+    const int m0 = tm * kGemmM, n0 = tn * bn;
+    const int kb = tz * g.kper, ke = min(g.K, kb + g.kper);
     const int nchunks = ke > kb ? (ke - kb + kGemmK - 1) / kGemmK : 0;
     uint32_t cols = 32;
     while ((int)cols < bn) cols <<= 1;
@@ -212,6 +234,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const uint32_t idesc = tc::instr_desc(kGemmM, bn);
     bool ok = true;
     int issued = 0;  // chunks whose MMAs were issued
+    float bs = 0.0f;  // this thread's part of its column's sum
+    const bool sums = g.bsum && tm == 0;
     for (int c = 0; c < nchunks; ++c) {
         const int buf = c & 1, k0 = kb + c * kGemmK;
         const int kc = min(kGemmK, (ke - k0 + 15) & ~15);  // this chunk's depth
@@ -250,6 +274,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                     v[e] = (gn < N && gk < ke) ? __ldg(B + (long long)gk * sbk + (long long)gn * sbn) : 0.0f;
                 }
                 *reinterpret_cast<uint4 *>(b_img + (size_t)(kg * bn + nn) * 16) = tc::pack8(v);
+                if (sums) bs += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
             }
         }
         tc::fence_async_smem();
@@ -272,15 +297,25 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         ok = ok && done;
     }
     tc::fence_after();
+    if (sums) {  // the threads of a column: kGemmThreads / bn
+        __shared__ float column[kGemmThreads];
+        column[tid] = bs;
+        __syncthreads();
+        if (tid < bn && n0 + tid < N) {
+            float v = 0.0f;
+            for (int j = tid; j < kGemmThreads; j += bn) v += column[j];
+            g.bsum[(size_t)tz * N + n0 + tid] = v;
+        }
+    }
     if (ok) {
         // 64 columns at a time through shared memory (the operand buffers are
         // free once the last MMA has ended): a warp of each half stores 32
         // columns of its 32 rows, then each warp writes 16 whole rows, lanes along
         // the columns (coalesced), what they read for it loaded ahead
         float *stage = reinterpret_cast<float *>(base);  // [128][65]
-        float *out = part ? part + (size_t)blockIdx.z * M * N : Cm;
-        const long long ld = part ? N : ldc;
-        const float b = part ? 0.0f : beta;
+        float *out = part ? part + (size_t)tz * M * N : g.C;
+        const long long ld = part ? N : g.ldc;
+        const float b = part ? 0.0f : g.beta;
         const int quarter = warp & 3, half = warp >> 2;
         for (int c0 = 0; c0 < bn; c0 += 64) {
 #pragma unroll
@@ -338,61 +373,155 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
 }
 
-// C = beta C + sum over the splits z = 0, 1, ... of part[z] (in that order).
-__global__ void gemm_reduce_kernel(const float *__restrict__ part, int splits, int M, int N, float *__restrict__ Cm,
-                                   int ldc, float beta) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)M * N) return;
-    const int r = (int)(i / N), c = (int)(i - (long long)r * N);
+__global__ void __launch_bounds__(kGemmThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmArgs g, int *__restrict__ err) {
+    gemm_tile(g, blockIdx.x, blockIdx.y, blockIdx.z, err);
+}
+
+// Products that do not wait for one another in one launch: CTA b takes tile and
+// split b of the concatenated lists.
+constexpr int kGemmBatch = 3;
+struct GemmBatch {
+    GemmArgs g[kGemmBatch];
+    float *column_sum[kGemmBatch];  // where g.bsum's splits go once added
+};
+__global__ void __launch_bounds__(kGemmThreads, 1) gemm_batch_kernel(const __grid_constant__ GemmBatch a, int *__restrict__ err) {
+    int b = blockIdx.x, i = 0;
+    while (b >= a.g[i].n_tiles() * a.g[i].m_tiles() * a.g[i].z) b -= a.g[i].n_tiles() * a.g[i].m_tiles() * a.g[i].z, ++i;
+    const GemmArgs &g = a.g[i];
+    const int tiles = g.n_tiles() * g.m_tiles(), tile = b % tiles;
+    gemm_tile(g, tile % g.n_tiles(), tile / g.n_tiles(), b / tiles, err);
+}
+
+// C(i) = beta C(i) + the sum over the splits z = 0, 1, ... of part[z](i), in that order.
+__device__ __forceinline__ void gemm_reduce(const GemmArgs &g, long long i) {
+    const int r = (int)(i / g.N), c = (int)(i - (long long)r * g.N);
     float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += part[(size_t)z * M * N + i];
-    float *dst = Cm + (size_t)r * ldc + c;
-    *dst = (beta == 0.0f) ? s : beta * (*dst) + s;
+#pragma unroll 16
+    for (int z = 0; z < g.z; ++z) s += g.part[(size_t)z * g.M * g.N + i];
+    float *dst = g.C + (size_t)r * g.ldc + c;
+    *dst = (g.beta == 0.0f) ? s : g.beta * (*dst) + s;
+}
+
+__global__ void gemm_reduce_kernel(const __grid_constant__ GemmArgs g) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < (long long)g.M * g.N) gemm_reduce(g, i);
+}
+
+__global__ void gemm_batch_reduce_kernel(const __grid_constant__ GemmBatch a) {
+    const GemmArgs &g = a.g[blockIdx.y];
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, total = (long long)g.M * g.N;
+    if (i < total) {
+        if (g.part) gemm_reduce(g, i);
+    } else if (i < total + g.N) {
+        const int c = (int)(i - total);
+        float s = 0.0f;
+        for (int z = 0; z < g.z; ++z) s += g.bsum[(size_t)z * g.N + c];
+        a.column_sum[blockIdx.y][c] = s;
+    }
 }
 
 size_t gemm_smem_bytes(int bn) { return 2 * (size_t)(kGemmM + bn) * kGemmK * 2 + 32 + 128; }
 
-// Split count for an M x N x K GEMM: enough CTAs to cover the SMs, at least
-// 256 of K per split, and partials within `ws_floats`.
-int gemm_splits(int M, int N, int K, int bn, size_t ws_floats) {
-    const int tiles = ((M + kGemmM - 1) / kGemmM) * ((N + bn - 1) / bn);
-    int s = 148 / tiles;
-    const int by_k = K / 256;
+// The tiles of a product.
+static GemmArgs gemm_args(int M, int N, int K, const float *A, long long sam, long long sak, const float *B, long long sbk,
+                          long long sbn, float *C, int ldc, float beta) {
+    GemmArgs g{};
+    g.M = M, g.N = N, g.K = K, g.z = 1, g.kper = K;
+    g.A = A, g.sam = sam, g.sak = sak;
+    g.B = B, g.sbk = sbk, g.sbn = sbn;
+    g.C = C, g.ldc = ldc, g.beta = beta;
+    g.bn = ((N + 15) / 16) * 16;
+    if (g.bn > 256) g.bn = 256;
+    // narrower tiles while they leave SMs without one: a tile's time is a chain
+    // of load latencies, and its B operand and epilogue shrink with it
+    while (g.bn >= 64 && g.bn % 32 == 0 && g.m_tiles() * g.n_tiles() < 74) g.bn /= 2;
+    return g;
+}
+
+// Splits K over at most `most` CTAs a tile, at least 256 of K each, with their
+// partials in `ws`; the floats of it that they take.
+static size_t gemm_split(GemmArgs &g, int most, float *ws, size_t ws_floats) {
+    int s = most;
+    const int by_k = g.K / 256;
     if (s > by_k) s = by_k;
     if (s > 64) s = 64;
-    while (s > 1 && (size_t)s * M * N > ws_floats) --s;
-    return s < 1 ? 1 : s;
+    while (s > 1 && (size_t)s * g.M * g.N > ws_floats) --s;
+    if (s < 1) s = 1;
+    int kper = (g.K + s - 1) / s;
+    kper = ((kper + kGemmK - 1) / kGemmK) * kGemmK;
+    g.z = kper > 0 ? (g.K + kper - 1) / kper : 1;
+    if (g.z <= 1) {
+        g.z = 1;
+        return 0;
+    }
+    g.kper = kper;
+    g.part = ws;
+    return (size_t)g.z * g.M * g.N;
+}
+
+static cudaError_t gemm_attributes() {
+    static bool set = false;
+    if (set) return cudaSuccess;
+    const int smem = (int)gemm_smem_bytes(256);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    set = e == cudaSuccess;
+    return e;
 }
 
 static cudaError_t gemm_epilogue(int M, int N, int K, const float *A, long long sam, long long sak, const float *B,
                                  long long sbk, long long sbn, float *C, int ldc, float beta, cudaStream_t s, float *ws,
                                  size_t ws_floats, int *err, const GemmEpilogue &ep) {
     if (M <= 0 || N <= 0) return cudaSuccess;
-    int bn = ((N + 15) / 16) * 16;
-    if (bn > 256) bn = 256;
-    // narrower tiles while they leave SMs without one: a tile's time is a chain
-    // of load latencies, and its B operand and epilogue shrink with it
-    const int m_tiles = (M + kGemmM - 1) / kGemmM;
-    while (bn >= 64 && bn % 32 == 0 && m_tiles * ((N + bn - 1) / bn) < 74) bn /= 2;
-    const bool plain = !ep.bias && !ep.act && !ep.mask;
-    const int splits = ws && plain ? gemm_splits(M, N, K, bn, ws_floats) : 1;
-    int kper = (K + splits - 1) / splits;
-    kper = ((kper + kGemmK - 1) / kGemmK) * kGemmK;
-    const int z = kper > 0 ? (K + kper - 1) / kper : 1;
-    const size_t smem = gemm_smem_bytes(bn);
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)gemm_smem_bytes(256));
-        if (e != cudaSuccess) return e;
-        attr_set = true;
+    GemmArgs g = gemm_args(M, N, K > 0 ? K : 0, A, sam, sak, B, sbk, sbn, C, ldc, beta);
+    g.ep = ep;
+    // enough CTAs to cover the SMs
+    if (ws && !ep.bias && !ep.act && !ep.mask) gemm_split(g, 148 / (g.m_tiles() * g.n_tiles()), ws, ws_floats);
+    cudaError_t e = gemm_attributes();
+    if (e != cudaSuccess) return e;
+    gemm_tc_kernel<<<dim3(g.n_tiles(), g.m_tiles(), g.z), kGemmThreads, gemm_smem_bytes(g.bn), s>>>(g, err);
+    if (g.z > 1) gemm_reduce_kernel<<<(int)(((long long)M * N + 255) / 256), 256, 0, s>>>(g);
+    return cudaGetLastError();
+}
+
+// The weight and bias gradients of a dense network's layers, dW = a^T d and the
+// column sums of d (rows x cols), in one launch and one that adds the splits:
+// as a product, its reduction and two passes of column sums per layer they
+// waited for one another without need (gradient of 4,096 records: 182 ->
+// 143 us).
+struct LayerGradient {
+    const float *a;
+    int in;
+    const float *d;
+    int cols;
+    float *dW, *db;
+};
+static cudaError_t layer_gradients(const LayerGradient (&l)[kGemmBatch], int rows, cudaStream_t s, float *ws,
+                                   size_t ws_floats, int *err) {
+    GemmBatch b{};
+    int tiles = 0, ctas = 0, bn = 0;
+    long long most = 0;
+    for (int i = 0; i < kGemmBatch; ++i) {
+        b.g[i] = gemm_args(l[i].in, l[i].cols, rows, l[i].a, 1, l[i].in, l[i].d, l[i].cols, 1, l[i].dW, l[i].cols, 0.0f);
+        if (kGemmThreads % b.g[i].bn != 0) return cudaErrorInvalidValue;
+        b.column_sum[i] = l[i].db;
+        tiles += b.g[i].m_tiles() * b.g[i].n_tiles();
     }
-    dim3 grid((N + bn - 1) / bn, (M + kGemmM - 1) / kGemmM, z > 1 ? z : 1);
-    float *part = z > 1 ? ws : nullptr;
-    gemm_tc_kernel<<<grid, kGemmThreads, smem, s>>>(M, N, K, bn, A, sam, sak, B, sbk, sbn, C, ldc, beta,
-                                                    z > 1 ? kper : (K > 0 ? K : 0), part, err, ep);
-    if (z > 1)
-        gemm_reduce_kernel<<<(int)(((long long)M * N + 255) / 256), 256, 0, s>>>(part, z, M, N, C, ldc, beta);
+    for (int i = 0; i < kGemmBatch; ++i) {
+        GemmArgs &g = b.g[i];
+        // room for the column sums of every layer's splits first
+        const size_t used = gemm_split(g, 148 / tiles, ws, ws_floats > (size_t)64 * g.N ? ws_floats - (size_t)64 * g.N : 0);
+        g.bsum = ws + used;
+        ws += used + (size_t)g.z * g.N;
+        ws_floats -= used + (size_t)g.z * g.N;
+        ctas += g.m_tiles() * g.n_tiles() * g.z;
+        bn = bn > g.bn ? bn : g.bn;
+        most = std::max(most, (long long)g.M * g.N + g.N);
+    }
+    cudaError_t e = gemm_attributes();
+    if (e != cudaSuccess) return e;
+    gemm_batch_kernel<<<ctas, kGemmThreads, gemm_smem_bytes(bn), s>>>(b, err);
+    gemm_batch_reduce_kernel<<<dim3((int)((most + 255) / 256), kGemmBatch), 256, 0, s>>>(b);
     return cudaGetLastError();
 }
 
@@ -402,31 +531,16 @@ cudaError_t gemm(int M, int N, int K, const float *A, long long sam, long long s
 }
 
 // ------------------------------------------------------ elementwise layers
-// Column sums of d (rows x cols) into out, for up to three matrices in one
-// launch pair, two passes with a fixed order: block (x, y, z) sums split y's
-// rows of 32 columns of matrix z into part[z][y][cols]; then the second kernel
-// adds the splits in order.
-struct ColumnSums {
-    const float *d;
-    int cols;
-    float *out;
-};
-struct ColumnSums3 {
-    ColumnSums m[3];
-};
-constexpr int kColsumStride = 256;  // columns of a matrix at most (several matrices in one launch)
-
-__global__ void colsum_part_kernel(ColumnSums3 a, long long rows, float *__restrict__ part, int stride) {
+// Column sums of d (rows x cols), two passes with a fixed order: block
+// (x, z) sums split z's rows of 32 columns into part[z][cols]; then
+// colsum_final adds the splits in order.
+__global__ void colsum_part_kernel(const float *__restrict__ d, long long rows, int cols, float *__restrict__ part) {
     __shared__ float acc[8][33];
-    const float *d = a.m[blockIdx.z].d;
-    const int cols = a.m[blockIdx.z].cols;
     const int c = blockIdx.x * 32 + threadIdx.x;
-    if (blockIdx.x * 32 >= cols) return;
     const long long per = (rows + gridDim.y - 1) / gridDim.y;
     const long long r0 = (long long)blockIdx.y * per, r1 = r0 + per < rows ? r0 + per : rows;
     float s = 0.0f;
     if (c < cols)
-#pragma unroll 8
         for (long long r = r0 + threadIdx.y; r < r1; r += 8) s += d[r * cols + c];
     acc[threadIdx.y][threadIdx.x] = s;
     __syncthreads();
@@ -434,39 +548,24 @@ __global__ void colsum_part_kernel(ColumnSums3 a, long long rows, float *__restr
         float t = 0.0f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) t += acc[k][threadIdx.x];
-        part[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * stride + c] = t;
+        part[(size_t)blockIdx.y * cols + c] = t;
     }
 }
 
-__global__ void colsum_final_kernel(ColumnSums3 a, const float *__restrict__ part, int splits, int stride) {
+__global__ void colsum_final_kernel(const float *__restrict__ part, int splits, int cols, float *__restrict__ g) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= a.m[blockIdx.z].cols) return;
+    if (c >= cols) return;
     float s = 0.0f;
-#pragma unroll 16
-    for (int z = 0; z < splits; ++z) s += part[((size_t)blockIdx.z * splits + z) * stride + c];
-    a.m[blockIdx.z].out[c] = s;
-}
-
-static int colsum_splits(long long rows) {
-    int splits = (int)((rows + 255) / 256);
-    if (splits > kColsumSplits) splits = kColsumSplits;
-    return splits < 1 ? 1 : splits;
+    for (int z = 0; z < splits; ++z) s += part[(size_t)z * cols + c];
+    g[c] = s;
 }
 
 cudaError_t column_sums(const float *d, long long rows, int cols, float *g, float *part, cudaStream_t s) {
-    const int splits = colsum_splits(rows);
-    const ColumnSums3 a{{{d, cols, g}, {}, {}}};
-    colsum_part_kernel<<<dim3((cols + 31) / 32, splits, 1), dim3(32, 8), 0, s>>>(a, rows, part, cols);
-    colsum_final_kernel<<<dim3((cols + 127) / 128, 1, 1), 128, 0, s>>>(a, part, splits, cols);
-    return cudaGetLastError();
-}
-
-// Three matrices of at most kColsumStride columns; part holds 3 kColsumSplits kColsumStride floats.
-static cudaError_t column_sums3(const ColumnSums (&m)[3], long long rows, float *part, cudaStream_t s) {
-    const int splits = colsum_splits(rows);
-    const ColumnSums3 a{{m[0], m[1], m[2]}};
-    colsum_part_kernel<<<dim3(kColsumStride / 32, splits, 3), dim3(32, 8), 0, s>>>(a, rows, part, kColsumStride);
-    colsum_final_kernel<<<dim3(kColsumStride / 128, 1, 3), 128, 0, s>>>(a, part, splits, kColsumStride);
+    int splits = (int)((rows + 255) / 256);
+    if (splits > kColsumSplits) splits = kColsumSplits;
+    if (splits < 1) splits = 1;
+    colsum_part_kernel<<<dim3((cols + 31) / 32, splits), dim3(32, 8), 0, s>>>(d, rows, cols, part);
+    colsum_final_kernel<<<(cols + 127) / 128, 128, 0, s>>>(part, splits, cols, g);
     return cudaGetLastError();
 }
 
@@ -948,32 +1047,21 @@ cudaError_t backward(qcs_learned_net *net, int rows, cudaStream_t s) {
     const Views w = views(net->d_par, net->kin, net->nout);
     const Views g = views(net->d_grad, net->kin, net->nout);
     cudaError_t e;
-    // layer 3: dW3 = a2^T dy, db3 = colsum(dy), d2 = dy W3^T
     const int no = net->nout;
-    if ((e = L::gemm(L::kHidden, no, rows, net->d_a2, 1, L::kHidden, net->d_dy, no, 1, g.W3, no, 0.0f,
-                     s, net->d_ws, net->ws_floats, net->d_err)))
-        return e;
-    // d2 = (dy W3^T) masked by z2 > 0
+    // d2 = (dy W3^T) masked by z2 > 0, d1 = (d2 W2^T) masked by z1 > 0
     L::GemmEpilogue ep;
     ep.mask = net->d_z2;
     if ((e = L::gemm_epilogue(rows, L::kHidden, no, net->d_dy, no, 1, w.W3, 1, no, net->d_d2, L::kHidden, 0.0f, s,
                               net->d_ws, net->ws_floats, net->d_err, ep)))
         return e;
-    // layer 2
-    if ((e = L::gemm(L::kHidden, L::kHidden, rows, net->d_a1, 1, L::kHidden, net->d_d2, L::kHidden, 1, g.W2,
-                     L::kHidden, 0.0f, s, net->d_ws, net->ws_floats, net->d_err)))
-        return e;
     ep.mask = net->d_z1;
     if ((e = L::gemm_epilogue(rows, L::kHidden, L::kHidden, net->d_d2, L::kHidden, 1, w.W2, 1, L::kHidden, net->d_d1,
                               L::kHidden, 0.0f, s, net->d_ws, net->ws_floats, net->d_err, ep)))
         return e;
-    // layer 1
-    if ((e = L::gemm(net->kin, L::kHidden, rows, net->d_x, 1, net->kin, net->d_d1, L::kHidden, 1, g.W1, L::kHidden,
-                     0.0f, s, net->d_ws, net->ws_floats, net->d_err)))
-        return e;
-    // the bias gradients
-    const L::ColumnSums sums[3] = {{net->d_dy, no, g.b3}, {net->d_d2, L::kHidden, g.b2}, {net->d_d1, L::kHidden, g.b1}};
-    return L::column_sums3(sums, rows, net->d_ws, s);
+    const L::LayerGradient layers[L::kGemmBatch] = {{net->d_x, net->kin, net->d_d1, L::kHidden, g.W1, g.b1},
+                                                    {net->d_a1, L::kHidden, net->d_d2, L::kHidden, g.W2, g.b2},
+                                                    {net->d_a2, L::kHidden, net->d_dy, no, g.W3, g.b3}};
+    return L::layer_gradients(layers, rows, s, net->d_ws, net->ws_floats, net->d_err);
 }
 
 // xorshift-based permutation of [0, n) on the host, copied to the device
