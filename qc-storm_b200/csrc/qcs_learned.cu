@@ -125,7 +125,9 @@ __global__ void targets_kernel(const uint16_t *__restrict__ rois, const float *_
 // two, 6 us more over the eight of a gradient), 256 threads keep twice the
 // loads in flight, and bias, ReLU and mask go with the store instead of a
 // launch and a pass over the matrix each.  Gradient of 4,096 records: 303 ->
-// 182 us, then 143 with the weight gradients in one launch (layer_gradients).
+// 182 us, 143 with the weight gradients in one launch (layer_gradients), 133 with
+// whole chunks staged by constant steps (the loops' index arithmetic was half of
+// a product's instructions; convolutional network 2,292 -> 1,984 us).
 constexpr int kGemmM = 128, kGemmK = 128;
 
 // What a GEMM's result goes through before it is stored (only unsplit, beta
@@ -177,6 +179,60 @@ __device__ __forceinline__ void stage_k_rows(uint8_t *img, int rows, const float
     }
 }
 
+// stage_k_rows for a whole chunk (kGemmK deep) of ROWS rows, all in range: every
+// address is a constant step from the thread's first, and all loads are issued
+// before the first store.
+template <int ROWS>
+__device__ __forceinline__ void stage_k_full(uint8_t *img, const float *__restrict__ src, long long ld) {
+    constexpr int WARPS = kGemmThreads / 32, G = ROWS / 8;       // groups of 8 rows
+    constexpr int SETS = G > WARPS ? G / WARPS : 1;              // groups per warp
+    constexpr int KSTEP = 16 * (G < WARPS ? WARPS / G : 1), PER = kGemmK / KSTEP;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k4 = lane & 3;
+    const int r = (warp % G) * 8 + (lane >> 2), k0 = G < WARPS ? warp / G * 16 : 0;
+    uint8_t *dst = img + (size_t)((k0 >> 3) + (k4 >> 1)) * ROWS * 16 + r * 16 + (k4 & 1) * 8;
+    float4 v[SETS][PER];
+#pragma unroll
+    for (int s = 0; s < SETS; ++s) {
+        const float *p = src + (long long)(r + s * WARPS * 8) * ld + k0 + k4 * 4;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) v[s][i] = __ldg(reinterpret_cast<const float4 *>(p + i * KSTEP));
+    }
+#pragma unroll
+    for (int s = 0; s < SETS; ++s)
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[s][i].x, v[s][i].y), __floats2bfloat162_rn(v[s][i].z, v[s][i].w)};
+            *reinterpret_cast<uint2 *>(dst + (i * (KSTEP / 8) * ROWS + s * WARPS * 8) * 16) = *reinterpret_cast<uint2 *>(h);
+        }
+}
+
+// The same for an operand whose rows are adjacent in memory (element (r, k) at
+// src[r + k * ld]); each thread's column sum when SUM (a thread keeps its row).
+template <int ROWS>
+__device__ __forceinline__ float stage_r_full(uint8_t *img, const float *__restrict__ src, long long ld) {
+    constexpr int KG = kGemmThreads / ROWS, PER = kGemmK / 8 / KG;  // K groups of 8 at a time, and per thread
+    constexpr int AHEAD = PER < 4 ? PER : 4;
+    const int r = threadIdx.x % ROWS, kg = threadIdx.x / ROWS;
+    uint8_t *dst = img + (size_t)(kg * ROWS + r) * 16;
+    float sum = 0.0f;
+#pragma unroll
+    for (int b = 0; b < PER; b += AHEAD) {
+        float v[AHEAD][8];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            const float *p = src + r + (long long)((b + i) * KG + kg) * 8 * ld;
+#pragma unroll
+            for (int e = 0; e < 8; ++e, p += ld) v[i][e] = __ldg(p);
+        }
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) {
+            *reinterpret_cast<uint4 *>(dst + (size_t)(b + i) * KG * ROWS * 16) = tc::pack8(v[i]);
+            sum += ((v[i][0] + v[i][1]) + (v[i][2] + v[i][3])) + ((v[i][4] + v[i][5]) + (v[i][6] + v[i][7]));
+        }
+    }
+    return sum;
+}
+
 // One product, its tiles and its share of K per split (z = 1: unsplit).
 struct GemmArgs {
     int M, N, K, bn, kper, z;
@@ -195,9 +251,11 @@ struct GemmArgs {
     __host__ __device__ int m_tiles() const { return (M + kGemmM - 1) / kGemmM; }
 };
 
-// Tile (tn, tm) of split tz; every thread of the CTA calls it.
+// Tile (tn, tm) of split tz; every thread of the CTA calls it.  BN: g.bn, or 0
+// for any (whole chunks are then not staged by constant steps).
+template <int BN>
 __device__ __forceinline__ void gemm_tile(const GemmArgs &g, int tn, int tm, int tz, int *__restrict__ err) {
-    const int M = g.M, N = g.N, bn = g.bn;
+    const int M = g.M, N = g.N, bn = BN > 0 ? BN : g.bn;
     const float *__restrict__ A = g.A, *__restrict__ B = g.B;
     const long long sam = g.sam, sak = g.sak, sbk = g.sbk, sbn = g.sbn;
     float *__restrict__ part = g.part;
@@ -244,7 +302,14 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs &g, int tn, int tm, int
             if (!ok) break;
         }
         uint8_t *a_img = base + buf * a_bytes, *b_img = base + 2 * a_bytes + buf * b_bytes;
-        if (a_rows) {
+        // the whole chunk inside the operands
+        const bool whole_k = kc == kGemmK && k0 + kGemmK <= ke;
+        const bool whole_a = whole_k && m0 + kGemmM <= M, whole_b = whole_k && n0 + bn <= N;
+        if (whole_a && a_rows) {
+            stage_k_full<kGemmM>(a_img, A + (long long)m0 * sam + k0, sam);
+        } else if (whole_a && sam == 1) {
+            stage_r_full<kGemmM>(a_img, A + m0 + (long long)k0 * sak, sak);
+        } else if (a_rows) {
             stage_k_rows(a_img, kGemmM, A, sam, m0, M, k0, ke, kc);
         } else {
             // row tid % 128, every other K group of the chunk
@@ -260,7 +325,12 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs &g, int tn, int tm, int
                 *reinterpret_cast<uint4 *>(a_img + (size_t)(kg * kGemmM + row) * 16) = tc::pack8(v);
             }
         }
-        if (b_rows) {
+        if (BN > 0 && whole_b && b_rows) {
+            stage_k_full<BN ? BN : 128>(b_img, B + (long long)n0 * sbn + k0, sbn);
+        } else if (BN > 0 && whole_b && sbn == 1) {
+            const float sum = stage_r_full<BN ? BN : 128>(b_img, B + n0 + (long long)k0 * sbk, sbk);
+            if (sums) bs += sum;
+        } else if (b_rows) {
             stage_k_rows(b_img, bn, B, sbn, n0, N, k0, ke, kc);
         } else {
             // bn rows (n) x 8 K groups
@@ -373,8 +443,9 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs &g, int tn, int tm, int
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
 }
 
+template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmArgs g, int *__restrict__ err) {
-    gemm_tile(g, blockIdx.x, blockIdx.y, blockIdx.z, err);
+    gemm_tile<BN>(g, blockIdx.x, blockIdx.y, blockIdx.z, err);
 }
 
 // Products that do not wait for one another in one launch: CTA b takes tile and
@@ -389,7 +460,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_batch_kernel(const __gri
     while (b >= a.g[i].n_tiles() * a.g[i].m_tiles() * a.g[i].z) b -= a.g[i].n_tiles() * a.g[i].m_tiles() * a.g[i].z, ++i;
     const GemmArgs &g = a.g[i];
     const int tiles = g.n_tiles() * g.m_tiles(), tile = b % tiles;
-    gemm_tile(g, tile % g.n_tiles(), tile / g.n_tiles(), b / tiles, err);
+    const int tn = tile % g.n_tiles(), tm = tile / g.n_tiles(), tz = b / tiles;
+    if (g.bn == 32)
+        gemm_tile<32>(g, tn, tm, tz, err);
+    else if (g.bn == 16)
+        gemm_tile<16>(g, tn, tm, tz, err);
+    else
+        gemm_tile<0>(g, tn, tm, tz, err);
 }
 
 // C(i) = beta C(i) + the sum over the splits z = 0, 1, ... of part[z](i), in that order.
@@ -463,7 +540,10 @@ static cudaError_t gemm_attributes() {
     static bool set = false;
     if (set) return cudaSuccess;
     const int smem = (int)gemm_smem_bytes(256);
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tc_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     set = e == cudaSuccess;
     return e;
@@ -479,7 +559,8 @@ static cudaError_t gemm_epilogue(int M, int N, int K, const float *A, long long 
     if (ws && !ep.bias && !ep.act && !ep.mask) gemm_split(g, 148 / (g.m_tiles() * g.n_tiles()), ws, ws_floats);
     cudaError_t e = gemm_attributes();
     if (e != cudaSuccess) return e;
-    gemm_tc_kernel<<<dim3(g.n_tiles(), g.m_tiles(), g.z), kGemmThreads, gemm_smem_bytes(g.bn), s>>>(g, err);
+    auto k = g.bn == 16 ? gemm_tc_kernel<16> : (g.bn == 32 ? gemm_tc_kernel<32> : (g.bn == 128 ? gemm_tc_kernel<128> : gemm_tc_kernel<0>));
+    k<<<dim3(g.n_tiles(), g.m_tiles(), g.z), kGemmThreads, gemm_smem_bytes(g.bn), s>>>(g, err);
     if (g.z > 1) gemm_reduce_kernel<<<(int)(((long long)M * N + 255) / 256), 256, 0, s>>>(g);
     return cudaGetLastError();
 }
