@@ -203,6 +203,9 @@ int qcs_extract_reset_roi_num(qcs_extract_data *c, void *stream);
  * (waits for the last extraction); NULL on error. */
 const uint16_t *qcs_extract_h_image_roi(qcs_extract_data *c);
 const float *qcs_extract_h_wle_para(qcs_extract_data *c);
+/* The accumulated count and both host copies with one read of the count (the
+ * three calls above read it, and wait for the device, once each). */
+int qcs_extract_read_records(qcs_extract_data *c, int *n, const uint16_t **h_rois, const float **h_wle);
 /* d_ImageROI-equivalent accumulation buffer and Get_d_WLEPara()
  * (LDROIExtraction.cu:201), device memory, to feed qcs_loc_localize_device
  * without a host round trip; qcs_extract_device_roi_num: device int holding

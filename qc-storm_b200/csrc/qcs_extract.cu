@@ -897,6 +897,16 @@ static int copy_to_host(qcs_extract_data *c) {
     return QCS_OK;
 }
 
+int qcs_extract_read_records(qcs_extract_data *c, int *n, const uint16_t **h_rois, const float **h_wle) {
+    if (!c || !n || !h_rois || !h_wle) return fail(QCS_ERR_ARG, "null argument");
+    const int st = copy_to_host(c);
+    if (st) return st;
+    *n = c->h_state[qcs::kStAccum];
+    *h_rois = c->h_rois;
+    *h_wle = c->h_wle;
+    return QCS_OK;
+}
+
 const uint16_t *qcs_extract_h_image_roi(qcs_extract_data *c) {
     if (!c || copy_to_host(c) != QCS_OK) return nullptr;
     return c->h_rois;

@@ -115,6 +115,7 @@ _SIGS = {
     "qcs_extract_reset_roi_num": (C.c_int, [C.c_void_p, C.c_void_p]),
     "qcs_extract_h_image_roi": (C.c_void_p, [C.c_void_p]),
     "qcs_extract_h_wle_para": (C.c_void_p, [C.c_void_p]),
+    "qcs_extract_read_records": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_void_p), C.POINTER(C.c_void_p)]),
     "qcs_extract_d_image_roi": (C.c_void_p, [C.c_void_p]),
     "qcs_extract_d_wle_para": (C.c_void_p, [C.c_void_p]),
     "qcs_extract_device_roi_num": (C.c_void_p, [C.c_void_p]),
@@ -488,15 +489,13 @@ class ExtractContext:
 
     def records(self):
         """Host copies of the accumulated (records[n, R(R+1)] uint16, wle[n, 6] float32)."""
-        n = self.accumulated()
-        pr = self.lib.qcs_extract_h_image_roi(self.h)
-        pw = self.lib.qcs_extract_h_wle_para(self.h)
-        if not pr or not pw:
-            raise QcsError(4, self.lib.qcs_last_error().decode())
+        count, pr, pw = C.c_int(0), C.c_void_p(), C.c_void_p()
+        check(self.lib.qcs_extract_read_records(self.h, C.byref(count), C.byref(pr), C.byref(pw)))
+        n = count.value
         if n == 0:
             return np.zeros((0, self.whole), np.uint16), np.zeros((0, 6), np.float32)
-        rois = np.ctypeslib.as_array((C.c_uint16 * (self.whole * n)).from_address(pr)).reshape(n, self.whole).copy()
-        wle = np.ctypeslib.as_array((C.c_float * (6 * n)).from_address(pw)).reshape(n, 6).copy()
+        rois = np.ctypeslib.as_array((C.c_uint16 * (self.whole * n)).from_address(pr.value)).reshape(n, self.whole).copy()
+        wle = np.ctypeslib.as_array((C.c_float * (6 * n)).from_address(pw.value)).reshape(n, 6).copy()
         return rois, wle
 
     def frame_range(self):
