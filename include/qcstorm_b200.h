@@ -465,8 +465,10 @@ int qcs_fit_single_group_device(int loc_type, const qcs_loc_para *p, const uint1
  * (also 4 and 16 for GS2D 7x7), and keeps in the context, per batch size,
  * the fastest; qcs_loc_localize_device then fits a batch of n records with
  * the lanes of the first entry whose size is >= n (larger batches: one
- * thread per ROI).  Every choice gives the same rows bit for bit.  n >= 64
- * records; overwrites the context's rows. */
+ * thread per ROI).  Without a table it chooses by the queue's length: 32 or 16
+ * lanes per ROI for short ones, one thread per ROI for long ones.  Every choice
+ * gives the same rows bit for bit.  n >= 64 records; overwrites the context's
+ * rows. */
 int qcs_loc_autotune(qcs_loc_data *c, const qcs_loc_para *p, const uint16_t *d_rois, const float *d_wle, int n,
                      void *stream);
 /* The tuning table (returns its length; sizes / lanes may be NULL), or sets it
@@ -478,9 +480,8 @@ int qcs_loc_set_tuning(qcs_loc_data *c, const int *sizes, const int *lanes, int 
  * 256, ... records with the lane-group kernel and with one thread per ROI,
  * and keeps the longest queue for which the lane groups are faster: a stage
  * whose queue (read on the device) is at most that long uses them.  The
- * limits (-1: one thread per ROI always; 0: the built-in default, about three
- * waves of the lane-group kernel), read or set here.  The rows are the same
- * either way. */
+ * limits (-1: one thread per ROI always; 0: the built-in default, 30,000),
+ * read or set here.  The rows are the same either way. */
 int qcs_loc_tuning_multi(const qcs_loc_data *c, int *limit_2e, int *limit_3e);
 int qcs_loc_set_tuning_multi(qcs_loc_data *c, int limit_2e, int limit_3e);
 /* Per-GPU tuning cache: writes the context's tuning (lanes table and

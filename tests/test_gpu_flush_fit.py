@@ -4,7 +4,7 @@ fit_single_kernel takes exp and log without subnormal handling where the
 background or the exponents' range allows it, and the general forms for a warp
 where some ROI does not.  Records whose fits clamp the background to zero, push
 widths and positions far out, or hold constant, zero or saturated pixels reach
-both sides of that line.  fit_single_group_kernel, which evaluates the same
+both sides of that line.  fit_lanes_kernel, which evaluates the same
 terms with other code, must give the same rows bit for bit (NaN as NaN), on
 records at 4-byte and at 2-byte boundaries.
 """
