@@ -731,7 +731,8 @@ int qcs_extract_init_ex(const qcs_loc_para *p, int max_batched_num, int capacity
     cudaError_t e = cudaMalloc((void **)&c->d_raw, px * sizeof(uint16_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_bg, px * sizeof(uint16_t));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_pos, px_pad);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_chunk, (c->nchunks_max + (size_t)(c->nchunks_max + qcs::kSuper - 1) / qcs::kSuper) * sizeof(int));
+    const size_t counts = c->nchunks_max + (size_t)(c->nchunks_max + qcs::kSuper - 1) / qcs::kSuper;
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_chunk, counts * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_state, qcs::kStNum * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_var, 4 * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_var_acc, 4 * sizeof(unsigned long long));

@@ -505,8 +505,9 @@ cudaError_t wle_sorter_create(int capacity, void *scratch, WleSorter **out) {
 
     cudaGraphConditionalHandle h = 0;
     cudaGraphNode_t kn = nullptr, cn = nullptr;
-    cudaError_t e = cudaMemset(w->flag, 0, 3 * sizeof(int));
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&w->cap, cudaStreamNonBlocking);
+    cudaError_t e = cudaStreamCreateWithFlags(&w->cap, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w->flag, 0, 3 * sizeof(int), w->cap);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(w->cap);  // before a call on any stream
     if (e == cudaSuccess) e = cudaGraphCreate(&w->graph, 0);
     if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, w->graph, 0, cudaGraphCondAssignDefault);
     if (e == cudaSuccess) {
