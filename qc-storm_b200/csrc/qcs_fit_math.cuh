@@ -751,6 +751,12 @@ __device__ __forceinline__ float ex2_flush(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// 2^x with its subnormal results (and x log2 e for x: __expf of every float).
+__device__ __forceinline__ float ex2_keep(float x) {
+    float y;
+    asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ float lg2_flush(float x) {
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -760,6 +766,11 @@ __device__ __forceinline__ f32x2 ex2_flush2(f32x2 x) {
     float a, b;
     unpack2(x, a, b);
     return pack2(ex2_flush(a), ex2_flush(b));
+}
+__device__ __forceinline__ f32x2 ex2_keep2(f32x2 x) {
+    float a, b;
+    unpack2(x, a, b);
+    return pack2(ex2_keep(a), ex2_keep(b));
 }
 __device__ __forceinline__ f32x2 lg2_flush2(f32x2 x) {
     float a, b;
@@ -838,7 +849,12 @@ struct LaneLayout {
 //    that parameter, and after it is moved back its rounded value stays: 26
 //    exponentials instead of 66 for three emitters), then lane j sums point j.
 //  - The inverse Hessian's update: one element per lane and round.
-// A line-search term takes two pixels at a time in packed instructions.
+// A line-search term takes two pixels at a time in packed instructions, with the
+// flushing exp and log where safe() and, for several emitters, exps_normal() say
+// that they change nothing.  The latter is asked once a line search, and point by
+// point only where the line as a whole fails it: 2E, 3E and 1E stages of 100,000
+// 11x11 records 2,083 -> 2,095 us with it (2,119 with the keeping exp throughout,
+// 2,106 with the general terms where a point fails).
 // Only for roundings fixed in the source (DIST, SUM2 != kCompiler).  pos: the
 // pixels' centres, col + 0.5 of PIXP pixels, then row + 0.5.
 template <int R, int KIND, int DIST, int G>
@@ -856,12 +872,33 @@ struct LaneFit {
         if (LOW) return v < 0.01f ? 0.01f : v;
         return v < 0.0f ? 0.0f : v;
     }
-    // The flushing forms change nothing at clamped parameters with this
-    // background and sum of amplitudes: an exp below 2^-126 times its amplitude
-    // is lost under the background also in the partial sums of the model
-    // (flush_safe).
-    __device__ __forceinline__ static bool safe(float B, float sumA) {
-        return B * QCS_BSCALE >= fmaxf(1e-30f, sumA * QCS_ASCALE * 0x1p-45f);
+    // Whether the flushing log, and for one emitter the flushing exp, change
+    // nothing at clamped parameters with this background and amplitude: the
+    // model is then at least the background, a normal number, and an exp below
+    // 2^-126 times the amplitude is lost under it (flush_safe).
+    __device__ __forceinline__ static bool safe(float B, float A) {
+        return B * QCS_BSCALE >= (E::M == 1 ? fmaxf(1e-30f, A * QCS_ASCALE * 0x1p-45f) : 1e-30f);
+    }
+    // Whether no exp is subnormal at any (clamped) parameters between v and u and
+    // 0.01 beyond, so that the flushing exp is the other's value.  With several
+    // emitters the background's size does not settle that: where one emitter's
+    // product is a tie of the model's sum, another's subnormal exp decides the
+    // rounding.  The farthest pixel and the widest spread bound every exponent;
+    // 86 leaves its rounding below 126 ln 2 = 87.3.  A NaN parameter is NaN in
+    // both forms.
+    __device__ __forceinline__ static bool exps_normal(const float (&v)[P], const float (&u)[P]) {
+        if (E::M == 1) return true;  // safe() is enough
+        float dx = 0.0f, dy = 0.0f, sx = 0.0f, sy = 0.0f;
+#pragma unroll
+        for (int m = 0; m < E::M; m++) {
+            dx = fmaxf(dx, fmaxf(fabsf(v[E::x(m)] - R / 2.0f), fabsf(u[E::x(m)] - R / 2.0f)));
+            dy = fmaxf(dy, fmaxf(fabsf(v[E::y(m)] - R / 2.0f), fabsf(u[E::y(m)] - R / 2.0f)));
+            sx = fmaxf(sx, fmaxf(v[E::sx(m)], u[E::sx(m)]));
+            sy = fmaxf(sy, fmaxf(v[E::sy(m)], u[E::sy(m)]));
+        }
+        dx += R / 2 + 0.01f;
+        dy += R / 2 + 0.01f;
+        return (dx * dx * (sx + 0.01f) + dy * dy * (sy + 0.01f)) * QCS_SSCALE <= 86.0f;
     }
     __device__ __forceinline__ static float exponent(float cp, float rp, float x, float y, float sx, float sy) {
         const float dx = cp - x, dy = rp - y;
@@ -869,8 +906,10 @@ struct LaneFit {
                                                  __fmul_rn(__fmul_rn(dy, dy), sy), QCS_SSCALE);
         return __fmul_rn(__fmul_rn(-sum_of_products<DIST>(dx, dx, dy, dy), sx), QCS_SSCALE);
     }
+    template <bool KEEP>
     __device__ __forceinline__ static float expo(float cp, float rp, float x, float y, float sx, float sy) {
-        return ex2_flush(__fmul_rn(exponent(cp, rp, x, y, sx, sy), kLog2E));
+        const float t = __fmul_rn(exponent(cp, rp, x, y, sx, sy), kLog2E);
+        return KEEP ? ex2_keep(t) : ex2_flush(t);
     }
     // deviance term from the emitters' exponentials e and amplitudes A, and the background B (fit units)
     __device__ __forceinline__ static float term(const float (&e)[E::M], const float (&A)[E::M], float B, float2 pl) {
@@ -894,6 +933,7 @@ struct LaneFit {
     }
     __device__ __forceinline__ static f32x2 pair_at(const float *p) { return *reinterpret_cast<const f32x2 *>(p); }
     // expo and term of two pixels
+    template <bool KEEP>
     __device__ __forceinline__ static f32x2 expo2(f32x2 cp, f32x2 rp, f32x2 x, f32x2 y, f32x2 sx, f32x2 sy) {
         const f32x2 s01 = pack2(QCS_SSCALE, QCS_SSCALE), dx = sub2(cp, x), dy = sub2(rp, y);
         f32x2 t;
@@ -904,7 +944,7 @@ struct LaneFit {
             const f32x2 d = DIST == kFuseFirst ? fma2(dx, dx, mul2(dy, dy)) : fma2(dy, dy, mul2(dx, dx));
             t = mul2(mul2(mul2(d, sx), s01), pack2(kLog2E, kLog2E));
         }
-        return ex2_flush2(t);
+        return KEEP ? ex2_keep2(t) : ex2_flush2(t);
     }
     __device__ __forceinline__ static f32x2 term2(const f32x2 (&e)[E::M], const f32x2 (&A)[E::M], f32x2 B, f32x2 pix,
                                                   f32x2 lg) {
@@ -948,43 +988,48 @@ struct LaneFit {
         return total;
     }
 
-    // Losses at x + d * step[j], j < KPTS, in every lane.
-    __device__ __forceinline__ void losses(const float *x, const float *d, const float (&step)[KPTS],
+    // The terms of pixels 2 k0, 2 k0 + 1, 2 (k0 + LP), ... at v into part, two at a time.
+    template <bool KEEP>
+    __device__ __forceinline__ void terms(const float (&v)[P], float *part, int k0) const {
+        f32x2 A2[E::M], x2[E::M], y2[E::M], sx2[E::M], sy2[E::M];
+        const f32x2 B2 = pack2(v[P - 1] * QCS_BSCALE, v[P - 1] * QCS_BSCALE);
+#pragma unroll
+        for (int m = 0; m < E::M; m++) {
+            const float A = v[E::a(m)] * QCS_ASCALE, sx = E::AS ? v[E::sx(m)] : -v[E::sx(m)], sy = v[E::sy(m)];
+            A2[m] = pack2(A, A);
+            x2[m] = pack2(v[E::x(m)], v[E::x(m)]);
+            y2[m] = pack2(v[E::y(m)], v[E::y(m)]);
+            sx2[m] = pack2(sx, sx);
+            sy2[m] = pack2(sy, sy);
+        }
+// (unrolled rounds are slower: the loop is short and the kernel is bound by instruction fetch as well)
+#pragma unroll 1
+        for (int k = 2 * k0; k < PIX; k += 2 * LP) {
+            const f32x2 cp = pair_at(pos + k), rp = pair_at(pos + PIXP + k);
+            f32x2 e[E::M];
+#pragma unroll
+            for (int m = 0; m < E::M; m++) e[m] = expo2<KEEP>(cp, rp, x2[m], y2[m], sx2[m], sy2[m]);
+            *reinterpret_cast<f32x2 *>(part + k) = term2(e, A2, B2, pair_at(s + L::VAL + k), pair_at(s + L::LOG + k));
+        }
+    }
+
+    // Losses at x + d * step[j], j < KPTS, in every lane; normal: exps_normal
+    // holds there.
+    __device__ __forceinline__ void losses(const float *x, const float *d, const float (&step)[KPTS], bool normal,
                                            float (&f)[KPTS]) const {
         const int j = lane / LP, k0 = lane - j * LP;
         float st = step[0];
 #pragma unroll
         for (int i = 1; i < KPTS; i++) st = j == i ? step[i] : st;
-        float v[P], A[E::M], sumA = 0.0f;
+        float v[P];
 #pragma unroll
         for (int k = 0; k < P; k++) v[k] = bound(__fmaf_rn(d[k], st, x[k]));
-#pragma unroll
-        for (int m = 0; m < E::M; m++) {
-            A[m] = v[E::a(m)];
-            sumA += A[m];
-        }
         float *part = s + L::PART + j * PIXP;
-        if (__all_sync(mask, safe(v[P - 1], sumA))) {
-            f32x2 A2[E::M], x2[E::M], y2[E::M], sx2[E::M], sy2[E::M];
-            const f32x2 B2 = pack2(v[P - 1] * QCS_BSCALE, v[P - 1] * QCS_BSCALE);
-#pragma unroll
-            for (int m = 0; m < E::M; m++) {
-                const float sx = E::AS ? v[E::sx(m)] : -v[E::sx(m)], sy = v[E::sy(m)];
-                A2[m] = pack2(A[m] * QCS_ASCALE, A[m] * QCS_ASCALE);
-                x2[m] = pack2(v[E::x(m)], v[E::x(m)]);
-                y2[m] = pack2(v[E::y(m)], v[E::y(m)]);
-                sx2[m] = pack2(sx, sx);
-                sy2[m] = pack2(sy, sy);
-            }
-// (unrolled rounds are slower: the loop is short and the kernel is bound by instruction fetch as well)
-#pragma unroll 1
-            for (int k = 2 * k0; k < PIX; k += 2 * LP) {
-                const f32x2 cp = pair_at(pos + k), rp = pair_at(pos + PIXP + k);
-                f32x2 e[E::M];
-#pragma unroll
-                for (int m = 0; m < E::M; m++) e[m] = expo2(cp, rp, x2[m], y2[m], sx2[m], sy2[m]);
-                *reinterpret_cast<f32x2 *>(part + k) = term2(e, A2, B2, pair_at(s + L::VAL + k), pair_at(s + L::LOG + k));
-            }
+        if (__all_sync(mask, safe(v[P - 1], v[0]))) {
+            if (normal || __all_sync(mask, exps_normal(v, v)))
+                terms<false>(v, part, k0);
+            else
+                terms<true>(v, part, k0);
         } else {
 #pragma unroll 1
             for (int k = k0; k < PIX; k += LP) part[k] = term_general(k, v);
@@ -996,9 +1041,45 @@ struct LaneFit {
         __syncwarp(mask);
     }
 
-    __device__ __forceinline__ void gradient(const float *x, float *grad) const {
+    // The terms of this lane's pixels at the gradient's 2P points into part (see gradient).
+    template <bool KEEP>
+    __device__ __forceinline__ void point_terms(const float (&b)[P], const float (&lo)[P], const float (&hi)[P],
+                                                const float (&r)[P], float *part) const {
+#pragma unroll 1
+        for (int k = lane; k < PIX; k += G) {
+            const float2 c = make_float2(pos[k], pos[PIXP + k]), pl = make_float2(s[L::VAL + k], s[L::LOG + k]);
+            float v[P], e[E::M];
+#pragma unroll
+            for (int i = 0; i < P; i++) v[i] = b[i];
+#pragma unroll
+            for (int m = 0; m < E::M; m++) e[m] = 0.0f;
+#pragma unroll
+            for (int i = 0; i < P; i++) {
+                float A[E::M], en[E::M];
+                // emitters whose exponent the parameter before this one moved, or none is known yet
+#pragma unroll
+                for (int m = 0; m < E::M; m++)
+                    if (!E::in(m, i) && (i == 0 || E::in(m, i - 1)))
+                        e[m] = expo<KEEP>(c.x, c.y, v[E::x(m)], v[E::y(m)], v[E::sx(m)], v[E::sy(m)]);
+#pragma unroll
+                for (int side = 0; side < 2; side++) {
+                    v[i] = side ? hi[i] : lo[i];
+#pragma unroll
+                    for (int m = 0; m < E::M; m++) {
+                        A[m] = v[E::a(m)];
+                        en[m] = E::in(m, i) ? expo<KEEP>(c.x, c.y, v[E::x(m)], v[E::y(m)], v[E::sx(m)], v[E::sy(m)]) : e[m];
+                    }
+                    part[(2 * i + side) * PIXP + k] = term(en, A, v[P - 1], pl);
+                }
+                v[i] = r[i];
+            }
+        }
+    }
+
+    // (normal: exps_normal holds at x)
+    __device__ __forceinline__ void gradient(const float *x, float *grad, bool normal) const {
         // parameter k: b before it is moved, lo / hi its two points, r after it is moved back
-        float b[P], lo[P], hi[P], r[P], sumA = 0.0f;
+        float b[P], lo[P], hi[P], r[P];
 #pragma unroll
         for (int k = 0; k < P; k++) {
             // (the first loss call, at parameter 0's lower point, clamps all the others)
@@ -1007,39 +1088,13 @@ struct LaneFit {
             hi[k] = bound(lo[k] + 0.004f);
             r[k] = bound(hi[k] - 0.002f);
         }
-#pragma unroll
-        for (int m = 0; m < E::M; m++) sumA += fmaxf(b[E::a(m)], fmaxf(hi[E::a(m)], r[E::a(m)]));
         float *part = s + L::PART;
-        if (safe(lo[P - 1], sumA) && safe(b[P - 1], sumA)) {
-#pragma unroll 1
-            for (int k = lane; k < PIX; k += G) {
-                const float2 c = make_float2(pos[k], pos[PIXP + k]), pl = make_float2(s[L::VAL + k], s[L::LOG + k]);
-                float v[P], e[E::M];
-#pragma unroll
-                for (int i = 0; i < P; i++) v[i] = b[i];
-#pragma unroll
-                for (int m = 0; m < E::M; m++) e[m] = 0.0f;
-#pragma unroll
-                for (int i = 0; i < P; i++) {
-                    float A[E::M], en[E::M];
-                    // emitters whose exponent the parameter before this one moved, or none is known yet
-#pragma unroll
-                    for (int m = 0; m < E::M; m++)
-                        if (!E::in(m, i) && (i == 0 || E::in(m, i - 1)))
-                            e[m] = expo(c.x, c.y, v[E::x(m)], v[E::y(m)], v[E::sx(m)], v[E::sy(m)]);
-#pragma unroll
-                    for (int side = 0; side < 2; side++) {
-                        v[i] = side ? hi[i] : lo[i];
-#pragma unroll
-                        for (int m = 0; m < E::M; m++) {
-                            A[m] = v[E::a(m)];
-                            en[m] = E::in(m, i) ? expo(c.x, c.y, v[E::x(m)], v[E::y(m)], v[E::sx(m)], v[E::sy(m)]) : e[m];
-                        }
-                        part[(2 * i + side) * PIXP + k] = term(en, A, v[P - 1], pl);
-                    }
-                    v[i] = r[i];
-                }
-            }
+        const float A = fmaxf(b[0], fmaxf(hi[0], r[0]));
+        if (safe(lo[P - 1], A) && safe(b[P - 1], A)) {
+            if (normal || exps_normal(b, b))  // (every point is within 0.0041 of b)
+                point_terms<false>(b, lo, hi, r, part);
+            else
+                point_terms<true>(b, lo, hi, r, part);
         } else {
 #pragma unroll 1
             for (int j = 0; j < NE; j++) {
@@ -1118,7 +1173,7 @@ struct LaneFit {
         static_assert(kBisections == 11 && P <= G, "one evaluation, then three rounds of three; one direction per lane");
         float grad[P], d[P];
         for (int e = lane; e < P * P; e += G) s[L::H + e] = e % (P + 1) == 0 ? 1.0f : 0.0f;
-        gradient(x, grad);
+        gradient(x, grad, false);
 #pragma unroll
         for (int k = 0; k < P; k++) d[k] = -grad[k];
 #pragma unroll 1
@@ -1129,6 +1184,16 @@ struct LaneFit {
             total = ((float)P) / total;
 #pragma unroll
             for (int k = 0; k < P; k++) d[k] = d[k] * total;
+            bool normal;  // along the whole line
+            {
+                float v[P], u[P];
+#pragma unroll
+                for (int k = 0; k < P; k++) {
+                    v[k] = x[k];
+                    u[k] = x[k] + d[k];
+                }
+                normal = exps_normal(v, u);
+            }
             float p0 = 0.00001f, p1 = 1.0f, f0 = 0.0f, f1 = 0.0f, f[KPTS];
             // one bisection step: the moved end takes the midpoint and its loss
             auto move = [&](float fm) {
@@ -1141,7 +1206,7 @@ struct LaneFit {
             };
             {
                 const float st[KPTS] = {0.0001f, 1.0f, (p0 + p1) * 0.5f, 0.0001f};
-                losses(x, d, st, f);
+                losses(x, d, st, normal, f);
                 f0 = f[0];
                 f1 = f[1];
                 move(f[2]);
@@ -1154,7 +1219,7 @@ struct LaneFit {
                 const float m2 = (q0 + q1) * 0.5f;
                 // the third midpoint: the lower half kept (upper end moved to m2), or the upper
                 const float st[KPTS] = {m1, m2, (q0 + m2) * 0.5f, (m2 + q1) * 0.5f};
-                losses(x, d, st, f);
+                losses(x, d, st, normal, f);
                 move(f[0]);
                 const bool lower = f0 < f1;
                 move(f[1]);
@@ -1178,7 +1243,7 @@ struct LaneFit {
                 float yk[P];
 #pragma unroll
                 for (int k = 0; k < P; k++) yk[k] = grad[k];
-                gradient(x, grad);
+                gradient(x, grad, normal);  // x is on the line, or raised to 0.01
 #pragma unroll
                 for (int k = 0; k < P; k++) yk[k] = grad[k] - yk[k];
                 update(sk, yk, grad, d);
