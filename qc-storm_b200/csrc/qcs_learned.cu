@@ -24,6 +24,7 @@
 
 #include "../../include/qcstorm_b200.h"
 #include "qcs_error.h"
+#include "qcs_gemm_plan.h"
 #include "qcs_kernels.h"
 #include "qcs_learned.h"
 #include "qcs_tc.cuh"
@@ -128,7 +129,7 @@ __global__ void targets_kernel(const uint16_t *__restrict__ rois, const float *_
 // 182 us, 143 with the weight gradients in one launch (layer_gradients), 133 with
 // whole chunks staged by constant steps (the loops' index arithmetic was half of
 // a product's instructions; convolutional network 2,292 -> 1,984 us).
-constexpr int kGemmM = 128, kGemmK = 128;
+constexpr int kGemmM = 128;
 
 // What a GEMM's result goes through before it is stored (only unsplit, beta
 // 0): C += bias per column, act = relu(C); or C = 0 where mask <= 0 (the
@@ -515,27 +516,6 @@ static GemmArgs gemm_args(int M, int N, int K, const float *A, long long sam, lo
     return g;
 }
 
-// Splits K over at most `most` CTAs a tile, at least 256 of K each, with their
-// partials in `ws`; the floats of it that they take.
-static size_t gemm_split(GemmArgs &g, int most, float *ws, size_t ws_floats) {
-    int s = most;
-    const int by_k = g.K / 256;
-    if (s > by_k) s = by_k;
-    if (s > 64) s = 64;
-    while (s > 1 && (size_t)s * g.M * g.N > ws_floats) --s;
-    if (s < 1) s = 1;
-    int kper = (g.K + s - 1) / s;
-    kper = ((kper + kGemmK - 1) / kGemmK) * kGemmK;
-    g.z = kper > 0 ? (g.K + kper - 1) / kper : 1;
-    if (g.z <= 1) {
-        g.z = 1;
-        return 0;
-    }
-    g.kper = kper;
-    g.part = ws;
-    return (size_t)g.z * g.M * g.N;
-}
-
 static cudaError_t gemm_attributes() {
     static bool set = false;
     if (set) return cudaSuccess;
@@ -556,7 +536,12 @@ static cudaError_t gemm_epilogue(int M, int N, int K, const float *A, long long 
     GemmArgs g = gemm_args(M, N, K > 0 ? K : 0, A, sam, sak, B, sbk, sbn, C, ldc, beta);
     g.ep = ep;
     // enough CTAs to cover the SMs
-    if (ws && !ep.bias && !ep.act && !ep.mask) gemm_split(g, 148 / (g.m_tiles() * g.n_tiles()), ws, ws_floats);
+    if (ws && !ep.bias && !ep.act && !ep.mask) {
+        const GemmSplit k = gemm_split(M, N, g.K, 148 / (g.m_tiles() * g.n_tiles()), ws_floats);
+        g.z = k.z;
+        g.kper = k.kper;
+        g.part = k.z > 1 ? ws : nullptr;
+    }
     cudaError_t e = gemm_attributes();
     if (e != cudaSuccess) return e;
     auto k = g.bn == 16 ? gemm_tc_kernel<16> : (g.bn == 32 ? gemm_tc_kernel<32> : (g.bn == 128 ? gemm_tc_kernel<128> : gemm_tc_kernel<0>));
@@ -588,13 +573,15 @@ static cudaError_t layer_gradients(const LayerGradient (&l)[kGemmBatch], int row
         b.column_sum[i] = l[i].db;
         tiles += b.g[i].m_tiles() * b.g[i].n_tiles();
     }
+    LayerSplit plan[kGemmBatch];
+    const int M[kGemmBatch] = {l[0].in, l[1].in, l[2].in}, N[kGemmBatch] = {l[0].cols, l[1].cols, l[2].cols};
+    if (!plan_layers(kGemmBatch, M, N, rows, 148 / tiles, ws_floats, plan)) return cudaErrorInvalidValue;
     for (int i = 0; i < kGemmBatch; ++i) {
         GemmArgs &g = b.g[i];
-        // room for the column sums of every layer's splits first
-        const size_t used = gemm_split(g, 148 / tiles, ws, ws_floats > (size_t)64 * g.N ? ws_floats - (size_t)64 * g.N : 0);
-        g.bsum = ws + used;
-        ws += used + (size_t)g.z * g.N;
-        ws_floats -= used + (size_t)g.z * g.N;
+        g.z = plan[i].split.z;
+        g.kper = plan[i].split.kper;
+        g.part = g.z > 1 ? ws + plan[i].part : nullptr;
+        g.bsum = ws + plan[i].sums;
         ctas += g.m_tiles() * g.n_tiles() * g.z;
         bn = bn > g.bn ? bn : g.bn;
         most = std::max(most, (long long)g.M * g.N + g.N);
