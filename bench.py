@@ -1474,9 +1474,10 @@ def consec_measure(stream, dist, world):
 
 
 def autotune_measure(stream, dist, world):
-    """The autotuner on small calls: qcs_loc_autotune's table for GS2D 7x7 and
-    the device time of 2,000-record calls (WLE pre-pass, fit, CRLB) with and
-    without it (the rows are identical)."""
+    """The autotuner on small calls: qcs_loc_autotune's table for GS2D 7x7 (8: by
+    the queue's length) and the device time of 2,000- and 20,000-record calls
+    (WLE pre-pass, fit, CRLB) with it, with one thread per ROI and by length (the
+    rows are identical)."""
     import torch
     from qcstorm_b200 import lib, synth
     rec, para, _ = synth.gs2d_rois(20_000, R=R, seed=99)
@@ -1489,7 +1490,7 @@ def autotune_measure(stream, dist, world):
     out = {"table": [{"records_up_to": a, "lanes_per_roi": b} for a, b in table]}
     for m in (2000, 20_000):
         res = {}
-        for name, tab in (("one_thread_per_roi", []), ("tuned", table)):
+        for name, tab in (("one_thread_per_roi", [(1 << 30, 1)]), ("by_length", []), ("tuned", table)):
             ctx.set_tuning(tab)
             for _ in range(3):
                 ctx.localize_device(d.data_ptr(), m, 0, sh)

@@ -452,27 +452,31 @@ int qcs_wle_estimate_device(qcs_loc_data *c, const uint16_t *d_rois, int n, cons
  * loc_type: QCS_LOCTYPE_*; rows: n x 12 in d_loc, CRLB columns left 0. */
 int qcs_fit_single_device(int loc_type, const qcs_loc_para *p, const uint16_t *d_rois, const float *d_wle, int n,
                           float *d_loc, void *stream);
-/* The fit of qcs_fit_single_device with `lanes` lanes per ROI (8; also 4 or
- * 16 for GS2D 7x7): the same rows bit for bit, with about half the latency
- * per ROI, for short batches.  ROI sizes: GS2D 7, 9, 11, 13 and AS3D 7, 9, 11
+/* The fit of qcs_fit_single_device with at least `lanes` lanes per ROI (8;
+ * also 4 or 16 for GS2D 7x7): the same rows bit for bit with a fraction of the
+ * latency per ROI, for short batches.  8 lanes (also for 4) at 7x7, 16 at the
+ * larger sizes, whose terms leave no room for narrower groups.  ROI sizes: GS2D 7, 9, 11, 13 and AS3D 7, 9, 11
  * (the sizes whose pixel-distance rounding is fixed in the source);
  * QCS_ERR_ARG otherwise. */
 int qcs_fit_single_group_device(int loc_type, const qcs_loc_para *p, const uint16_t *d_rois, const float *d_wle,
                                 int n, float *d_loc, int lanes, void *stream);
 /* Autotuner (no counterpart in the reference): times the single-emitter fit of
  * the first m records of d_rois / d_wle (device, WLE rows given) for m = 256,
- * 1,024, 4,096, ... up to n with one thread per ROI and with 8 lanes per ROI
- * (also 4 and 16 for GS2D 7x7), and keeps in the context, per batch size,
- * the fastest; qcs_loc_localize_device then fits a batch of n records with
- * the lanes of the first entry whose size is >= n (larger batches: one
- * thread per ROI).  Without a table it chooses by the queue's length: 32 or 16
- * lanes per ROI for short ones, one thread per ROI for long ones.  Every choice
+ * 1,024, 4,096, ... up to n with the default, a choice by the queue's length
+ * (32 or 16 lanes per ROI for short queues, one thread per ROI for long ones,
+ * lane groups beside it for a short rest), with one thread per ROI and, for
+ * GS2D 7x7, with 16 lanes per ROI, and keeps in the context, per batch size,
+ * the default unless another is at least 5% faster; qcs_loc_localize_device
+ * then fits a batch of n records as the first entry whose size is >= n says
+ * (larger batches, and every batch without a table: the default).  Every choice
  * gives the same rows bit for bit.  n >= 64 records; overwrites the context's
  * rows. */
 int qcs_loc_autotune(qcs_loc_data *c, const qcs_loc_para *p, const uint16_t *d_rois, const float *d_wle, int n,
                      void *stream);
 /* The tuning table (returns its length; sizes / lanes may be NULL), or sets it
- * (count 0..8 entries of (largest batch, lanes 1 / 4 / 8 / 16); 0 clears it). */
+ * (count 0..8 entries of (largest batch, lanes 1 / 4 / 8 / 16); 0 clears it).
+ * 8 stands for the choice by the queue's length, 1 for one thread per ROI; 4 and
+ * 16 are at least that many lanes at GS2D 7x7 and the same as 8 elsewhere. */
 int qcs_loc_tuning(const qcs_loc_data *c, int *sizes, int *lanes, int max_entries);
 int qcs_loc_set_tuning(qcs_loc_data *c, const int *sizes, const int *lanes, int count);
 /* With multi-emitter fitting, qcs_loc_autotune also times each multi-emitter
@@ -488,7 +492,9 @@ int qcs_loc_set_tuning_multi(qcs_loc_data *c, int limit_2e, int limit_3e);
  * multi-emitter limits) to a text file tagged with the GPU's name, ROI size,
  * localization type and multi-emitter setting; loading sets the context's
  * tuning from such a file and refuses (QCS_ERR_STATE) one written for another
- * GPU model or shape, so a caller tunes once per machine and reloads. */
+ * GPU model or shape, so a caller tunes once per machine and reloads.  A file of
+ * version 1 holds choices measured on kernels that no longer exist: it is read
+ * and leaves the context at its defaults. */
 int qcs_loc_save_tuning(const qcs_loc_data *c, const char *path);
 int qcs_loc_load_tuning(qcs_loc_data *c, const char *path);
 /* Model selection of multi-emitter calls (no counterpart in the reference,

@@ -84,8 +84,8 @@ struct qcs_loc_data {
     int *d_slots3 = nullptr, *d_ids3 = nullptr;
     int capture3 = 0;  // qcs_loc_set_three_emitter_capture
     const qcs::ThreeEmitterStart *three = nullptr;  // set for the duration of a learned call with a 3E net
-    // autotuned lanes per ROI of the single-emitter fit by batch size: batches of
-    // at most tune_n[k] records use tune_lanes[k] (first match), larger ones 1; an empty table: by queue length
+    // autotuned lanes per ROI of the single-emitter fit by batch size: batches of at most tune_n[k] records use
+    // tune_lanes[k] (first match; 8: by the queue's length); larger ones, and all with an empty table, by length
     int tune_count = 0;
     int tune_n[8] = {0};
     int tune_lanes[8] = {0};
@@ -315,10 +315,17 @@ static int ensure_three(qcs_loc_data *c) {
     return QCS_OK;
 }
 
-static int tuned_lanes(const qcs_loc_data *c, int n) {
+// CascadeArgs::lanes of a batch of n records.  8 in a table is the choice by the
+// queue's length, at every shape; more than one lane whatever the length exists
+// for GS2D 7x7 (4 and 16).
+static int tuned_lanes(const qcs_loc_data *c, const qcs_loc_para *p, int n) {
+    const bool gs7 = p->LocType != QCS_LOCTYPE_AS3D && p->ROISize == 7;
     for (int k = 0; k < c->tune_count; ++k)
-        if (n <= c->tune_n[k]) return c->tune_lanes[k];
-    return c->tune_count ? 1 : 0;  // longer than tuned: one thread per ROI; not tuned: by the queue's length
+        if (n <= c->tune_n[k]) {
+            const int lanes = c->tune_lanes[k];
+            return lanes == 1 || (gs7 && lanes != 8) ? lanes : 0;
+        }
+    return 0;
 }
 
 int qcs_loc_localize_device(qcs_loc_data *c, const uint16_t *d_rois, const float *d_wle, const qcs_loc_para *p,
@@ -340,7 +347,7 @@ int qcs_loc_localize_device(qcs_loc_data *c, const uint16_t *d_rois, const float
     a.loc = c->d_loc;
     a.max_rows = c->max_rows;
     a.stream = s;
-    a.lanes = tuned_lanes(c, n);
+    a.lanes = tuned_lanes(c, p, n);
     a.group_limit2 = c->tune_limit2;
     a.group_limit3 = c->tune_limit3;
     QCS_CUDA(run_localization(c, a), "localization cascade");
@@ -1233,6 +1240,8 @@ int qcs_fit_single_group_device(int loc_type, const qcs_loc_para *p, const uint1
     return QCS_OK;
 }
 
+static constexpr float kTuneMargin = 0.95f;
+
 int qcs_loc_autotune(qcs_loc_data *c, const qcs_loc_para *p, const uint16_t *d_rois, const float *d_wle, int n,
                      void *stream) {
     int st = check_call(c, p, n);
@@ -1248,11 +1257,12 @@ int qcs_loc_autotune(qcs_loc_data *c, const qcs_loc_para *p, const uint16_t *d_r
     const bool single_ok = qcs::group_fit_supported(kind, p->ROISize) && p->LocType != QCS_LOCTYPE_DH3D;
     const bool multi_ok = p->MultiEmitterFitEn && p->LocType != QCS_LOCTYPE_DH3D;
     if (!single_ok && !multi_ok) return QCS_OK;
-    // lanes per ROI to try: 1 (one thread per ROI) and 8; 4 and 16 exist for GS2D 7x7 only
-    const int cand7[4] = {1, 4, 8, 16}, cand_other[2] = {1, 8};
-    const bool gs7 = kind == qcs::kGS2D && p->ROISize == 7;
-    const int *cand = gs7 ? cand7 : cand_other;
-    const int ncand = gs7 ? 4 : 2;
+    // what to try: the choice by the queue's length (8), one thread per ROI (1), and for GS2D 7x7 16 lanes.  The
+    // first is the default; another is taken only where it is clearly faster (kTuneMargin), as an entry holds for
+    // every batch down to the next smaller one, whose lengths the default tells apart and the others do not
+    // (20,000 11x11 records: 328 us by length, 459 with one thread per ROI; 65,536: the same).
+    const int cand[3] = {8, 1, 16};
+    const int ncand = kind == qcs::kGS2D && p->ROISize == 7 ? 3 : 2;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     QCS_CUDA(cudaEventCreate(&e0), "tuning events");
     cudaError_t e = cudaEventCreate(&e1);
@@ -1266,6 +1276,7 @@ int qcs_loc_autotune(qcs_loc_data *c, const qcs_loc_para *p, const uint16_t *d_r
     f.mo = qcs::MultiOut{nullptr, nullptr};
     f.para = qcs::core_para(q);
     f.stream = s;
+    f.exact = !p->MultiEmitterFitEn;  // as the call that the entry is for
     int sizes[8], k = 0;
     if (single_ok) {
         for (int m = 256; m < n && k < 7; m *= 4) sizes[k++] = m;
@@ -1276,11 +1287,12 @@ int qcs_loc_autotune(qcs_loc_data *c, const qcs_loc_para *p, const uint16_t *d_r
         f.q = qcs::Queue{nullptr, nullptr, m};
         f.max_count = m;
         float best = 1e30f;
-        int best_lanes = 1;
+        int best_lanes = 8;
         for (int j = 0; j < ncand && e == cudaSuccess; ++j) {
             const int lanes = cand[j];
             auto run = [&]() {
-                return lanes == 1 ? qcs::launch_fit(kind, p->ROISize, f) : qcs::launch_fit_group(kind, p->ROISize, lanes, f);
+                return lanes == 1 ? qcs::launch_fit(kind, p->ROISize, f)
+                                  : qcs::launch_fit_group(kind, p->ROISize, lanes == 8 ? 0 : lanes, f);
             };
             e = run();  // warm-up
             if (e == cudaSuccess) e = cudaEventRecord(e0, s);
@@ -1289,12 +1301,12 @@ int qcs_loc_autotune(qcs_loc_data *c, const qcs_loc_para *p, const uint16_t *d_r
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);
             float ms = 0;
             if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-            if (e == cudaSuccess && ms < best) {
+            if (e == cudaSuccess && ms < (j == 0 ? best : best * kTuneMargin)) {
                 best = ms;
                 best_lanes = lanes;
             }
         }
-        c->tune_n[i] = m;  // batches above the largest tuned size keep one thread per ROI
+        c->tune_n[i] = m;
         c->tune_lanes[i] = best_lanes;
     }
     // Multi-emitter stages: the longest queue for which the lane-group kernel beats one thread per ROI,
@@ -1372,7 +1384,7 @@ int qcs_loc_save_tuning(const qcs_loc_data *c, const char *path) {
     if (!c || !path) return fail(QCS_ERR_ARG, "null argument");
     FILE *f = fopen(path, "w");
     if (!f) return fail(QCS_ERR_ARG, "cannot open the tuning file for writing");
-    fprintf(f, "qcstorm_b200_tuning 1\ngpu %s\nroi_size %d\nloc_type %d\nmulti %d\nlanes %d", gpu_tag().c_str(),
+    fprintf(f, "qcstorm_b200_tuning 2\ngpu %s\nroi_size %d\nloc_type %d\nmulti %d\nlanes %d", gpu_tag().c_str(),
             c->para.ROISize, c->para.LocType, c->para.MultiEmitterFitEn, c->tune_count);
     for (int i = 0; i < c->tune_count; ++i) fprintf(f, " %d %d", c->tune_n[i], c->tune_lanes[i]);
     fprintf(f, "\nlimits %d %d\n", c->tune_limit2, c->tune_limit3);
@@ -1388,7 +1400,7 @@ int qcs_loc_load_tuning(qcs_loc_data *c, const char *path) {
     int version = 0, R = 0, lt = 0, multi = 0, count = 0, sizes[8], lanes[8], l2 = 0, l3 = 0;
     bool ok = fscanf(f, " qcstorm_b200_tuning %d gpu %255s roi_size %d loc_type %d multi %d lanes %d", &version, gpu,
                      &R, &lt, &multi, &count) == 6 &&
-              version == 1 && count >= 0 && count <= 8;
+              (version == 1 || version == 2) && count >= 0 && count <= 8;
     for (int i = 0; ok && i < count; ++i) ok = fscanf(f, " %d %d", &sizes[i], &lanes[i]) == 2;
     ok = ok && fscanf(f, " limits %d %d", &l2, &l3) == 2;
     fclose(f);
@@ -1396,8 +1408,13 @@ int qcs_loc_load_tuning(qcs_loc_data *c, const char *path) {
     if (gpu_tag() != gpu || R != c->para.ROISize || lt != c->para.LocType || multi != c->para.MultiEmitterFitEn)
         return fail(QCS_ERR_STATE, "the tuning file was written for another GPU model or ROI shape");
     int st = qcs_loc_set_tuning(c, sizes, lanes, count);
+    if (!st) st = qcs_loc_set_tuning_multi(c, l2, l3);
     if (st) return st;
-    return qcs_loc_set_tuning_multi(c, l2, l3);
+    if (version == 1) {  // measured on kernels that are gone: the defaults are as good or better
+        c->tune_count = 0;
+        c->tune_limit2 = c->tune_limit3 = 0;
+    }
+    return QCS_OK;
 }
 
 int qcs_loc_tuning_multi(const qcs_loc_data *c, int *limit_2e, int *limit_3e) {

@@ -454,7 +454,7 @@ cudaError_t run_cascade(const CascadeArgs &a, const CascadeState &st) {
     FitLaunch f = cascade_single_launch(a, st);
     f.exact = !a.para.MultiEmitterFitEn && !a.n_dev;  // the queue is the call's n records
     if (a.lanes != 1 && group_fit_supported(kind, a.para.ROISize))
-        e = launch_fit_group(kind, a.para.ROISize, (kind == kGS2D && a.para.ROISize == 7) || a.lanes == 0 ? a.lanes : 8, f);
+        e = launch_fit_group(kind, a.para.ROISize, a.lanes, f);
     else
         e = launch_fit(kind, a.para.ROISize, f);
     if (e != cudaSuccess) return e;

@@ -82,7 +82,7 @@ struct CascadeArgs {
     int max_rows;
     cudaStream_t stream;
     const uint8_t *pred = nullptr;  // learned emitter-count class per record, or null (the reference's split)
-    // lanes per ROI of the single-emitter fit: 0 (by the queue's length), 1 (one thread per ROI) or 4 / 8 / 16
+    // lanes per ROI of the single-emitter fit: 0 (by the queue's length), 1 (one thread per ROI) or, GS2D 7x7, 4 / 16
     int lanes = 0;
     const TwoEmitterStart *two = nullptr;  // learned two-emitter starts (GS2D), or null (the reference's)
     const ThreeEmitterStart *three = nullptr;  // learned three-emitter starts (GS2D), or null (the reference's)
