@@ -739,13 +739,13 @@ __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
     return d;
 }
 
-// e^x = 2^(x log2 e) and ln x = log2(x) ln 2 through the flushing base-2
-// instructions: without the scaling around subnormal results and arguments
-// that __expf and __logf carry (about 6.7 of the 22.8 instructions the loss
-// issued per pixel).  Where the result of exp and the argument of log are
-// normal the values are those of __expf and __logf bit for bit (every float
-// was compared); a subnormal exp is 0 here.  The loss takes this form only
-// where that changes no sum (flush_safe).
+// e^x = 2^(x log2 e) and ln x = log2(x) ln 2 on the ex2 and lg2 instructions
+// that flush subnormals.  Where the result of exp and the argument of log are
+// normal the values are those of __expf and __logf bit for bit, and a subnormal
+// exp is 0 here (every float is compared in tests/test_gpu_evaluators.py).  They
+// take fewer issue slots, which bound the loss with __expf and __logf (85% of the
+// slots, 61% of the special-function pipe); the loss takes this form only where
+// that changes no sum (flush_safe).
 __device__ __forceinline__ float ex2_flush(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
