@@ -943,12 +943,12 @@ template <int R, int KIND, int DIST = ArithSpec<KIND, R>::DIST, int MASK = Arith
 __global__ void __launch_bounds__(kTPB) fit_multi_kernel(const uint16_t *__restrict__ rois,
                                                          const float *__restrict__ wle, Queue q,
                                                          float *__restrict__ loc, MultiOut mo, CorePara c,
-                                                         double *__restrict__ ll, int min_n) {
+                                                         double *__restrict__ ll, int min_n, int again) {
     typedef SmemLayout<R, KIND> L;
     enum { P = KindTraits<KIND>::P, PIX = R * R, WHOLE = R * (R + 1) };
     extern __shared__ float smem[];
     const int n = queue_len(q);
-    if (n <= min_n) return;  // a queue this short is the lane-group kernel's
+    if (n <= min_n || (n > kThreadWave && n <= again)) return;  // the lane-group kernel's (MultiLanes)
     const int base = blockIdx.x * kTPB;
     if (base >= n) return;
     const int cnt = min(kTPB, n - base);
@@ -990,8 +990,8 @@ __global__ void __launch_bounds__(kTPB) fit_multi_kernel(const uint16_t *__restr
 // For queues too short to fill the GPU with one thread per ROI, where that
 // launch lasts as long as one thread's whole fit.  Each group takes queue
 // entries g, g + groups, ... on its own (no block barrier after the table of
-// pixel centres); a queue outside min_n < n <= max_n (< 0: no bound) is
-// another launch's.
+// pixel centres); a queue outside min_n < n <= max_n (< 0: no bound) and
+// kThreadWave < n <= again is another launch's.
 template <int R, int KIND, int G>
 struct LaneShape {
     typedef LaneLayout<R, KIND> L;
@@ -1012,7 +1012,7 @@ template <int R, int KIND, int G, int DIST = ArithSpec<KIND, R>::DIST, int MASK 
           int SUM2 = ArithSpec<KIND, R>::SUM2>
 __global__ void __launch_bounds__(kGroupTPB, (LaneShape<R, KIND, G>::BLOCKS)) fit_lanes_kernel(
     const uint16_t *__restrict__ rois, const float *__restrict__ wle, Queue q, float *__restrict__ loc,
-    uint8_t *__restrict__ to2e, MultiOut mo, CorePara c, double *__restrict__ ll, int min_n, int max_n, int rest_most) {
+    uint8_t *__restrict__ to2e, MultiOut mo, CorePara c, double *__restrict__ ll, int min_n, int max_n, int again, int rest_most) {
     typedef LaneLayout<R, KIND> L;
     typedef LaneShape<R, KIND, G> S;
     constexpr bool MULTI = Emitters<KIND>::M > 1;
@@ -1020,7 +1020,7 @@ __global__ void __launch_bounds__(kGroupTPB, (LaneShape<R, KIND, G>::BLOCKS)) fi
     static_assert(DIST != kCompiler && (!MULTI || SUM2 == kFuseFirst), "roundings fixed in the source");
     extern __shared__ __align__(16) float smem[];
     const int n = queue_len(q);
-    const bool whole = n > min_n && (max_n < 0 || n <= max_n);
+    const bool whole = n > min_n && (max_n < 0 || n <= max_n || (n > kThreadWave && n <= again));
     const int rest = whole ? n : queue_rest<R, KIND>(n, rest_most);
     // beside the one-thread kernel of the queue's other entries: ends after it
     // does, so that what follows on the stream finds its rows
@@ -1460,17 +1460,17 @@ cudaError_t launch_single(const FitLaunch &a, int min_n = -1, int rest_most = 0)
     return cudaGetLastError();
 }
 
-// Queues of min_n < n <= max_n (< 0: any length) entries with G lanes per ROI,
-// and the rest of longer ones (queue_rest; rest_most > 0: launched right after
-// the one-thread kernel, and runs beside it).
+// Queues of min_n < n <= max_n (< 0: any length) entries, and of kThreadWave < n
+// <= again, with G lanes per ROI, and the rest of longer ones (queue_rest;
+// rest_most > 0: launched right after the one-thread kernel, and runs beside it).
 template <int R, int KIND, int G>
-cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n, int rest_most = 0) {
+cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n, int rest_most = 0, int again = 0) {
     typedef LaneShape<R, KIND, G> S;
     const size_t smem = S::FLOATS * sizeof(float);
     auto k = fit_lanes_kernel<R, KIND, G>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int longest = max_n >= 0 && max_n < rest_most ? rest_most : max_n;
+    const int longest = max_n < 0 ? -1 : max(max_n, max(rest_most, again));
     const long long most = longest >= 0 && longest < a.max_count ? longest : a.max_count;
     const long long need = (most + S::SLOTS - 1) / S::SLOTS;
     const int grid = (int)(need < 148 * S::BLOCKS ? need : 148 * S::BLOCKS);
@@ -1485,7 +1485,7 @@ cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n, int rest_most
     cfg.stream = a.stream;
     cfg.attrs = &beside;
     cfg.numAttrs = rest_most > 0 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, a.rois, a.wle, a.q, a.loc, a.to2e, a.mo, a.para, a.ll, min_n, max_n, rest_most);
+    return cudaLaunchKernelEx(&cfg, k, a.rois, a.wle, a.q, a.loc, a.to2e, a.mo, a.para, a.ll, min_n, max_n, again, rest_most);
 }
 
 // The ROIs that G lanes each fit at once on the whole GPU.
@@ -1527,18 +1527,33 @@ cudaError_t launch_by_length(const FitLaunch &a) {
     return e;
 }
 
-// Longest multi-emitter queue that lane groups fit by default: the two- and
-// three-emitter stages of 100,000 1-3 emitter records of 7x7 (27,300 and 6,600
-// ROIs) take as long with lane groups as with one thread per ROI, shorter
-// queues and 11x11 ROIs up to ten times less (1,000 records of 7x7: the whole
-// call 257 us against 1,493 us; 20,000: 611 against 1,649; 11x11: 244 against
-// 1,156 and 808 against 3,396).
-constexpr int kGroupQueueLimit = 30000;
+// Multi-emitter queues that lane groups fit by default: up to `most`, and from
+// kThreadWave + 1 to `again`.  Lane groups take a time that grows with the
+// queue, one thread per ROI the same for any queue up to 18,944 ROIs and about
+// half as long again (11x11: twice as long) for one more, so the two cross
+// twice.  Stages of triplet records, lane groups' time less the other's, us:
+//   2E 7x7     11,000 -25   12,500 +42   18,944 +221  18,945 -17    21,000 +31
+//   3E 7x7     11,000 -152  14,000 +7    18,944 +319  18,945 -146   22,000 +131
+//   2E 11x11   11,000 -93   13,000 +40   18,944 +481  18,945 -482   26,000 +29
+//   3E 11x11   11,000 -577  17,000 +7    18,944 +248  18,945 -1,496 30,000 -220
+//   AS3D-2E    11,000 -177  16,000 +39   18,944 +204  18,945 -55    21,000 +56
+// (1,000 ROIs: -392, -801, -872, -1,702, -678; whole calls of 7x7 triplets with
+// one thread per ROI: 1,472 at 1,000, 1,646 at 18,944, 2,319 at 18,945).
+template <int KIND, int R>
+struct MultiLanes;
+template <> struct MultiLanes<k2E, 7> { enum { most = 12000, again = 0 }; };
+template <> struct MultiLanes<k3E, 7> { enum { most = 13500, again = 20500 }; };
+template <> struct MultiLanes<k2E, 11> { enum { most = 12500, again = 25000 }; };
+template <> struct MultiLanes<k3E, 11> { enum { most = 16500, again = 30000 }; };
+template <> struct MultiLanes<kAS3D2E, 7> { enum { most = 15000, again = 20000 }; };
 
 }  // namespace
 
 int multi_group_default_limit(int kind, int R) {
-    return multi_group_supported(kind, R) ? kGroupQueueLimit : 0;
+    if (kind == kAS3D2E) return R == 7 ? MultiLanes<kAS3D2E, 7>::most : 0;
+    if (kind == k2E) return R == 7 ? MultiLanes<k2E, 7>::most : (R == 11 ? MultiLanes<k2E, 11>::most : 0);
+    if (kind == k3E) return R == 7 ? MultiLanes<k3E, 7>::most : (R == 11 ? MultiLanes<k3E, 11>::most : 0);
+    return 0;
 }
 
 bool multi_group_available(int kind, int R) { return multi_group_supported(kind, R); }
@@ -1549,18 +1564,20 @@ namespace {
 // device and only one of them fits it (no host synchronisation).
 template <int R, int KIND>
 cudaError_t launch_multi(const FitLaunch &a) {
-    int min_n = -1;
+    int min_n = -1, again = 0;
     cudaError_t e;
     if constexpr (multi_group_supported(KIND, R)) {
         if (!a.thread_per_roi) {
             // group_limit > 0: tuned; < 0: one thread per ROI always; 0: the default
-            min_n = a.group_limit > 0 ? a.group_limit : (a.group_limit < 0 ? -1 : kGroupQueueLimit);
+            min_n = a.group_limit > 0 ? a.group_limit : (a.group_limit < 0 ? -1 : (int)MultiLanes<KIND, R>::most);
+            again = a.group_limit == 0 ? (int)MultiLanes<KIND, R>::again : 0;
             // a warp per ROI; at 7x7 half a warp beyond one wave of those (the sums, which every lane of a
             // group repeats, are then shared by two ROIs); at 11x11 half the warps' shared memory would not fit
             const int wave = R == 7 ? min(min_n, kLaneWave<R, KIND, 32>) : min_n;
-            if (min_n > 0 && (e = launch_lanes<R, KIND, 32>(a, -1, wave)) != cudaSuccess) return e;
+            if (min_n > 0 && (e = launch_lanes<R, KIND, 32>(a, -1, wave, 0, R == 7 ? 0 : again)) != cudaSuccess) return e;
             if constexpr (R == 7)
-                if (min_n > wave && a.max_count > wave && (e = launch_lanes<R, KIND, 16>(a, wave, min_n)) != cudaSuccess)
+                if (min_n > wave && a.max_count > wave &&
+                    (e = launch_lanes<R, KIND, 16>(a, wave, min_n, 0, again)) != cudaSuccess)
                     return e;
             if (a.max_count <= min_n) return cudaSuccess;  // the queue cannot outgrow the group kernel
         }
@@ -1571,7 +1588,7 @@ cudaError_t launch_multi(const FitLaunch &a) {
     if (e != cudaSuccess) return e;
     const int grid = (a.max_count + kTPB - 1) / kTPB;
     if (grid == 0) return cudaSuccess;
-    k<<<grid, kTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.mo, a.para, a.ll, min_n);
+    k<<<grid, kTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.mo, a.para, a.ll, min_n, again);
     return cudaGetLastError();
 }
 

@@ -1,8 +1,9 @@
 """Two- and three-emitter stages at the lengths where their kernel changes.
 
 Up to one wave of warps (2,368 ROIs at four blocks an SM) a stage's queue takes a
-warp per ROI, up to 30,000 half a warp at 7x7 and further rounds of warps at
-11x11, beyond that one thread per ROI.  Every record here is one that reaches the
+warp per ROI, then half a warp at 7x7 and further rounds of warps at 11x11 up to
+12,000 to 16,500 ROIs, then one thread per ROI, with lane groups again for some
+lengths above its wave of 18,944.  Every record here is one that reaches the
 stage, so that the queue's length is the call's; the fit ratios say so.  All must
 give the one-thread rows, second emitters among them, bit for bit (NaN as NaN).
 """
@@ -13,6 +14,7 @@ import pytest
 
 from qcstorm_b200 import lib as qlib
 from qcstorm_b200 import synth
+from test_gpu_autotune_default import call_us
 from test_gpu_lanes_fit import device
 
 pytestmark = pytest.mark.gpu
@@ -47,7 +49,7 @@ def reaching(loc_type, R):
 
 
 @pytest.mark.parametrize("loc_type,R", [(0, 7), (0, 11), (1, 7)])
-@pytest.mark.parametrize("n", [2368, 2369, 4737, 30000, 30001])
+@pytest.mark.parametrize("n", [2368, 2369, 4737, 12000, 12001, 13501, 16501, 18944, 18945, 20001, 25000, 30001])
 def test_stage_lengths(cuda_ok, loc_type, R, n):
     base, para = reaching(loc_type, R)
     rec = np.resize(base, (n, base.shape[1]))
@@ -66,3 +68,23 @@ def test_stage_lengths(cuda_ok, loc_type, R, n):
         ctx.close()
     np.testing.assert_array_equal(out[0], out[2])
     np.testing.assert_array_equal(out[1], out[2])
+
+
+@pytest.mark.parametrize("loc_type,R", [(0, 7), (0, 11), (1, 7)])
+@pytest.mark.parametrize("n", [1000, 11000, 18000, 18950, 27000])
+def test_default_is_no_slower_than_either_kernel(cuda_ok, loc_type, R, n):
+    """The default against each kernel for the whole queue: wrong by at most a tenth of the call."""
+    import torch
+    base, para = reaching(loc_type, R)
+    rec = np.resize(base, (n, base.shape[1]))
+    rec[:, R * R + 2], rec[:, R * R + 3] = np.arange(n) & 0xFFFF, np.arange(n) >> 16
+    d = device(rec)
+    ctx = qlib.LocContext(para, n)
+    wle = torch.from_numpy(ctx.wle(rec)).cuda()
+    torch.cuda.synchronize()
+    us = []
+    for limit in (0, 1 << 30, -1):
+        ctx.set_tuning_multi(limit, limit)
+        us.append(call_us(ctx, d, wle, n))
+    ctx.close()
+    assert us[0] < 1.1 * min(us[1:])
