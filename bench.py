@@ -22,7 +22,9 @@ inside the timed region; `e2e.sync_value`: the synchronous
 qcs_loc_bfgs_mle_localization, one call at a time); `roofline` is the fit kernel against the measured
 special-function-unit rate (the loss is exp/log bound, not HBM or tensor
 bound); `cpu_baseline` is the reference's own code compiled for the host
-(oracle/_ref) on all host cores.
+(oracle/_ref) on all host cores; `parts` holds a few figures of the other
+measurements, which are printed in full on stderr (a line of 24 kB is cut by
+some readers).
 
 --impl reference times the reference's CPU implementation of the same step
 (oracle/_ref/libqcs_ref_host.so: the reference sources compiled for the CPU,
@@ -763,7 +765,8 @@ def learned_measure(args, streams, ctxs, para, d_batches, h_batches, rec0, truth
         "autotuned_schedule": {"iters": tuned_schedule[0], "bisections": tuned_schedule[1],
                                "rule": "qcs_learned_autotune: fastest schedule with acceptance within 0.5 points of "
                                        "the best"},
-        # mlp_tc (features + network), WLE (5), fit_learned, flag_queue, group refit, refit CRLB, counters, CRLB
+        # mlp_tc (features + network), WLE (3), fit_learned, flag_queue, refits (by length: three launches, two of
+        # them return at once), refit CRLB, counters, CRLB
         "gpu_launches_per_step": 12,
         "e2e": {"value": e2e_steps * N_PER_STEP * world / e2e_s, "unit": UNIT,
                 "h2d_bytes_per_step": N_PER_STEP * R * (R + 1) * 2,
@@ -1473,6 +1476,46 @@ def consec_measure(stream, dist, world):
             "call": "qcs_consec_fit_device (link by sorted (frame, y) search, merge, remove, CRLB)"}
 
 
+# Figures of the line's parts that are printed with the headline.
+SUMMARY = ["value_one_stream", "learned_other_configs.as3d.plain_fits_per_s", "learned_other_configs.as3d.learned_fits_per_s",
+           "learned_other_configs.multi.plain_fits_per_s", "learned_other_configs.multi.learned_fits_per_s",
+           "learned_other_configs.multi.lr_selection.fits_per_s", "learned_mixed_7_9_11.plain_fits_per_s",
+           "learned_mixed_7_9_11.learned_fits_per_s", "consecutive_fit.rows_per_s", "consecutive_fit.statistics.rows_per_s",
+           "autotune.call_2000_records.tuned_ms", "autotune.call_2000_records.one_thread_per_roi_ms",
+           "frames.frames_per_s", "frames.e2e.frames_per_s", "frames.graph.frames_per_s", "frames.learned.frames_per_s",
+           "frames.learned_multi_starts.frames_per_s", "frames.cpu_baseline.value"]
+
+
+def summary(line):
+    """The SUMMARY figures of the line that are there (a part may be switched off)."""
+    out = {}
+    for path in SUMMARY:
+        v = line
+        for k in path.split("."):
+            v = v.get(k) if isinstance(v, dict) else None
+        if v is not None:
+            out[path] = v
+    return out
+
+
+# Keys of the printed line, beside the figures of SUMMARY.
+HEAD = ["metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+        "vs_baseline", "dtype", "data", "learned_value", "learned_vs_plain", "learned_e2e_value",
+        "learned_rmse_px", "plain_rmse_px", "learned_rmse_px_own", "plain_rmse_px_own", "learned_accept",
+        "plain_accept", "learned_equal_rmse", "crlb_px", "fisher_crlb_px", "plain_rmse_over_fisher_crlb",
+        "learned_rmse_over_fisher_crlb", "learned_equal_rmse_within_2pct_of_crlb", "learned_no_refit_value",
+        "learned_no_refit_vs_plain", "learned_no_refit_rmse_px", "learned_no_refit_accept", "learned_conv_value",
+        "learned_conv_vs_plain", "learned_conv_rmse_px", "gpu_launches", "windows",
+        "clocks", "roofline",
+        "e2e", "cpu_baseline", "config"]
+
+
+def printed(line):
+    """(the one line on stdout, the parts in full for stderr), as JSON."""
+    return (json.dumps({**{k: line[k] for k in HEAD if k in line}, "parts": summary(line)}),
+            json.dumps({k: v for k, v in line.items() if k not in HEAD}))
+
+
 def autotune_measure(stream, dist, world):
     """The autotuner on small calls: qcs_loc_autotune's table for GS2D 7x7 (8: by
     the queue's length) and the device time of 2,000- and 20,000-record calls
@@ -1802,9 +1845,9 @@ def main():
     def step(k, s, c=None):
         (c or ctxs[k % IN_FLIGHT]).localize_device(d_batches[k % BATCHES].data_ptr(), N_PER_STEP, 0, s.cuda_stream)
 
-    # psf_width, nn_keys_flag, the sort's condition kernel (the sort itself only for out-of-order records),
-    # nn_scan_select, classify, init_counters, fit, finish, crlb
-    launches_per_step = 9
+    # widths_keys, the sort's condition kernel (the sort itself only for out-of-order records), nn_scan_select,
+    # init_counters, fit (100,000 records: no rest beside it), crlb
+    launches_per_step = 6
 
     # ---- device-timed steps: IN_FLIGHT contexts in turn on their streams
     sampler, spath = start_clock_sampler(local)
@@ -1950,18 +1993,9 @@ def main():
                 "learned_conv_value": learned["conv"]["value"], "learned_conv_vs_plain": learned["conv"]["vs_plain"],
                 "learned_conv_rmse_px": learned["conv"]["accuracy"]["rmse_px"]["conv"],
             })
-        # short keys first: the headline survives a truncated tail of the line
-        head = ["metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
-                "vs_baseline", "dtype", "data", "learned_value", "learned_vs_plain", "learned_e2e_value",
-                "learned_rmse_px", "plain_rmse_px", "learned_rmse_px_own", "plain_rmse_px_own", "learned_accept",
-                "plain_accept", "learned_equal_rmse", "crlb_px", "fisher_crlb_px", "plain_rmse_over_fisher_crlb",
-                "learned_rmse_over_fisher_crlb", "learned_equal_rmse_within_2pct_of_crlb", "learned_no_refit_value",
-                "learned_no_refit_vs_plain", "learned_no_refit_rmse_px", "learned_no_refit_accept", "learned_conv_value",
-                "learned_conv_vs_plain", "learned_conv_rmse_px", "gpu_launches", "windows",
-                "clocks", "roofline",
-                "e2e", "cpu_baseline", "config"]
-        line = {**{k: line[k] for k in head if k in line}, **{k: v for k, v in line.items() if k not in head}}
-        print(json.dumps(line), flush=True)
+        headline, parts = printed(line)
+        print(parts, file=sys.stderr, flush=True)
+        print(headline, flush=True)
     for c in ctxs:
         c.close()
     if dist:
