@@ -485,8 +485,8 @@ int qcs_loc_set_tuning(qcs_loc_data *c, const int *sizes, const int *lanes, int 
  * and keeps the longest queue for which the lane groups are faster: a stage
  * whose queue (read on the device) is at most that long uses them.  The
  * limits (-1: one thread per ROI always; 0: the built-in default, 12,000 to
- * 16,500 by stage and ROI size and again for queues a little above 18,944), read
- * or set here.  The rows are the same either way. */
+ * 16,500 by stage and ROI size and again for queues a little above one thread per
+ * ROI's wave), read or set here.  The rows are the same either way. */
 int qcs_loc_tuning_multi(const qcs_loc_data *c, int *limit_2e, int *limit_3e);
 int qcs_loc_set_tuning_multi(qcs_loc_data *c, int limit_2e, int limit_3e);
 /* Per-GPU tuning cache: writes the context's tuning (lanes table and

@@ -943,12 +943,12 @@ template <int R, int KIND, int DIST = ArithSpec<KIND, R>::DIST, int MASK = Arith
 __global__ void __launch_bounds__(kTPB) fit_multi_kernel(const uint16_t *__restrict__ rois,
                                                          const float *__restrict__ wle, Queue q,
                                                          float *__restrict__ loc, MultiOut mo, CorePara c,
-                                                         double *__restrict__ ll, int min_n, int again) {
+                                                         double *__restrict__ ll, int min_n, int from, int again) {
     typedef SmemLayout<R, KIND> L;
     enum { P = KindTraits<KIND>::P, PIX = R * R, WHOLE = R * (R + 1) };
     extern __shared__ float smem[];
     const int n = queue_len(q);
-    if (n <= min_n || (n > kThreadWave && n <= again)) return;  // the lane-group kernel's (MultiLanes)
+    if (n <= min_n || (n > from && n <= again)) return;  // the lane-group kernel's (MultiLanes)
     const int base = blockIdx.x * kTPB;
     if (base >= n) return;
     const int cnt = min(kTPB, n - base);
@@ -991,7 +991,7 @@ __global__ void __launch_bounds__(kTPB) fit_multi_kernel(const uint16_t *__restr
 // launch lasts as long as one thread's whole fit.  Each group takes queue
 // entries g, g + groups, ... on its own (no block barrier after the table of
 // pixel centres); a queue outside min_n < n <= max_n (< 0: no bound) and
-// kThreadWave < n <= again is another launch's.
+// from < n <= again is another launch's.
 template <int R, int KIND, int G>
 struct LaneShape {
     typedef LaneLayout<R, KIND> L;
@@ -1012,7 +1012,8 @@ template <int R, int KIND, int G, int DIST = ArithSpec<KIND, R>::DIST, int MASK 
           int SUM2 = ArithSpec<KIND, R>::SUM2>
 __global__ void __launch_bounds__(kGroupTPB, (LaneShape<R, KIND, G>::BLOCKS)) fit_lanes_kernel(
     const uint16_t *__restrict__ rois, const float *__restrict__ wle, Queue q, float *__restrict__ loc,
-    uint8_t *__restrict__ to2e, MultiOut mo, CorePara c, double *__restrict__ ll, int min_n, int max_n, int again, int rest_most) {
+    uint8_t *__restrict__ to2e, MultiOut mo, CorePara c, double *__restrict__ ll, int min_n, int max_n, int from, int again,
+    int rest_most) {
     typedef LaneLayout<R, KIND> L;
     typedef LaneShape<R, KIND, G> S;
     constexpr bool MULTI = Emitters<KIND>::M > 1;
@@ -1020,7 +1021,7 @@ __global__ void __launch_bounds__(kGroupTPB, (LaneShape<R, KIND, G>::BLOCKS)) fi
     static_assert(DIST != kCompiler && (!MULTI || SUM2 == kFuseFirst), "roundings fixed in the source");
     extern __shared__ __align__(16) float smem[];
     const int n = queue_len(q);
-    const bool whole = n > min_n && (max_n < 0 || n <= max_n || (n > kThreadWave && n <= again));
+    const bool whole = n > min_n && (max_n < 0 || n <= max_n || (n > from && n <= again));
     const int rest = whole ? n : queue_rest<R, KIND>(n, rest_most);
     // beside the one-thread kernel of the queue's other entries: ends after it
     // does, so that what follows on the stream finds its rows
@@ -1460,11 +1461,11 @@ cudaError_t launch_single(const FitLaunch &a, int min_n = -1, int rest_most = 0)
     return cudaGetLastError();
 }
 
-// Queues of min_n < n <= max_n (< 0: any length) entries, and of kThreadWave < n
-// <= again, with G lanes per ROI, and the rest of longer ones (queue_rest;
+// Queues of min_n < n <= max_n (< 0: any length) entries, and of from < n <=
+// again, with G lanes per ROI, and the rest of longer ones (queue_rest;
 // rest_most > 0: launched right after the one-thread kernel, and runs beside it).
 template <int R, int KIND, int G>
-cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n, int rest_most = 0, int again = 0) {
+cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n, int rest_most = 0, int from = 0, int again = 0) {
     typedef LaneShape<R, KIND, G> S;
     const size_t smem = S::FLOATS * sizeof(float);
     auto k = fit_lanes_kernel<R, KIND, G>;
@@ -1485,7 +1486,8 @@ cudaError_t launch_lanes(const FitLaunch &a, int min_n, int max_n, int rest_most
     cfg.stream = a.stream;
     cfg.attrs = &beside;
     cfg.numAttrs = rest_most > 0 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, a.rois, a.wle, a.q, a.loc, a.to2e, a.mo, a.para, a.ll, min_n, max_n, again, rest_most);
+    return cudaLaunchKernelEx(&cfg, k, a.rois, a.wle, a.q, a.loc, a.to2e, a.mo, a.para, a.ll, min_n, max_n, from, again,
+                              rest_most);
 }
 
 // The ROIs that G lanes each fit at once on the whole GPU.
@@ -1527,11 +1529,11 @@ cudaError_t launch_by_length(const FitLaunch &a) {
     return e;
 }
 
-// Multi-emitter queues that lane groups fit by default: up to `most`, and from
-// kThreadWave + 1 to `again`.  Lane groups take a time that grows with the
-// queue, one thread per ROI the same for any queue up to 18,944 ROIs and about
-// half as long again (11x11: twice as long) for one more, so the two cross
-// twice.  Stages of triplet records, lane groups' time less the other's, us:
+// Multi-emitter queues that lane groups fit by default: up to `most`, and past
+// thread_wave up to `again`.  Lane groups take a time that grows with the queue,
+// one thread per ROI the same for any queue up to its wave and about half as long
+// again (11x11: twice as long) for one more, so the two cross twice.  Stages of
+// triplet records, lane groups' time less the other's, us:
 //   2E 7x7     11,000 -25   12,500 +42   18,944 +221  18,945 -17    21,000 +31
 //   3E 7x7     11,000 -152  14,000 +7    18,944 +319  18,945 -146   22,000 +131
 //   2E 11x11   11,000 -93   13,000 +40   18,944 +481  18,945 -482   26,000 +29
@@ -1541,11 +1543,20 @@ cudaError_t launch_by_length(const FitLaunch &a) {
 // one thread per ROI: 1,472 at 1,000, 1,646 at 18,944, 2,319 at 18,945).
 template <int KIND, int R>
 struct MultiLanes;
-template <> struct MultiLanes<k2E, 7> { enum { most = 12000, again = 0 }; };
+template <> struct MultiLanes<k2E, 7> { enum { most = 12000, again = 20500 }; };
 template <> struct MultiLanes<k3E, 7> { enum { most = 13500, again = 20500 }; };
 template <> struct MultiLanes<k2E, 11> { enum { most = 12500, again = 25000 }; };
 template <> struct MultiLanes<k3E, 11> { enum { most = 16500, again = 30000 }; };
 template <> struct MultiLanes<kAS3D2E, 7> { enum { most = 15000, again = 20000 }; };
+
+// Longest queue that fit_multi_kernel fits in one wave, launched for max_count
+// ROIs.  A grid of more than three blocks an SM is packed deeper on fewer SMs at
+// 7x7, where four fit: 16,000 triplets take 1,629 us in a grid for 25,000 and
+// 2,325 in one for 30,000, as long as 19,000 (15,000: 1,624 in either).
+template <int R>
+constexpr int thread_wave(int max_count) {
+    return R == 7 && max_count > 148 * 3 * kTPB ? 15000 : kThreadWave;
+}
 
 }  // namespace
 
@@ -1564,6 +1575,7 @@ namespace {
 // device and only one of them fits it (no host synchronisation).
 template <int R, int KIND>
 cudaError_t launch_multi(const FitLaunch &a) {
+    const int from = thread_wave<R>(a.max_count);
     int min_n = -1, again = 0;
     cudaError_t e;
     if constexpr (multi_group_supported(KIND, R)) {
@@ -1574,10 +1586,11 @@ cudaError_t launch_multi(const FitLaunch &a) {
             // a warp per ROI; at 7x7 half a warp beyond one wave of those (the sums, which every lane of a
             // group repeats, are then shared by two ROIs); at 11x11 half the warps' shared memory would not fit
             const int wave = R == 7 ? min(min_n, kLaneWave<R, KIND, 32>) : min_n;
-            if (min_n > 0 && (e = launch_lanes<R, KIND, 32>(a, -1, wave, 0, R == 7 ? 0 : again)) != cudaSuccess) return e;
+            if (min_n > 0 && (e = launch_lanes<R, KIND, 32>(a, -1, wave, 0, from, R == 7 ? 0 : again)) != cudaSuccess)
+                return e;
             if constexpr (R == 7)
                 if (min_n > wave && a.max_count > wave &&
-                    (e = launch_lanes<R, KIND, 16>(a, wave, min_n, 0, again)) != cudaSuccess)
+                    (e = launch_lanes<R, KIND, 16>(a, wave, min_n, 0, from, again)) != cudaSuccess)
                     return e;
             if (a.max_count <= min_n) return cudaSuccess;  // the queue cannot outgrow the group kernel
         }
@@ -1588,7 +1601,7 @@ cudaError_t launch_multi(const FitLaunch &a) {
     if (e != cudaSuccess) return e;
     const int grid = (a.max_count + kTPB - 1) / kTPB;
     if (grid == 0) return cudaSuccess;
-    k<<<grid, kTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.mo, a.para, a.ll, min_n, again);
+    k<<<grid, kTPB, smem, a.stream>>>(a.rois, a.wle, a.q, a.loc, a.mo, a.para, a.ll, min_n, from, again);
     return cudaGetLastError();
 }
 

@@ -14,8 +14,9 @@ from test_gpu_lanes_fit import device
 pytestmark = pytest.mark.gpu
 
 
-def call_us(ctx, d, wle, n):
-    """Device time of one localization of n records: the least of ten runs of ten."""
+def call_us(ctx, d, wle, n, counted=None):
+    """Device time of one localization of n records (counted: the count on the device and its bound): the least
+    of ten runs of ten."""
     import torch
     s = torch.cuda.Stream()
     best = float("inf")
@@ -23,7 +24,10 @@ def call_us(ctx, d, wle, n):
         a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
         a.record(s)
         for _ in range(10):
-            ctx.localize_device(d.data_ptr(), n, wle.data_ptr(), s.cuda_stream)
+            if counted:
+                ctx.localize_device_n(d.data_ptr(), wle.data_ptr(), counted[0].data_ptr(), counted[1], s.cuda_stream)
+            else:
+                ctx.localize_device(d.data_ptr(), n, wle.data_ptr(), s.cuda_stream)
         b.record(s)
         b.synchronize()
         best = min(best, a.elapsed_time(b) * 100)

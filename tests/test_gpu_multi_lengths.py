@@ -3,7 +3,7 @@
 Up to one wave of warps (2,368 ROIs at four blocks an SM) a stage's queue takes a
 warp per ROI, then half a warp at 7x7 and further rounds of warps at 11x11 up to
 12,000 to 16,500 ROIs, then one thread per ROI, with lane groups again for some
-lengths above its wave of 18,944.  Every record here is one that reaches the
+lengths above its wave (18,944; 15,000 at 7x7 in a launch for many more).  Every record here is one that reaches the
 stage, so that the queue's length is the call's; the fit ratios say so.  All must
 give the one-thread rows, second emitters among them, bit for bit (NaN as NaN).
 """
@@ -71,20 +71,26 @@ def test_stage_lengths(cuda_ok, loc_type, R, n):
 
 
 @pytest.mark.parametrize("loc_type,R", [(0, 7), (0, 11), (1, 7)])
-@pytest.mark.parametrize("n", [1000, 11000, 18000, 18950, 27000])
-def test_default_is_no_slower_than_either_kernel(cuda_ok, loc_type, R, n):
-    """The default against each kernel for the whole queue: wrong by at most a tenth of the call."""
+@pytest.mark.parametrize("n,most", [(n, n) for n in (1000, 11000, 18000, 18950, 27000)] + [
+    (n, 60000) for n in (14500, 16000, 20400, 27000)])
+def test_default_is_no_slower_than_either_kernel(cuda_ok, loc_type, R, n, most):
+    """The default against each kernel for the whole queue: wrong by at most a tenth of the call.  most: the
+    call's bound, its count on the device where that is above n; the rows are those of one thread per ROI."""
     import torch
     base, para = reaching(loc_type, R)
     rec = np.resize(base, (n, base.shape[1]))
     rec[:, R * R + 2], rec[:, R * R + 3] = np.arange(n) & 0xFFFF, np.arange(n) >> 16
     d = device(rec)
-    ctx = qlib.LocContext(para, n)
+    ctx = qlib.LocContext(para, most)
     wle = torch.from_numpy(ctx.wle(rec)).cuda()
+    count = torch.tensor([n], dtype=torch.int32, device="cuda")
     torch.cuda.synchronize()
-    us = []
+    us, rows = [], []
     for limit in (0, 1 << 30, -1):
         ctx.set_tuning_multi(limit, limit)
-        us.append(call_us(ctx, d, wle, n))
+        us.append(call_us(ctx, d, wle, n, None if most == n else (count, most)))
+        rows.append(ctx.read_rows()[0])
     ctx.close()
+    np.testing.assert_array_equal(rows[0], rows[2])
+    np.testing.assert_array_equal(rows[1], rows[2])
     assert us[0] < 1.1 * min(us[1:])
