@@ -30,7 +30,7 @@ N = 1024  # cases of a class
 
 
 @pytest.fixture(scope="module")
-def checker(cuda_ok):
+def gpu_side(cuda_ok):
     src = [SRC, os.path.join(CSRC, "qcs_fit_math.cuh")]
     if not os.path.exists(OUT) or os.path.getmtime(OUT) < max(map(os.path.getmtime, src)):
         os.makedirs(os.path.dirname(OUT), exist_ok=True)
@@ -40,9 +40,9 @@ def checker(cuda_ok):
     return C.CDLL(OUT)
 
 
-def test_flushing_exp_and_log_over_every_float(checker):
+def test_flushing_exp_and_log_over_every_float(gpu_side):
     out = (C.c_ulonglong * 4)()
-    assert checker.check_exp_log(out) == 0
+    assert gpu_side.check_exp_log(out) == 0
     assert list(out) == [0, 0, 0, 0]
 
 
@@ -77,7 +77,7 @@ def parameters(kind, R, name, rng):
     return np.concatenate(cols, 1).astype(np.float32)
 
 
-def differences(checker, kind, R, lanes, name):
+def differences(gpu_side, kind, R, lanes, name):
     """(cases whose losses or gradient differ, share of the losses at x in the flushing form)."""
     rng = np.random.default_rng(100 * R + 10 * kind + lanes)
     x = parameters(kind, R, name, rng)
@@ -90,7 +90,7 @@ def differences(checker, kind, R, lanes, name):
     fast, general = np.zeros((N, wide), np.float32), np.ones((N, wide), np.float32)
     path = np.zeros(N, np.int32)
     p = [C.c_void_p(a.ctypes.data) for a in (pix, sigma, x, d, fast, general, path)]
-    assert checker.check_evaluator(R, kind, lanes, N, *p) == 0
+    assert gpu_side.check_evaluator(R, kind, lanes, N, *p) == 0
     same = (fast.view(np.uint32) == general.view(np.uint32)) | (np.isnan(fast) & np.isnan(general))
     return int((~same).any(1).sum()), float((path & 1).mean())
 
@@ -102,8 +102,8 @@ EVALUATORS = [(k, R, lanes) for k, R in SINGLE for lanes in (1, 16, 32)] + MULTI
 
 @pytest.mark.parametrize("kind,R,lanes", EVALUATORS)
 @pytest.mark.parametrize("name", ["ordinary", "dark", "narrow", "outside", "ties"])
-def test_evaluator_equals_the_general_loss_and_gradient(checker, kind, R, lanes, name):
-    bad, flushing = differences(checker, kind, R, lanes, name)
+def test_evaluator_equals_the_general_loss_and_gradient(gpu_side, kind, R, lanes, name):
+    bad, flushing = differences(gpu_side, kind, R, lanes, name)
     assert bad == 0
     if name == "ordinary":
         # the comparison is with the flushing form: 1.28 photons of background at least; several emitters: unless
